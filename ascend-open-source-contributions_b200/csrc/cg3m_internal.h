@@ -149,11 +149,9 @@ enum : int {
     kStatWords = 8
 };
 
-// Output rows of the exact recompute's tile; its width is ozaki_tile_n(n).
-// It runs on every tile holding a 16 x 16 tile with more than kSparseMax
-// flagged outputs.
+// Side of the exact recompute's tiles.  It runs on every tile holding a 16 x 16
+// tile with more than kSparseMax flagged outputs.
 constexpr int kOzakiTile = 256;
-int ozaki_tile_n(int n);
 
 // Exponents, rounding counts, residue planes and product residues of the
 // tensor-core forms' exact recompute (ozaki.cu), carved from the rounding
@@ -163,10 +161,10 @@ struct OzLayout {
     int* F = nullptr;            // op(B) column exponents
     int* CA = nullptr;           // rounded parts per op(A) row
     int* CB = nullptr;           // rounded parts per op(B) column
-    uint8_t* tile_ran = nullptr; // per exact tile: 1 when it ran
-    int8_t* planes_a = nullptr;  // operand residues, [modulus][part][row][kpitch]
+    uint8_t* tile_ran = nullptr; // per exact tile: 1 when it runs (written by the density test)
+    int8_t* planes_a = nullptr;  // operand residues, [modulus][image][row][kpitch]
     int8_t* planes_b = nullptr;
-    uint8_t* residues = nullptr; // product residues, [modulus][part][col / 16][y_pad][16]
+    uint8_t* residues = nullptr; // product residues, [modulus][image][col / 16][y_pad][16]
     int kpitch = 0;
     size_t plane_bytes = 0;
     int y_pad = 0;               // order rounded up to whole exact tiles
@@ -177,11 +175,11 @@ OzLayout oz_layout(int n, uint8_t* base, std::vector<size_t>* guards = nullptr);
 // Residues of op(A) rows and op(B) columns (needs only the packed rows).
 cudaError_t launch_ozaki_split(cudaStream_t s, int n, int pitch, const float2* rows_a, const float2* rows_b,
                                const OzLayout& L);
-// The exact products of every tile holding a dense 16 x 16 tile and their
+// The exact products of every tile marked in L.tile_ran and their
 // reconstruction into every output of those tiles; outputs it cannot certify
 // are marked in fallback_bits.  Two launches; mark(i) after the i-th (1-based).
-cudaError_t launch_ozaki_tiles(cudaStream_t s, int n, const OzLayout& L, const uint32_t* tile_count, uint32_t* stats, uint32_t* fallback_bits, float2* C,
-                               int* status, int* launched, const std::function<void(int)>& mark);
+cudaError_t launch_ozaki_tiles(cudaStream_t s, int n, const OzLayout& L, uint32_t* stats, uint32_t* fallback_bits,
+                               float2* C, int* status, int* launched, const std::function<void(int)>& mark);
 // Bytes of the rounding-correction region for a square problem of order n.
 size_t rounding_bytes(int n, int form, std::vector<size_t>* guards = nullptr);
 // Device address of the pass's counters (flagged, recomputed as tiles, one by

@@ -157,21 +157,39 @@ __global__ void select_kernel(int n, const float2* __restrict__ C, const float* 
 }
 
 // Per 256 x 256 tile (blockIdx.x: op(A) row band, blockIdx.y: op(B) column
-// band): when none of its 16 x 16 count tiles holds more than kSparseMax
-// flagged outputs (the exact recompute's and the pair kernel's own test), the
-// form's products run there and read that row band of op(A) and column band
-// of op(B), so both bands are marked for the rest of the pack.
+// band): the exact recompute takes it (tile_ran) when one of its 16 x 16 count
+// tiles holds more than kSparseMax flagged outputs.  Otherwise the form's
+// products run there (the pair kernel's own test of the same counts) and read
+// that row band of op(A) and column band of op(B), so both bands are marked
+// for the rest of the pack.
 static_assert(kOzakiTile / kTile == 16, "16 x 16 count tiles per exact tile");
 __global__ void __launch_bounds__(256) band_need_kernel(int n, const uint32_t* __restrict__ tile_count,
-                                                         uint8_t* __restrict__ band_a, uint8_t* __restrict__ band_b)
+                                                         uint8_t* __restrict__ band_a, uint8_t* __restrict__ band_b,
+                                                         uint8_t* __restrict__ tile_ran, uint32_t* __restrict__ stats)
 {
     const int g16 = (n + kTile - 1) / kTile;
     const int gi = blockIdx.x * 16 + threadIdx.x % 16;
     const int gj = blockIdx.y * 16 + threadIdx.x / 16;
-    const bool dense = gi < g16 && gj < g16 && tile_count[(size_t)gj * g16 + gi] > kSparseMax;
-    if (!__syncthreads_or(dense) && threadIdx.x == 0) {
-        band_a[blockIdx.x] = 1;
-        band_b[blockIdx.y] = 1;
+    const uint32_t count = gi < g16 && gj < g16 ? tile_count[(size_t)gj * g16 + gi] : 0u;
+    const bool run = __syncthreads_or(count > kSparseMax);
+    if (threadIdx.x == 0) {
+        tile_ran[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = run ? 1 : 0;
+        if (run) {
+            atomicAdd(&stats[kStatExactTiles], 1u);
+            // output positions of the tile inside the matrix (the roofline's work)
+            const int rows = min(kOzakiTile, n - (int)blockIdx.x * kOzakiTile);
+            const int cols = min(kOzakiTile, n - (int)blockIdx.y * kOzakiTile);
+            atomicAdd(&stats[kStatExactOutputs], (uint32_t)(rows * cols));
+        } else {
+            band_a[blockIdx.x] = 1;
+            band_b[blockIdx.y] = 1;
+        }
+    }
+    if (run) {
+        const uint32_t flagged = __reduce_add_sync(0xffffffffu, count);
+        if ((threadIdx.x & 31) == 0 && flagged != 0) {
+            atomicAdd(&stats[kStatDenseOutputs], flagged);
+        }
     }
 }
 
@@ -614,22 +632,6 @@ __global__ void __launch_bounds__(256) lanes_needed_kernel(int n, int tc, const 
 
 // ---- 4c. per-output recompute of sparse tiles ----------------------------------
 
-// Whether the exact (int8 residue) recompute tile holding 16 x 16 tile (gi, gj)
-// runs, i.e. holds a dense 16 x 16 tile (ozaki_pair_kernel's predicate).
-__device__ __forceinline__ bool ozaki_tile_dense(const uint32_t* tile_count, int tiles16, int gi, int gj, int gn)
-{
-    constexpr int G = kOzakiTile / kTile;  // count tiles down the exact tile; gn across it
-    const int bi = gi / G * G, bj = gj / gn * gn;
-    bool dense = false;
-    for (int q = 0; q < G * gn; ++q) {
-        const int qi = bi + q % G, qj = bj + q / G;
-        if (qi < tiles16 && qj < tiles16) {
-            dense |= tile_count[qj * tiles16 + qi] > kSparseMax;
-        }
-    }
-    return dense;
-}
-
 // Per-output recompute, one block of 64 threads per 16 x 16 output tile.
 //   kSparseFp32 / kSparseFp64: tiles holding between 1 and kSparseMax
 //     flagged outputs (FP64: outside every tile the exact recompute takes);
@@ -653,7 +655,7 @@ __global__ void __launch_bounds__(kLanes) recompute_sparse(int n, int span,
                                                           const uint32_t* __restrict__ bits,
                                                           const uint32_t* __restrict__ tile_count,
                                                           uint32_t* __restrict__ stats, float2* __restrict__ C,
-                                                          int exact_gn)
+                                                          const uint8_t* __restrict__ tile_ran, int exact_tiles)
 {
     constexpr bool FP64 = MODE != kSparseFp32;
     __shared__ float sr[kLanes], si[kLanes], tr[kLanes], ti[kLanes];
@@ -693,7 +695,8 @@ __global__ void __launch_bounds__(kLanes) recompute_sparse(int n, int span,
         }
     }
     // The exact recompute writes (or marks) every flagged output of its tiles.
-    if (MODE == kSparseFp64 && ozaki_tile_dense(tile_count, tiles, gi, gj, exact_gn)) {
+    if (MODE == kSparseFp64 &&
+        tile_ran[(size_t)(gj * kTile / kOzakiTile) * exact_tiles + gi * kTile / kOzakiTile]) {
         return;
     }
     if (l == 0) {
@@ -1115,7 +1118,6 @@ cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan&
     // exactly one of them.
     const int tiles16 = (n + kTile - 1) / kTile;
     float2* C = static_cast<float2*>(p.C);
-    const int exact_gn = plan.form == CG3M_FORM_FP32 ? 1 : ozaki_tile_n(n) / kTile;
     const int pitch = row_pitch(n);
     // lane-major copies of the rows and columns the per-output kernels read
     auto lanes = [&]() {
@@ -1137,7 +1139,7 @@ cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan&
         // stride walk) saved ~0.02 ms of block launches where no tile has work
         // but made the reference's data (~7 flagged outputs per tile) 1.6-2.5x slower
         kernel<<<tiles16 * tiles16, kLanes, 0, s>>>(n, span, L.lanes_a, L.lanes_b, bits, L.tile_count, L.stats, C,
-                                                    exact_gn);
+                                                    L.oz.tile_ran, L.oz.y_pad / kOzakiTile);
         const cudaError_t e = cudaGetLastError();
         mark(++count);
         return e;
@@ -1163,7 +1165,8 @@ cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan&
             err = cudaErrorInvalidValue;  // beyond the gated orders
         }
         if (err == cudaSuccess) {
-            band_need_kernel<<<dim3(bands, bands), 256, 0, s>>>(n, L.tile_count, L.band, L.band + kMaxBands);
+            band_need_kernel<<<dim3(bands, bands), 256, 0, s>>>(n, L.tile_count, L.band, L.band + kMaxBands,
+                                                            L.oz.tile_ran, L.stats);
             err = cudaGetLastError();
             mark(++count);
         }
@@ -1178,8 +1181,8 @@ cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan&
         if (err == cudaSuccess) {
             int oz_launched = 0;
             const int before = count;
-            err = launch_ozaki_tiles(s, n, L.oz, L.tile_count, L.stats, L.fallback_bits, C, status,
-                                     &oz_launched, [&](int i) { mark(before + i); });
+            err = launch_ozaki_tiles(s, n, L.oz, L.stats, L.fallback_bits, C, status, &oz_launched,
+                                     [&](int i) { mark(before + i); });
             count += oz_launched;
         }
         if (err == cudaSuccess) {
