@@ -11,19 +11,19 @@
 // while the accumulation stays FP32.
 //
 // B200 design.  One CTA per 128 x BN output tile (cta_group::1, M = 128,
-// N = BN = 128), 320 threads:
+// N = BN = 128), 576 threads:
 //   warp 0       TMA producer: per K-block and component c in {re, im, sum}
 //                one 3-D box for A (all split planes of c) and one for B,
 //                128-byte rows with the 128-byte swizzle, into a 192 KB
 //                ring (3 stages for 3xTF32, 2 for split-BF16; 64-byte rows
 //                give deeper rings but measured slower);
-//   warp 1       allocates TMEM (512 columns; 256 for BN = 64); one lane
-//                issues every tcgen05.mma: accumulator c (columns
+//   warp 1       allocates TMEM (512 columns; 256 for BN = 64); one elected
+//                lane issues every tcgen05.mma: accumulator c (columns
 //                [BN*c, BN*c + BN)) +=
 //                sum over split pairs (i, j) of A_c,i * B_c,j, smallest terms
 //                first; tcgen05.commit releases each ring slot;
-//   warps 2-9    epilogue: after every 128-term K segment, tcgen05.ld of
-//                P0, P1, P2 (one TMEM lane = one output row, BN/2 columns per
+//   warps 2-17   epilogue: after every 128-term K segment, tcgen05.ld of
+//                P0, P1, P2 (one TMEM lane = one output row, BN/4 columns per
 //                warp), Re_s = P0-P1, Im_s = P2-(P0+P1) added to running Re,
 //                Im in registers with round-to-nearest FP32; at the end
 //                alpha/beta and a column-major C store in which each warp
@@ -56,13 +56,20 @@ constexpr int TILE_M = 128;                     // M of the MMA and rows of the 
 constexpr int ROW_BYTES = 128;                  // one K-block row of one plane (128-byte swizzle)
 constexpr int A_PLANE = TILE_M * ROW_BYTES;     // 16 KB: one A plane, 128 rows
 constexpr int RING_BYTES = 192 * 1024;          // operand ring; stages = RING_BYTES / stage size
-constexpr int kEpilogueWarps = 8;
+constexpr int kEpilogueWarps = 16;
 constexpr int kThreads = (2 + kEpilogueWarps) * 32;
-// 10 warps land 3/3/2/2 on the SM's four sub-partitions, whose register files
-// hold 16K registers each: 3 warps x 32 threads x 168 registers is the most
-// that still launches, so each epilogue thread keeps 2 x 64 running sums
-// (BN = 128) and streams TMEM through 8-column pieces.
-
+// Four epilogue warps per TMEM lane quadrant, 32 columns each: the drain of P0
+// and P1 has to end while the tensor core works on P2, and the more warps
+// share it the shorter its chain of TMEM loads.  18 warps launch at up to 96
+// registers a thread (five warps on the busiest sub-partition's 16K), enough
+// for 2 x 32 running sums.  With eight warps of 64 columns 3xTF32 took 461 us
+// at 1500 x 3100 x 2000 and 76.8 at 1024^3, with sixteen 449 and 67.8.
+//
+// The warp that issues the MMAs stays together and elects one lane, so their
+// descriptors sit in uniform registers: issued from a lane-0 branch, each MMA
+// (64 cycles of the tensor pipe at M = 256, N = 128) waited for its operands.
+// Same shapes, both changes: 527 -> 449 and 78.0 -> 67.8 us; split-BF16 x6 at
+// 4096^3 (bound by L2 and the power limit) 1.68 -> 1.53 ms.
 template <int FORM>
 struct TcCfg;
 
@@ -148,7 +155,7 @@ struct TcGeom {
     static constexpr int B_PLANE = BN * ROW_BYTES;
     static constexpr int STAGE_BYTES = Cfg::S * (A_PLANE + B_PLANE);
     static constexpr int STAGES = RING_BYTES / STAGE_BYTES;
-    static constexpr int COLS = BN / 2;                        // columns per epilogue thread
+    static constexpr int COLS = BN / (kEpilogueWarps / 4);     // columns per epilogue thread
     static constexpr int TMEM_COLS = 4 * BN;                   // 3 accumulators + the spare block
     static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024 + 256;
     static_assert(TMEM_COLS == 256 || TMEM_COLS == 512, "TMEM allocation must be a power of two");
@@ -346,36 +353,44 @@ __global__ void __launch_bounds__(kThreads, 1)
     // segment, one ring stage holding component c's split planes of A and B.
     if (warp == 0) {
         // ---------------- TMA producer ----------------
-        if (lane == 0) {
+        // The whole warp walks the loop, one elected lane issues.
+        const bool issuer = elect_one();
+        if (issuer) {
             tma_prefetch_desc(&tmA);
             tma_prefetch_desc(&tmB);
-            int it = 0;
-            bool stop = false;
-            for (int seg = 0; seg < segments && !stop; ++seg) {
-                const int kb0 = seg * seg_blocks, kb1 = min(kblocks, kb0 + seg_blocks);
-                for (int c = 0; c < 3 && !stop; ++c) {
-                    for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                        const int s = it % STAGES;
-                        if ((it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, p.status)) ||
-                            *abort_flag) {
-                            *abort_flag = 1;
-                            stop = true;
-                            break;
-                        }
-                        uint8_t* st = ring + s * STAGE_BYTES;
+        }
+        int it = 0;
+        bool stop = false;
+        for (int seg = 0; seg < segments && !stop; ++seg) {
+            const int kb0 = seg * seg_blocks, kb1 = min(kblocks, kb0 + seg_blocks);
+            for (int c = 0; c < 3 && !stop; ++c) {
+                for (int kb = kb0; kb < kb1; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    if (!warp_all((it < STAGES || mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, p.status)) &&
+                                  !*abort_flag)) {
+                        *abort_flag = 1;
+                        stop = true;
+                        break;
+                    }
+                    uint8_t* st = ring + s * STAGE_BYTES;
+                    if (issuer) {
                         mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
                         tma_load_3d(st, &tmA, &full[s], kbeg + kb * Cfg::BK, m0, c * Cfg::ZS);
                         tma_load_3d(st + Cfg::S * A_PLANE, &tmB, &full[s], kbeg + kb * Cfg::BK, n0, c * Cfg::ZS);
                     }
                 }
             }
-            for (int j = it > STAGES ? it - STAGES : 0; j < it; ++j) {
-                mbar_wait(&full[j % STAGES], (j / STAGES) & 1, p.status);
-            }
+        }
+        for (int j = it > STAGES ? it - STAGES : 0; j < it; ++j) {
+            mbar_wait(&full[j % STAGES], (j / STAGES) & 1, p.status);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        // The whole warp walks the loop, one elected lane issues.
+        {
+            const bool issuer = elect_one();
+            // descriptor of the ring's start; the address field counts 16 bytes
+            const uint64_t desc0 = smem_desc(smem_u32(ring));
             const uint32_t idesc = instr_desc<Cfg::FMT, BN>();
             int it = 0;
             bool stop = false;
@@ -383,7 +398,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int kb0 = seg * seg_blocks, kb1 = min(kblocks, kb0 + seg_blocks);
                 for (int c = 0; c < 3 && !stop; ++c) {
                     if (seg > 0) {
-                        if (!mbar_wait(&acc_free[c], (seg - 1) & 1, p.status)) {
+                        if (!warp_all(mbar_wait(&acc_free[c], (seg - 1) & 1, p.status))) {
                             *abort_flag = 1;
                             stop = true;
                             break;
@@ -393,49 +408,55 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const uint32_t d = tmem + (uint32_t)(c * BN);
                     for (int kb = kb0; kb < kb1; ++kb, ++it) {
                         const int s = it % STAGES;
-                        if (!mbar_wait(&full[s], (it / STAGES) & 1, p.status)) {
+                        if (!warp_all(mbar_wait(&full[s], (it / STAGES) & 1, p.status))) {
                             *abort_flag = 1;
                             stop = true;
                             break;
                         }
                         tc_fence_after();
-                        const uint32_t a_base = smem_u32(ring + s * STAGE_BYTES);
-                        const uint32_t b_base = a_base + Cfg::S * A_PLANE;
+                        const uint64_t a_desc = desc0 + (uint32_t)(s * (STAGE_BYTES >> 4));
+                        const uint64_t b_desc = a_desc + (uint32_t)((Cfg::S * A_PLANE) >> 4);
+                        if (issuer) {
 #pragma unroll
-                        for (int kk = 0; kk < KSTEPS; ++kk) {
+                            for (int kk = 0; kk < KSTEPS; ++kk) {
 #pragma unroll
-                            for (int q = 0; q < Cfg::NPAIRS; ++q) {
-                                const int2 ij = Cfg::pair(q);
-                                const uint64_t ad = smem_desc(a_base + ij.x * A_PLANE + kk * 32);
-                                const uint64_t bd = smem_desc(b_base + ij.y * G::B_PLANE + kk * 32);
-                                const uint32_t acc = (kb > kb0 || kk > 0 || q > 0) ? 1u : 0u;
-                                if constexpr (Cfg::FMT == 2) {
-                                    umma_tf32(d, ad, bd, idesc, acc);
-                                } else {
-                                    umma_f16(d, ad, bd, idesc, acc);
+                                for (int q = 0; q < Cfg::NPAIRS; ++q) {
+                                    const int2 ij = Cfg::pair(q);
+                                    const uint64_t ad = a_desc + (uint32_t)((ij.x * A_PLANE + kk * 32) >> 4);
+                                    const uint64_t bd = b_desc + (uint32_t)((ij.y * G::B_PLANE + kk * 32) >> 4);
+                                    const uint32_t acc = (kb > kb0 || kk > 0 || q > 0) ? 1u : 0u;
+                                    if constexpr (Cfg::FMT == 2) {
+                                        umma_tf32(d, ad, bd, idesc, acc);
+                                    } else {
+                                        umma_f16(d, ad, bd, idesc, acc);
+                                    }
                                 }
                             }
+                            umma_commit(&empty[s]);
                         }
-                        umma_commit(&empty[s]);
                     }
                     if (!stop && c > 0) {
                         // Fires when every MMA issued so far has completed: after c == 1
                         // both P0 and P1 of the segment are final, after c == 2 all three.
-                        umma_commit(&acc_full[c]);
+                        if (issuer) {
+                            umma_commit(&acc_full[c]);
+                        }
                     }
                 }
             }
-            umma_commit(mma_done);
+            if (issuer) {
+                umma_commit(mma_done);
+            }
             mbar_wait(mma_done, 0, p.status);  // nothing may still write TMEM when it is freed
         }
     } else {
-        // ---------------- epilogue warps 2..9 ----------------
-        // TMEM lane quadrant = warp % 4; warps 2-5 take the first BN/2 columns,
-        // warps 6-9 the second half, of every accumulator and of the spare block.
+        // ---------------- epilogue warps 2..17 ----------------
+        // TMEM lane quadrant = warp % 4; the four warps of a quadrant take 32
+        // columns each of every accumulator and of the spare block.
         const int quad = warp & 3;
-        const int half = (warp - 2) >> 2;
+        const int group = (warp - 2) >> 2;
         const int row = m0 + quad * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * COLS);
+        const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(group * COLS);
         const uint32_t spare = lane_addr + (uint32_t)(3 * BN);
         float re[COLS], im[COLS];
         bool go = true;
@@ -493,7 +514,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (go && row < p.m) {
 #pragma unroll
             for (int j = 0; j < COLS; ++j) {
-                const int col = n0 + half * COLS + j;
+                const int col = n0 + group * COLS + j;
                 if (col < p.n) {
                     if (p.parts == 1) {
                         float2* cp = p.C + (size_t)col * p.ldc + row;
@@ -601,32 +622,40 @@ __global__ void __launch_bounds__(kLeadThreads, 1)
 
     if (warp == 0) {
         // ---------------- TMA producer: one stage per K-block ----------------
-        if (lane == 0) {
+        // The whole warp walks the loop, one elected lane issues.
+        const bool issuer = elect_one();
+        if (issuer) {
             tma_prefetch_desc(&tmA);
             tma_prefetch_desc(&tmB);
-            int it = 0;
-            for (; it < kblocks; ++it) {
-                const int s = it % kLeadStages;
-                if ((it >= kLeadStages && !mbar_wait(&empty[s], ((it / kLeadStages) - 1) & 1, p.status)) ||
-                    *abort_flag) {
-                    *abort_flag = 1;
-                    break;
-                }
-                uint8_t* st = ring + s * kLeadStage;
-                const int k = it * Cfg::BK;
+        }
+        int it = 0;
+        for (; it < kblocks; ++it) {
+            const int s = it % kLeadStages;
+            if (!warp_all((it < kLeadStages || mbar_wait(&empty[s], ((it / kLeadStages) - 1) & 1, p.status)) &&
+                          !*abort_flag)) {
+                *abort_flag = 1;
+                break;
+            }
+            uint8_t* st = ring + s * kLeadStage;
+            const int k = it * Cfg::BK;
+            if (issuer) {
                 mbar_arrive_expect_tx(&full[s], kLeadStage);
                 tma_load_3d(st, &tmA, &full[s], k, m0, 0);
                 tma_load_3d(st + A_PLANE, &tmA, &full[s], k, m0, Cfg::ZS);
                 tma_load_3d(st + 2 * A_PLANE, &tmB, &full[s], k, n0, 0);
                 tma_load_3d(st + 3 * A_PLANE, &tmB, &full[s], k, n0, Cfg::ZS);
             }
-            for (int j = it > kLeadStages ? it - kLeadStages : 0; j < it; ++j) {
-                mbar_wait(&full[j % kLeadStages], (j / kLeadStages) & 1, p.status);
-            }
+        }
+        for (int j = it > kLeadStages ? it - kLeadStages : 0; j < it; ++j) {
+            mbar_wait(&full[j % kLeadStages], (j / kLeadStages) & 1, p.status);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        // The whole warp walks the loop, one elected lane issues.
+        {
+            const bool issuer = elect_one();
+            // descriptor of the ring's start; the address field counts 16 bytes
+            const uint64_t desc0 = smem_desc(smem_u32(ring));
             const uint32_t idesc = instr_desc<Cfg::FMT, kLeadBN>();
             const uint32_t idesc_neg = idesc | kNegateA;
             const uint32_t d_re = tmem, d_im = tmem + (uint32_t)kLeadBN;
@@ -634,7 +663,7 @@ __global__ void __launch_bounds__(kLeadThreads, 1)
             bool stop = false;
             for (int seg = 0; seg < segments && !stop; ++seg) {
                 if (seg > 0) {
-                    if (!mbar_wait(acc_free, (seg - 1) & 1, p.status)) {
+                    if (!warp_all(mbar_wait(acc_free, (seg - 1) & 1, p.status))) {
                         *abort_flag = 1;
                         break;
                     }
@@ -643,39 +672,43 @@ __global__ void __launch_bounds__(kLeadThreads, 1)
                 const int kb0 = seg * seg_blocks, kb1 = min(kblocks, kb0 + seg_blocks);
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
                     const int s = it % kLeadStages;
-                    if (!mbar_wait(&full[s], (it / kLeadStages) & 1, p.status)) {
+                    if (!warp_all(mbar_wait(&full[s], (it / kLeadStages) & 1, p.status))) {
                         *abort_flag = 1;
                         stop = true;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t base = smem_u32(ring + s * kLeadStage);
+                    const uint64_t stage = desc0 + (uint32_t)(s * (kLeadStage >> 4));
+                    if (issuer) {
 #pragma unroll
-                    for (int kk = 0; kk < KSTEPS; ++kk) {
-                        const uint64_t a_re = smem_desc(base + kk * 32);
-                        const uint64_t a_im = smem_desc(base + A_PLANE + kk * 32);
-                        const uint64_t b_re = smem_desc(base + 2 * A_PLANE + kk * 32);
-                        const uint64_t b_im = smem_desc(base + 3 * A_PLANE + kk * 32);
-                        const uint32_t acc = (kb > kb0 || kk > 0) ? 1u : 0u;
-                        if constexpr (Cfg::FMT == 2) {
-                            umma_tf32(d_re, a_re, b_re, idesc, acc);
-                            umma_tf32(d_re, a_im, b_im, idesc_neg, 1u);
-                            umma_tf32(d_im, a_re, b_im, idesc, acc);
-                            umma_tf32(d_im, a_im, b_re, idesc, 1u);
-                        } else {
-                            umma_f16(d_re, a_re, b_re, idesc, acc);
-                            umma_f16(d_re, a_im, b_im, idesc_neg, 1u);
-                            umma_f16(d_im, a_re, b_im, idesc, acc);
-                            umma_f16(d_im, a_im, b_re, idesc, 1u);
+                        for (int kk = 0; kk < KSTEPS; ++kk) {
+                            const uint64_t a_re = stage + (uint32_t)((kk * 32) >> 4);
+                            const uint64_t a_im = a_re + (uint32_t)(A_PLANE >> 4);
+                            const uint64_t b_re = a_re + (uint32_t)((2 * A_PLANE) >> 4);
+                            const uint64_t b_im = a_re + (uint32_t)((3 * A_PLANE) >> 4);
+                            const uint32_t acc = (kb > kb0 || kk > 0) ? 1u : 0u;
+                            if constexpr (Cfg::FMT == 2) {
+                                umma_tf32(d_re, a_re, b_re, idesc, acc);
+                                umma_tf32(d_re, a_im, b_im, idesc_neg, 1u);
+                                umma_tf32(d_im, a_re, b_im, idesc, acc);
+                                umma_tf32(d_im, a_im, b_re, idesc, 1u);
+                            } else {
+                                umma_f16(d_re, a_re, b_re, idesc, acc);
+                                umma_f16(d_re, a_im, b_im, idesc_neg, 1u);
+                                umma_f16(d_im, a_re, b_im, idesc, acc);
+                                umma_f16(d_im, a_im, b_re, idesc, 1u);
+                            }
                         }
+                        umma_commit(&empty[s]);
                     }
-                    umma_commit(&empty[s]);
                 }
-                if (!stop) {
+                if (!stop && issuer) {
                     umma_commit(acc_full);
                 }
             }
-            umma_commit(mma_done);
+            if (issuer) {
+                umma_commit(mma_done);
+            }
             mbar_wait(mma_done, 0, p.status);  // nothing may still write TMEM when it is freed
         }
     } else {
@@ -802,7 +835,7 @@ __global__ void __launch_bounds__(kLeadThreads, 1)
 //     arms it with the pair's byte count;
 //   - MMA completion is committed to `empty`, `acc_full` and `mma_done` in
 //     both CTAs (multicast commit); the odd CTA's epilogue warps arrive on the
-//     even CTA's `acc_free` (16 arrivals per phase);
+//     even CTA's `acc_free` (32 arrivals per phase);
 //   - TMEM (512 columns) is allocated and freed by warp 1 of both CTAs;
 //   - a cluster barrier after set-up and before tear-down keeps both CTAs'
 //     barriers and shared memory alive while the peer may use them.
@@ -817,7 +850,7 @@ struct PairGeom {
     static constexpr int B_PLANE = PAIR_BHALF * ROW_BYTES;            // 8 KB
     static constexpr int STAGE_BYTES = Cfg::S * (A_PLANE + B_PLANE);   // per CTA
     static constexpr int STAGES = PAIR_RING / STAGE_BYTES;
-    static constexpr int COLS = PAIR_BN / 2;
+    static constexpr int COLS = PAIR_BN / (kEpilogueWarps / 4);
     static constexpr int TMEM_COLS = 4 * PAIR_BN;
     static constexpr size_t SMEM = (size_t)STAGES * STAGE_BYTES + 1024 + 256;
 };
@@ -921,24 +954,29 @@ __global__ void __launch_bounds__(kThreads, 1)
 
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
-        if (lane == 0) {
+        // The whole warp walks the loop, one elected lane issues.
+        const bool issuer = elect_one();
+        if (issuer) {
             tma_prefetch_desc(&tmA);
             tma_prefetch_desc(&tmB);
-            int it = 0;
-            bool stop = false;
-            for (int seg = 0; seg < segments && !stop; ++seg) {
-                const int kb0 = seg * seg_blocks, kb1 = min(kblocks, kb0 + seg_blocks);
-                for (int c = 0; c < 3 && !stop; ++c) {
-                    for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                        const int s = it % STAGES;
-                        if ((it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, p.status)) ||
-                            *abort_flag) {
-                            *abort_flag = 1;
-                            stop = true;
-                            break;
-                        }
-                        uint8_t* st = ring + s * STAGE_BYTES;
-                        const uint32_t bar = mapa_shared(smem_u32(&full[s]), base);
+        }
+        const uint32_t full0 = mapa_shared(smem_u32(full), base);  // the even CTA's barriers
+        int it = 0;
+        bool stop = false;
+        for (int seg = 0; seg < segments && !stop; ++seg) {
+            const int kb0 = seg * seg_blocks, kb1 = min(kblocks, kb0 + seg_blocks);
+            for (int c = 0; c < 3 && !stop; ++c) {
+                for (int kb = kb0; kb < kb1; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    if (!warp_all((it < STAGES || mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, p.status)) &&
+                                  !*abort_flag)) {
+                        *abort_flag = 1;
+                        stop = true;
+                        break;
+                    }
+                    uint8_t* st = ring + s * STAGE_BYTES;
+                    const uint32_t bar = full0 + (uint32_t)s * 8u;
+                    if (issuer) {
                         if (leader) {
                             mbar_arrive_expect_tx(&full[s], 2 * STAGE_BYTES);
                         }
@@ -948,15 +986,19 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                 }
             }
-            if (leader) {
-                for (int j = it > STAGES ? it - STAGES : 0; j < it; ++j) {
-                    mbar_wait(&full[j % STAGES], (j / STAGES) & 1, p.status);
-                }
+        }
+        if (leader) {
+            for (int j = it > STAGES ? it - STAGES : 0; j < it; ++j) {
+                mbar_wait(&full[j % STAGES], (j / STAGES) & 1, p.status);
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (even CTA) ----------------
-        if (leader && lane == 0) {
+        // The whole warp walks the loop, one elected lane issues.
+        if (leader) {
+            const bool issuer = elect_one();
+            // descriptor of the ring's start; the address field counts 16 bytes
+            const uint64_t desc0 = smem_desc(smem_u32(ring));
             const uint32_t idesc = (1u << 4) | (Cfg::FMT << 7) | (Cfg::FMT << 10) | ((uint32_t)(BN >> 3) << 17) |
                                    ((uint32_t)((2 * TILE_M) >> 4) << 24);
             int it = 0;
@@ -965,7 +1007,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int kb0 = seg * seg_blocks, kb1 = min(kblocks, kb0 + seg_blocks);
                 for (int c = 0; c < 3 && !stop; ++c) {
                     if (seg > 0) {
-                        if (!mbar_wait_cluster(&acc_free[c], (seg - 1) & 1, p.status)) {
+                        if (!warp_all(mbar_wait_cluster(&acc_free[c], (seg - 1) & 1, p.status))) {
                             *abort_flag = 1;
                             stop = true;
                             break;
@@ -975,45 +1017,51 @@ __global__ void __launch_bounds__(kThreads, 1)
                     const uint32_t d = tmem + (uint32_t)(c * BN);
                     for (int kb = kb0; kb < kb1; ++kb, ++it) {
                         const int s = it % STAGES;
-                        if (!mbar_wait(&full[s], (it / STAGES) & 1, p.status)) {
+                        if (!warp_all(mbar_wait(&full[s], (it / STAGES) & 1, p.status))) {
                             *abort_flag = 1;
                             stop = true;
                             break;
                         }
                         tc_fence_after();
-                        const uint32_t a_base = smem_u32(ring + s * STAGE_BYTES);
-                        const uint32_t b_base = a_base + Cfg::S * A_PLANE;
+                        const uint64_t a_desc = desc0 + (uint32_t)(s * (STAGE_BYTES >> 4));
+                        const uint64_t b_desc = a_desc + (uint32_t)((Cfg::S * A_PLANE) >> 4);
+                        if (issuer) {
 #pragma unroll
-                        for (int kk = 0; kk < KSTEPS; ++kk) {
+                            for (int kk = 0; kk < KSTEPS; ++kk) {
 #pragma unroll
-                            for (int q = 0; q < Cfg::NPAIRS; ++q) {
-                                const int2 ij = Cfg::pair(q);
-                                const uint64_t ad = smem_desc(a_base + ij.x * A_PLANE + kk * 32);
-                                const uint64_t bd = smem_desc(b_base + ij.y * G::B_PLANE + kk * 32);
-                                const uint32_t acc = (kb > kb0 || kk > 0 || q > 0) ? 1u : 0u;
-                                if constexpr (Cfg::FMT == 2) {
-                                    umma_tf32_pair(d, ad, bd, idesc, acc);
-                                } else {
-                                    umma_f16_pair(d, ad, bd, idesc, acc);
+                                for (int q = 0; q < Cfg::NPAIRS; ++q) {
+                                    const int2 ij = Cfg::pair(q);
+                                    const uint64_t ad = a_desc + (uint32_t)((ij.x * A_PLANE + kk * 32) >> 4);
+                                    const uint64_t bd = b_desc + (uint32_t)((ij.y * G::B_PLANE + kk * 32) >> 4);
+                                    const uint32_t acc = (kb > kb0 || kk > 0 || q > 0) ? 1u : 0u;
+                                    if constexpr (Cfg::FMT == 2) {
+                                        umma_tf32_pair(d, ad, bd, idesc, acc);
+                                    } else {
+                                        umma_f16_pair(d, ad, bd, idesc, acc);
+                                    }
                                 }
                             }
+                            umma_commit_pair(&empty[s], pair_mask);
                         }
-                        umma_commit_pair(&empty[s], pair_mask);
                     }
                     if (!stop && c > 0) {
-                        umma_commit_pair(&acc_full[c], pair_mask);
+                        if (issuer) {
+                            umma_commit_pair(&acc_full[c], pair_mask);
+                        }
                     }
                 }
             }
-            umma_commit_pair(mma_done, pair_mask);
+            if (issuer) {
+                umma_commit_pair(mma_done, pair_mask);
+            }
             mbar_wait(mma_done, 0, p.status);  // nothing may still write TMEM when it is freed
         }
     } else {
-        // ---------------- epilogue warps 2..9 (both CTAs) ----------------
+        // ---------------- epilogue warps 2..17 (both CTAs) ----------------
         const int quad = warp & 3;
-        const int half = (warp - 2) >> 2;
+        const int group = (warp - 2) >> 2;
         const int row = m0 + quad * 32 + lane;
-        const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * COLS);
+        const uint32_t lane_addr = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(group * COLS);
         const uint32_t spare = lane_addr + (uint32_t)(3 * BN);
         const uint32_t free0 = mapa_shared(smem_u32(&acc_free[0]), base);
         const uint32_t free1 = mapa_shared(smem_u32(&acc_free[1]), base);
@@ -1080,7 +1128,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int rl = quad * 32 + lane;
 #pragma unroll
                 for (int j = 0; j < COLS; ++j) {
-                    const int cl = half * COLS + j;
+                    const int cl = group * COLS + j;
                     part_re[cl * TILE_M + rl] = re[j];
                     part_im[cl * TILE_M + rl] = im[j];
                 }
@@ -1088,7 +1136,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         } else if (go && row < p.m) {
 #pragma unroll
             for (int j = 0; j < COLS; ++j) {
-                const int col = n0 + half * COLS + j;
+                const int col = n0 + group * COLS + j;
                 if (col < p.n) {
                     if (p.parts == 1) {
                         float2* cp = p.C + (size_t)col * p.ldc + row;

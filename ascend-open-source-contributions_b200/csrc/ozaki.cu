@@ -472,45 +472,40 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
-        // The whole warp walks the loop, one elected lane issues.
-        const bool issuer = elect_one();
-        if (issuer) {
+        if (lane == 0) {
             tma_prefetch_desc(&tmA);
             tma_prefetch_desc(&tmB);
-        }
-        const uint32_t full0 = mapa_shared(smem_u32(full), 0);  // the even CTA's barriers
-        int it = 0;
-        bool stop = false;
-        for (int g = pid; g < total && !stop; g += pairs) {
-            const int plane = g / per_plane;
-            const OzUnit u = units[g - plane * per_plane];
-            const int m0 = u.tm * OZ_TILE_M + (int)rank * OZ_ROWS;
-            const int b0 = u.tn[0] * OZ_TN + (int)rank * OZ_ROWS, b1 = u.tn[1] * OZ_TN + (int)rank * OZ_ROWS;
-            for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
-                const int slot = it % OZ_STAGES;
-                if (!warp_all((it < OZ_STAGES || mbar_wait(&empty[slot], ((it / OZ_STAGES) - 1) & 1, p.status)) &&
-                              !*abort_flag)) {
-                    *abort_flag = 1;
-                    stop = true;
-                    break;
-                }
-                uint8_t* st = ring + slot * OZ_STAGE;
-                const uint32_t bar = full0 + (uint32_t)slot * 8u;
-                if (issuer) {
+            const uint32_t full0 = mapa_shared(smem_u32(full), 0);  // the even CTA's barriers
+            int it = 0;
+            bool stop = false;
+            for (int g = pid; g < total && !stop; g += pairs) {
+                const int plane = g / per_plane;
+                const OzUnit u = units[g - plane * per_plane];
+                const int m0 = u.tm * OZ_TILE_M + (int)rank * OZ_ROWS;
+                for (int kb = 0; kb < p.kblocks; ++kb, ++it) {
+                    const int slot = it % OZ_STAGES;
+                    if ((it >= OZ_STAGES && !mbar_wait(&empty[slot], ((it / OZ_STAGES) - 1) & 1, p.status)) ||
+                        *abort_flag) {
+                        *abort_flag = 1;
+                        stop = true;
+                        break;
+                    }
+                    uint8_t* st = ring + slot * OZ_STAGE;
+                    const uint32_t bar = full0 + (uint32_t)slot * 8u;
                     if (leader) {
                         mbar_arrive_expect_tx(&full[slot], 2 * (1 + u.halves) * OZ_PLANE);
                     }
                     tma_load_3d_pair(st, &tmA, bar, kb * OZ_BK, m0, plane);
-                    tma_load_3d_pair(st + OZ_PLANE, &tmB, bar, kb * OZ_BK, b0, plane);
-                    if (u.halves == 2) {
-                        tma_load_3d_pair(st + 2 * OZ_PLANE, &tmB, bar, kb * OZ_BK, b1, plane);
+                    for (int h = 0; h < u.halves; ++h) {
+                        tma_load_3d_pair(st + (1 + h) * OZ_PLANE, &tmB, bar, kb * OZ_BK,
+                                         u.tn[h] * OZ_TN + (int)rank * OZ_ROWS, plane);
                     }
                 }
             }
-        }
-        if (leader) {
-            for (int j = it > OZ_STAGES ? it - OZ_STAGES : 0; j < it; ++j) {
-                mbar_wait(&full[j % OZ_STAGES], (j / OZ_STAGES) & 1, p.status);
+            if (leader) {
+                for (int j = it > OZ_STAGES ? it - OZ_STAGES : 0; j < it; ++j) {
+                    mbar_wait(&full[j % OZ_STAGES], (j / OZ_STAGES) & 1, p.status);
+                }
             }
         }
     } else if (warp == 1) {
