@@ -12,23 +12,38 @@
 // Design.  One persistent kernel (grid = SM count x resident blocks) pulls
 // tasks from a device list through an atomic counter; a task is (problem,
 // output tile, K partition), and the list is sorted by decreasing work so the
-// schedule ends on small tasks.  A task stages op(A) and op(B) straight from
-// the caller's interleaved complex matrices into shared-memory planes re, im,
-// fl(re+im) (op() and conjugation applied while staging, the next K-block
-// prefetched into registers during the current one's FFMAs), runs the 3M FFMA
-// micro-kernel of the drop-in (one thread per output, K in increasing order,
-// fmaf into P0, P1, P2 from +0), and either applies alpha/beta and stores, or
-// writes its partition's (Re, Im) partials and counts in on a per-tile counter;
-// the last partition to arrive merges all partitions in partition order with
-// the merge arithmetic of the drop-in and stores.  No block ever waits on
-// another.  Each output is thus a fixed function of the inputs and its K
-// split, bit-identical to the drop-in called with the same k_partitions.
+// schedule ends on small tasks.  A task copies op(A) and op(B) element by
+// element from the caller's interleaved complex matrices into shared memory
+// (8-byte cp.async, zero past the edges, transposed on the way when the matrix
+// runs along K), runs the 3M FFMA micro-kernel of the drop-in (one thread per
+// output, K in increasing order, fmaf into P0, P1, P2 from +0), and either
+// applies alpha/beta and stores, or writes its partition's (Re, Im) partials
+// and counts in on a per-tile counter; the last partition to arrive merges all
+// partitions in partition order with the merge arithmetic of the drop-in and
+// stores.  No block ever waits on another.  Each output is thus a fixed
+// function of the inputs and its K split, bit-identical to the drop-in called
+// with the same k_partitions.
 //
-// Tile (128x64, 64x64, 64x32, 32x32) and K split are chosen per problem from a
-// policy table; the autotuner times every candidate policy on the device with
-// the caller's A and B and a scratch C, keeps the fastest and caches it per
-// batch signature (device, ops, shapes).  Execute may replay a captured CUDA
-// graph holding the counter reset and the one kernel.
+// The micro-kernel works on the interleaved elements as they are: one packed
+// FMA multiplies (xr, xi) by (yr, yi) into (P0, P1), a second one two rows'
+// sums (xr + xi) by (yr + yi) into P2, and the sums are formed in registers.
+// No planes are written to shared memory, the operands of the packed FMAs need
+// no moves, and an element costs one 8-byte shared load for three products: at
+// 8 x 4 outputs per thread 96 bytes per 96 FMAs, which balances shared-memory
+// wavefronts and the FMA pipe.  What bounds the loop is the register file: a
+// packed FMA reads three register pairs, 2 cycles when one of them is reused
+// from the instruction before and 3 when not, so 48 of them with the sums take
+// 141 cycles a warp and K term (50 TFLOP/s by themselves, 42-43 with the copies
+// and epilogues; with planes converted into shared memory: 31-36).  Blocks of
+// 128 threads, three per SM, hide each other's barriers, prologues and
+// epilogues.  64 problems of 256 x 192 x 320: 313 -> 185 us, 512 unequal
+// problems 2190 -> 1700 us.
+//
+// Tile (64x64, 128x32, 32x128, 64x32, 32x32) and K split are chosen per problem
+// from a policy table; the autotuner times every candidate policy on the device
+// with the caller's A and B and a scratch C, keeps the fastest and caches it
+// per batch signature (device, ops, shapes).  Execute may replay a captured
+// CUDA graph holding the counter reset and the one kernel.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -37,6 +52,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "cg3m_internal.h"
@@ -46,12 +62,13 @@
 namespace cg3m {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;  // of the persistent kernels
 constexpr int BK = 16;
-#ifndef CG3M_BATCH_UNROLL
-#define CG3M_BATCH_UNROLL 4
-#endif
-constexpr int kUnroll = CG3M_BATCH_UNROLL;  // K terms unrolled in the FFMA loop
+// K terms unrolled in the FFMA loop.  64 problems of 256 x 192 x 320 in one
+// strided launch: 4 terms 207 us, 8 187, 16 185.  The heterogeneous kernel holds
+// five tile shapes' loops and misses the instruction cache at 16: 512 unequal
+// problems 4 terms 1766 us, 8 1700, 16 1721.
+constexpr int kUnroll = 16, kUnrollMixed = 8;
 
 // Product modes: the standard 3M identity (P0 = Ar.Br, P1 = Ai.Bi,
 // P2 = (Ar+Ai).(Br+Bi); Re = P0 - P1, Im = (P2 - P0) - P1) or four real
@@ -78,7 +95,9 @@ struct BTask {
 };
 
 // Tile shapes (BM x BN): 0: 128x64, 1: 64x64, 2: 128x32, 3: 32x128, 4: 64x32, 5: 32x32.
-// The four-product mode does not use tile 0 (its accumulators would not fit).
+// Tile 0 takes 256 threads in the one-launch kernel (three products only); in
+// the persistent kernels a task of tile 0 is two 64x64 tiles, one after the
+// other.
 constexpr int kTileCount = 6;
 __host__ __device__ constexpr int tile_bm(int t)
 {
@@ -91,22 +110,22 @@ __host__ __device__ constexpr int tile_bn(int t)
 
 template <int BM, int BN, int MODE>
 struct Cfg {
-    static constexpr int MT = BM / 16, NT = BN / 16;  // outputs per thread along m, n
-    static constexpr int VA = MT >= 4 ? 4 : MT, HA = MT / VA;
-    static constexpr int VB = NT >= 4 ? 4 : NT, HB = NT / VB;
-    static constexpr int SA = BM + 4, SB = BN + 4;  // padded plane strides (floats)
-    static constexpr int EA = BM * BK / kThreads, EB = BN * BK / kThreads;  // elements per thread per K-block
-    static constexpr int COMPS = MODE == kMode3M ? 3 : 2;                      // planes per operand
-    static constexpr int A_FLOATS = COMPS * BK * SA, B_FLOATS = COMPS * BK * SB;
-    static constexpr int ACC = MODE == kMode3M ? 3 : 4;                        // accumulators per output
+    static constexpr int AREA = BM * BN;
+    static constexpr int MT = AREA >= 4096 ? 8 : 4;                 // outputs per thread along m
+    static constexpr int NT = AREA >= 2048 ? 4 : 2;                 // and along n
+    static constexpr int TM = BM / MT, TN = BN / NT;                // threads along m, n
+    static constexpr int THREADS = TM * TN;
+    static constexpr int WX = TM < 8 ? TM : 8, WY = 32 / WX;        // a warp's threads along m, n
+    static constexpr int PA = BM + 1, PB = BN + 1;                  // pitch of one K term's elements
+    static constexpr int STAGE = BK * (PA + PB);                    // elements of one K-block
+    static constexpr int ACC2 = MODE == kMode3M ? MT / 2 : MT;      // packed accumulators besides (P0, P1)
 };
 
-// Shared memory: kStages raw stages of interleaved complex elements (as
-// copied, one slot per (thread, element)), then two plane buffers.
-constexpr int kStages = 4;
-constexpr int kRawElems = (128 + 64) * BK;  // largest BM + BN of any tile, times BK
-constexpr int kPlaneFloats = 3 * BK * (128 + 4) + 3 * BK * (64 + 4);
-constexpr size_t kSmemBytes = (size_t)kStages * kRawElems * sizeof(float2) + 2 * (size_t)kPlaneFloats * sizeof(float);
+// Shared memory: a ring of K-blocks, element (row r, K term kk) of op(A) at
+// kk * PA + r, of op(B) after it at kk * PB + r.  The odd pitch spreads the K
+// terms a half-warp writes over all banks when the matrix runs along K.
+constexpr int kStages = 3;
+constexpr size_t kSmemBytes = (size_t)kStages * BK * (128 + 32 + 2) * sizeof(float2);  // the largest 128-thread tile
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p)
 {
@@ -123,106 +142,70 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// One operand's share of a K-block for this thread (q = 0 .. E-1).  The
-// source's contiguous dimension goes to consecutive threads: rows
-// ("rows_contig": op(A) in {N, R}, op(B) in {T, C}; r = e % R, kk = e / R with
-// e = tid + q*kThreads) or K (8 consecutive K of 4 rows per warp; row
-// 16q + r0(tid), K index kk0(tid)).
-//   rows_contig: X[(row0 + r) + k*ld]      else: X[k + (row0 + r)*ld]
+// One operand's share of a K-block for this thread.  The source's contiguous
+// dimension goes to consecutive threads: rows (ROWS: op(A) in {N, R}, op(B) in
+// {T, C}; element (row0 + r, k) at X[(row0 + r) + k*ld]) or K (all BK terms of
+// a row by 16 consecutive threads; X[k + (row0 + r)*ld]).
+template <int R, int THREADS, bool ROWS>
 struct Feed {
-    const float2* origin;  // the matrix (source of the zero-byte copies)
-    const float2* base;    // element q = 0 at K-block 0
-    long long qstep;       // element offset between consecutive q
-    long long kbstep;      // element offset between consecutive K-blocks
-    int r, kk;             // block coordinates of element q = 0
-    int rq, kq;            // coordinate steps between consecutive q
-    int rows;              // valid rows of this tile
-    float conj;            // -1 for op C / R
-};
-
-template <int R>
-__device__ __forceinline__ Feed make_feed(const float2* X, int ld, bool rows_contig, int row0, int rows, int kbeg,
-                                          float conj)
-{
-    Feed f;
-    const int tid = threadIdx.x;
-    if (rows_contig) {
-        f.r = tid % R;
-        f.kk = tid / R;
-        f.rq = 0;
-        f.kq = kThreads / R;
-        f.base = X + (long long)(row0 + f.r) + (long long)(kbeg + f.kk) * ld;
-        f.qstep = (long long)f.kq * ld;
-        f.kbstep = (long long)BK * ld;
-    } else {
-        // Each warp covers 4 rows x 8 consecutive K: 64-byte global segments,
-        // and conflict-free plane stores (row stride = 4 banks mod 32).
-        f.kk = (tid % 8) + 8 * ((tid / 32) % 2);
-        f.r = ((tid / 8) % 4) + 4 * (tid / 64);
-        f.rq = kThreads / BK;
-        f.kq = 0;
-        f.base = X + (long long)(kbeg + f.kk) + (long long)(row0 + f.r) * ld;
-        f.qstep = (long long)f.rq * ld;
-        f.kbstep = BK;
+    static constexpr int PASS = THREADS / (ROWS ? R : BK);  // K terms (rows) one pass of the block covers
+    static constexpr int E = R * BK / THREADS;
+    static_assert(THREADS % (ROWS ? R : BK) == 0 && R * BK % THREADS == 0, "whole elements per thread");
+    static __device__ __forceinline__ int r0() { return ROWS ? threadIdx.x % R : threadIdx.x / BK; }
+    static __device__ __forceinline__ int k0() { return ROWS ? threadIdx.x / R : threadIdx.x % BK; }
+    // this thread's first element of the tile's first K-block
+    static __device__ __forceinline__ const float2* first(const float2* X, int ld, int row0, int kbeg)
+    {
+        return ROWS ? X + (row0 + r0()) + (long long)(kbeg + k0()) * ld
+                    : X + (kbeg + k0()) + (long long)(row0 + r0()) * ld;
     }
-    f.origin = X;
-    f.rows = rows;
-    f.conj = conj;
-    return f;
-}
-
-// Issue this thread's copies of K-block kb into raw slot `raw`; elements past
-// the tile or past the partition's K range read as zero.
-template <int E>
-__device__ __forceinline__ void issue(const Feed& f, float2* raw, int kb, int krel_end)
-{
-    const float2* src = f.base + (long long)kb * f.kbstep;
+    // Issue the copies of the K-block whose first element is src: `rows` valid
+    // rows and `kleft` K terms left; everything past them reads as zero (X, the
+    // matrix, is then the source of a zero-byte copy).
+    static __device__ __forceinline__ void issue(const float2* X, const float2* src, int ld, int rows, int kleft,
+                                                 float2* stage)
+    {
+        const uint32_t dst = smem_u32(stage + k0() * (R + 1) + r0());
 #pragma unroll
-    for (int q = 0; q < E; ++q) {
-        const int r = f.r + q * f.rq;
-        const int kk = kb * BK + f.kk + q * f.kq;
-        const bool ok = r < f.rows && kk < krel_end;
-        cp_async8(smem_u32(raw + threadIdx.x + q * kThreads),
-                  ok ? (const void*)(src + q * f.qstep) : (const void*)f.origin, ok ? 8 : 0);
-    }
-}
-
-// Convert this thread's own elements of a raw slot into the planes
-// re, im (conjugated) [, fl(re + im) for 3M] at dst[(c*BK + kk)*S + r].
-template <int S, int E, int COMPS>
-__device__ __forceinline__ void convert(const Feed& f, const float2* raw, float* dst)
-{
-#pragma unroll
-    for (int q = 0; q < E; ++q) {
-        const float2 v = raw[threadIdx.x + q * kThreads];
-        const float re = v.x, im = v.y * f.conj;
-        const int r = f.r + q * f.rq;
-        const int kk = f.kk + q * f.kq;
-        dst[(0 * BK + kk) * S + r] = re;
-        dst[(1 * BK + kk) * S + r] = im;
-        if constexpr (COMPS == 3) {
-            dst[(2 * BK + kk) * S + r] = __fadd_rn(re, im);
+        for (int q = 0; q < E; ++q) {
+            const bool ok = (ROWS ? r0() : r0() + q * PASS) < rows && (ROWS ? k0() + q * PASS : k0()) < kleft;
+            cp_async8(dst + (uint32_t)(q * PASS * (ROWS ? R + 1 : 1)) * 8u,
+                      ok ? (const void*)(src + (long long)(q * PASS) * ld) : (const void*)X, ok ? 8 : 0);
         }
     }
-}
+};
 
-template <int V>
-__device__ __forceinline__ void ld_vec(const float* p, float* out)
-{
-    if constexpr (V == 4) {
-        const float4 t = *reinterpret_cast<const float4*>(p);
-        out[0] = t.x;
-        out[1] = t.y;
-        out[2] = t.z;
-        out[3] = t.w;
-    } else if constexpr (V == 2) {
-        const float2 t = *reinterpret_cast<const float2*>(p);
-        out[0] = t.x;
-        out[1] = t.y;
-    } else {
-        out[0] = *p;
+// The copies of one K-block of both operands, and the step to the next.
+template <int BM, int BN, int THREADS>
+struct Feeds {
+    const float2 *sa, *sb;  // this thread's first element of the next K-block
+    __device__ __forceinline__ void start(const BProblem& p, int m0, int n0, int kbeg, bool na, bool nb)
+    {
+        sa = na ? Feed<BM, THREADS, true>::first(p.A, p.lda, m0, kbeg)
+                : Feed<BM, THREADS, false>::first(p.A, p.lda, m0, kbeg);
+        sb = nb ? Feed<BN, THREADS, false>::first(p.B, p.ldb, n0, kbeg)
+                : Feed<BN, THREADS, true>::first(p.B, p.ldb, n0, kbeg);
     }
-}
+    __device__ __forceinline__ void issue(const BProblem& p, int m0, int n0, int kleft, bool na, bool nb,
+                                          float2* stage)
+    {
+        if (na) {
+            Feed<BM, THREADS, true>::issue(p.A, sa, p.lda, p.m - m0, kleft, stage);
+            sa += (long long)BK * p.lda;
+        } else {
+            Feed<BM, THREADS, false>::issue(p.A, sa, p.lda, p.m - m0, kleft, stage);
+            sa += BK;
+        }
+        stage += BK * (BM + 1);
+        if (nb) {
+            Feed<BN, THREADS, false>::issue(p.B, sb, p.ldb, p.n - n0, kleft, stage);
+            sb += BK;
+        } else {
+            Feed<BN, THREADS, true>::issue(p.B, sb, p.ldb, p.n - n0, kleft, stage);
+            sb += (long long)BK * p.ldb;
+        }
+    }
+};
 
 // C = beta*C for k == 0 or alpha == 0 (beta == 0: zeros, C not read).
 __device__ __forceinline__ float2 beta_scaled(const EpiParams& e, const float2* cp)
@@ -235,10 +218,16 @@ __device__ __forceinline__ float2 beta_scaled(const EpiParams& e, const float2* 
                        __fadd_rn(__fmul_rn(e.br, c.y), __fmul_rn(e.bi, c.x)));
 }
 
-// Non-finite repair of one output (repair_four_product, epilogue.cuh).
-__device__ float2 repair_product(const BProblem& p, int row, int col)
+// Non-finite repair of one output (repair_four_product, epilogue.cuh), out of
+// line: rare, and inlined once per output it would dwarf the kernels.
+__device__ __noinline__ float2 repair_call(const float2* A, int lda, int ta, const float2* B, int ldb, int tb, int k,
+                                           int row, int col)
 {
-    return repair_four_product(p.A, p.lda, p.ta, p.B, p.ldb, p.tb, p.k, row, col);
+    return repair_four_product(A, lda, ta, B, ldb, tb, k, row, col);
+}
+__device__ __forceinline__ float2 repair_product(const BProblem& p, int row, int col)
+{
+    return repair_call(p.A, p.lda, p.ta, p.B, p.ldb, p.tb, p.k, row, col);
 }
 
 // Partition product (before alpha/beta) of the accumulators of one output.
@@ -254,176 +243,255 @@ __device__ __forceinline__ float2 part_product(float q0, float q1, float q2, flo
 
 __device__ __forceinline__ bool finite2(float2 v) { return isfinite(v.x) && isfinite(v.y); }
 
-// 16 x 16 threads over the tile; each warp is 8 (along m) x 4 (along n)
-// threads, so one vector load of A or B per warp spans at most 128 bytes
-// (one shared-memory wavefront).
-__device__ __forceinline__ int thread_tx() { return ((threadIdx.x >> 5) & 1) * 8 + (threadIdx.x & 7); }
-__device__ __forceinline__ int thread_ty() { return (threadIdx.x >> 6) * 4 + ((threadIdx.x & 31) >> 3); }
-
-// Accumulators: acc[c][i][jj] holds outputs (i, 2jj) and (i, 2jj + 1) of
-// accumulator c, updated together by one packed FMA (__ffma2_rn: two
-// independent round-to-nearest FP32 FMAs), so each output is still the same
-// FMA chain in increasing K.
+// This thread's place in the tile: its outputs are rows tx + TM i, columns
+// ty + TN j.  A half-warp's 8-byte loads cover at most 8 consecutive rows and
+// 4 columns, so each is one shared-memory wavefront.
 template <int BM, int BN, int MODE>
-using AccTile = float2[Cfg<BM, BN, MODE>::ACC][Cfg<BM, BN, MODE>::MT][Cfg<BM, BN, MODE>::NT / 2];
-
-template <int BM, int BN, int MODE>
-__device__ __forceinline__ float acc_at(const AccTile<BM, BN, MODE>& acc, int c, int i, int j)
+__device__ __forceinline__ int2 thread_xy()
 {
-    return (j & 1) ? acc[c][i][j >> 1].y : acc[c][i][j >> 1].x;
+    using G = Cfg<BM, BN, MODE>;
+    constexpr int WM = G::TM / G::WX;  // warps along m
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    return make_int2((warp % WM) * G::WX + lane % G::WX, (warp / WM) * G::WY + lane / G::WX);
 }
+
+// Packed pairs as 64-bit registers.
+__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ uint64_t pack2(float lo, float hi)
+{
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v)
+{
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+
+// Accumulators.  p[i][j] holds output (i, j)'s (P0, P1) = (sum xr yr, sum xi yi).
+// Three products: q[ii][j] holds P2 of outputs (2 ii, j) and (2 ii + 1, j); four
+// products: q[i][j] holds (sum xr yi, sum xi yr).  Every packed FMA
+// (__ffma2_rn) is two independent round-to-nearest FP32 FMAs, so each sum is
+// still one FMA chain in increasing K.
+template <int BM, int BN, int MODE>
+struct Acc {
+    uint64_t p[Cfg<BM, BN, MODE>::MT][Cfg<BM, BN, MODE>::NT];
+    uint64_t q[Cfg<BM, BN, MODE>::ACC2][Cfg<BM, BN, MODE>::NT];
+};
 
 // Partition product of output (i, j) of this thread.
 template <int BM, int BN, int MODE>
-__device__ __forceinline__ float2 acc_product(const AccTile<BM, BN, MODE>& acc, int i, int j)
+__device__ __forceinline__ float2 acc_product(const Acc<BM, BN, MODE>& acc, int i, int j)
 {
-    constexpr int L = Cfg<BM, BN, MODE>::ACC - 1;
-    return part_product<MODE>(acc_at<BM, BN, MODE>(acc, 0, i, j), acc_at<BM, BN, MODE>(acc, 1, i, j),
-                              acc_at<BM, BN, MODE>(acc, 2, i, j), acc_at<BM, BN, MODE>(acc, L, i, j));
+    const float2 p = unpack2(acc.p[i][j]);
+    if constexpr (MODE == kMode3M) {
+        const float2 q = unpack2(acc.q[i >> 1][j]);
+        return part_product<MODE>(p.x, p.y, (i & 1) ? q.y : q.x, 0.0f);
+    } else {
+        const float2 q = unpack2(acc.q[i][j]);
+        return part_product<MODE>(p.x, p.y, q.x, q.y);
+    }
+}
+
+// One staged K-block, BK terms in increasing K: a at the block's first term and
+// this thread's first row, b at its first column.  Conjugated operands (sa, sb
+// = -1) without touching x: y's imaginary part carries sa sb, so xi (sa sb yi)
+// is the product of the signed parts, and the sums are xr + sa xi and
+// yr + sa (sa sb yi), each one rounding.  Four products sign each operand.
+template <int BM, int BN, int MODE, bool CONJ, int UNROLL>
+__device__ __forceinline__ void k_block(const float2* a, const float2* b, float sa, float sb, Acc<BM, BN, MODE>& acc)
+{
+    using G = Cfg<BM, BN, MODE>;
+#pragma unroll UNROLL
+    for (int kk = 0; kk < BK; ++kk) {
+        uint64_t x[G::MT], y[G::NT];
+#pragma unroll
+        for (int i = 0; i < G::MT; ++i) {
+            x[i] = *reinterpret_cast<const uint64_t*>(a + kk * G::PA + i * G::TM);
+        }
+#pragma unroll
+        for (int j = 0; j < G::NT; ++j) {
+            y[j] = *reinterpret_cast<const uint64_t*>(b + kk * G::PB + j * G::TN);
+            if constexpr (CONJ) {
+                y[j] = mul2(y[j], pack2(1.0f, MODE == kMode3M ? sa * sb : sb));
+            }
+        }
+        if constexpr (MODE == kMode3M) {
+#pragma unroll
+            for (int j = 0; j < G::NT; ++j) {
+#pragma unroll
+                for (int i = 0; i < G::MT; ++i) {
+                    acc.p[i][j] = ffma2(x[i], y[j], acc.p[i][j]);
+                }
+            }
+            uint64_t xs[G::MT / 2];
+#pragma unroll
+            for (int i = 0; i < G::MT / 2; ++i) {
+                const float2 u = unpack2(x[2 * i]), v = unpack2(x[2 * i + 1]);
+                xs[i] = CONJ ? pack2(__fmaf_rn(u.y, sa, u.x), __fmaf_rn(v.y, sa, v.x))
+                             : pack2(__fadd_rn(u.x, u.y), __fadd_rn(v.x, v.y));
+            }
+#pragma unroll
+            for (int j = 0; j < G::NT; ++j) {
+                const float2 u = unpack2(y[j]);
+                const float s = CONJ ? __fmaf_rn(u.y, sa, u.x) : __fadd_rn(u.x, u.y);
+                const uint64_t ys = pack2(s, s);
+#pragma unroll
+                for (int i = 0; i < G::MT / 2; ++i) {
+                    acc.q[i][j] = ffma2(xs[i], ys, acc.q[i][j]);
+                }
+            }
+        } else {
+            if constexpr (CONJ) {
+#pragma unroll
+                for (int i = 0; i < G::MT; ++i) {
+                    x[i] = mul2(x[i], pack2(1.0f, sa));
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < G::NT; ++j) {
+                const float2 u = unpack2(y[j]);
+                const uint64_t swapped = pack2(u.y, u.x);
+#pragma unroll
+                for (int i = 0; i < G::MT; ++i) {
+                    acc.p[i][j] = ffma2(x[i], y[j], acc.p[i][j]);
+                    acc.q[i][j] = ffma2(x[i], swapped, acc.q[i][j]);
+                }
+            }
+        }
+    }
+}
+
+// This thread's outputs of the tile at (m0, n0): repair, alpha/beta, store.
+// C is read a column's worth at a time before anything of it is stored.
+template <int BM, int BN, int MODE>
+__device__ __forceinline__ void store_tile(const BProblem& p, int m0, int n0, int2 t, const Acc<BM, BN, MODE>& acc)
+{
+    using G = Cfg<BM, BN, MODE>;
+    const bool reads_c = !p.epi.unit && !p.epi.beta_zero;
+#pragma unroll
+    for (int j = 0; j < G::NT; ++j) {
+        const int col = n0 + t.y + G::TN * j;
+        if (col >= p.n) {
+            break;
+        }
+        float2* cp = p.C + (size_t)col * p.ldc + m0 + t.x;
+        float2 old[G::MT];
+#pragma unroll
+        for (int i = 0; i < G::MT; ++i) {
+            old[i] = reads_c && m0 + t.x + G::TM * i < p.m ? cp[G::TM * i] : make_float2(0.0f, 0.0f);
+        }
+#pragma unroll
+        for (int i = 0; i < G::MT; ++i) {
+            const int row = m0 + t.x + G::TM * i;
+            if (row < p.m) {
+                float2 v = acc_product<BM, BN, MODE>(acc, i, j);
+                if (p.repair && !finite2(v)) {
+                    v = repair_product(p, row, col);
+                }
+                cp[G::TM * i] = epilogue_with(v.x, v.y, p.epi, old[i]);
+            }
+        }
+    }
 }
 
 // The products of K terms [kbeg, kbeg + klen) of the BM x BN tile at (m0, n0),
-// accumulated from zero into acc: kStages raw slots of RAWS elements and two
-// plane buffers of PLS floats.
-template <int BM, int BN, int MODE, int RAWS, int PLS>
-__device__ __forceinline__ void accumulate(const BProblem& p, int m0, int n0, int kbeg, int klen, float2* raw,
-                                           float* planes, AccTile<BM, BN, MODE>& acc)
+// accumulated from zero into acc, through a ring of STAGES K-blocks.  Every
+// thread is past its last shared-memory read when the next barrier completes.
+template <int BM, int BN, int MODE, int STAGES, int UNROLL>
+__device__ __forceinline__ void accumulate(const BProblem& p, int m0, int n0, int kbeg, int klen, float2* ring,
+                                           Acc<BM, BN, MODE>& acc)
 {
     using G = Cfg<BM, BN, MODE>;
-    static_assert(G::A_FLOATS + G::B_FLOATS <= PLS, "planes exceed their buffer");
-    static_assert((BM + BN) * BK <= RAWS, "raw stage exceeds its slot");
-    static_assert((BM * BK) % kThreads == 0 && (BN * BK) % kThreads == 0, "whole elements per thread");
     const int nk = (klen + BK - 1) / BK;
-    const int tx = thread_tx(), ty = thread_ty();
+    const int2 t = thread_xy<BM, BN, MODE>();
     const bool na = p.ta == CG3M_OP_N || p.ta == CG3M_OP_R;
     const bool nb = p.tb == CG3M_OP_N || p.tb == CG3M_OP_R;
-    const Feed fa = make_feed<BM>(p.A, p.lda, na, m0, min(BM, p.m - m0), kbeg,
-                                  (p.ta == CG3M_OP_C || p.ta == CG3M_OP_R) ? -1.0f : 1.0f);
-    const Feed fb = make_feed<BN>(p.B, p.ldb, !nb, n0, min(BN, p.n - n0), kbeg,
-                                  (p.tb == CG3M_OP_C || p.tb == CG3M_OP_R) ? -1.0f : 1.0f);
+    const bool ca = p.ta == CG3M_OP_C || p.ta == CG3M_OP_R;
+    const bool cb = p.tb == CG3M_OP_C || p.tb == CG3M_OP_R;
+    const float sa = ca ? -1.0f : 1.0f, sb = cb ? -1.0f : 1.0f;
+    const bool conj = MODE == kMode3M ? ca != cb || ca : ca || cb;
+    Feeds<BM, BN, G::THREADS> feeds;
+    feeds.start(p, m0, n0, kbeg, na, nb);
 #pragma unroll
-    for (int c = 0; c < G::ACC; ++c)
+    for (int j = 0; j < G::NT; ++j) {
 #pragma unroll
-        for (int i = 0; i < G::MT; ++i)
+        for (int i = 0; i < G::MT; ++i) {
+            acc.p[i][j] = 0;
+        }
 #pragma unroll
-            for (int j = 0; j < G::NT / 2; ++j) {
-                acc[c][i][j] = make_float2(0.0f, 0.0f);
-            }
-
-    // Prologue: K-blocks 0 .. kStages-2 in flight (one commit group each,
-    // empty groups past the end keep the counting uniform).
+        for (int i = 0; i < G::ACC2; ++i) {
+            acc.q[i][j] = 0;
+        }
+    }
+    // Prologue: K-blocks 0 .. STAGES-2 in flight (one commit group each, empty
+    // groups past the end keep the counting uniform).
 #pragma unroll
-    for (int s = 0; s < kStages - 1; ++s) {
+    for (int s = 0; s < STAGES - 1; ++s) {
         if (s < nk) {
-            float2* slot = raw + s * RAWS;
-            issue<G::EA>(fa, slot, s, klen);
-            issue<G::EB>(fb, slot + BM * BK, s, klen);
+            feeds.issue(p, m0, n0, klen - s * BK, na, nb, ring + s * G::STAGE);
         }
         cp_async_commit();
     }
+    int slot = 0, refill = STAGES - 1;
     for (int kb = 0; kb < nk; ++kb) {
-        // Refill the slot converted in the previous iteration (by this same
-        // thread: each thread copies and converts only its own elements).
-        const int nxt = kb + kStages - 1;
+        cp_async_wait<STAGES - 2>();  // this thread's copies of K-block kb have landed
+        // Everyone's have, and everyone is done with K-block kb - 1, whose
+        // stage takes K-block kb + STAGES - 1.
+        __syncthreads();
+        const int nxt = kb + STAGES - 1;
         if (nxt < nk) {
-            float2* slot = raw + (nxt % kStages) * RAWS;
-            issue<G::EA>(fa, slot, nxt, klen);
-            issue<G::EB>(fb, slot + BM * BK, nxt, klen);
+            feeds.issue(p, m0, n0, klen - nxt * BK, na, nb, ring + refill * G::STAGE);
         }
         cp_async_commit();
-        cp_async_wait<kStages - 1>();  // this thread's copies of K-block kb have landed
-        const float2* slot = raw + (kb % kStages) * RAWS;
-        float* sA = planes + (kb & 1) * PLS;
-        float* sB = sA + G::A_FLOATS;
-        convert<G::SA, G::EA, G::COMPS>(fa, slot, sA);
-        convert<G::SB, G::EB, G::COMPS>(fb, slot + BM * BK, sB);
-        // Plane buffer kb&1 was last read in iteration kb-2; this barrier also
-        // orders iteration kb-1's reads before the next iteration's writes.
-        __syncthreads();
-        const float* a = sA + tx * G::VA;
-        const float* b = sB + ty * G::VB;
-#pragma unroll kUnroll
-        for (int kk = 0; kk < BK; ++kk) {
-            float x[G::COMPS][G::MT], y[G::COMPS][G::NT];
-#pragma unroll
-            for (int c = 0; c < G::COMPS; ++c) {
-#pragma unroll
-                for (int h = 0; h < G::HA; ++h) {
-                    ld_vec<G::VA>(a + (c * BK + kk) * G::SA + h * 16 * G::VA, x[c] + h * G::VA);
-                }
-#pragma unroll
-                for (int h = 0; h < G::HB; ++h) {
-                    ld_vec<G::VB>(b + (c * BK + kk) * G::SB + h * 16 * G::VB, y[c] + h * G::VB);
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < G::MT; ++i) {
-                float2 xb[G::COMPS];
-#pragma unroll
-                for (int c = 0; c < G::COMPS; ++c) {
-                    xb[c] = make_float2(x[c][i], x[c][i]);
-                }
-#pragma unroll
-                for (int jj = 0; jj < G::NT / 2; ++jj) {
-                    float2 yp[G::COMPS];
-#pragma unroll
-                    for (int c = 0; c < G::COMPS; ++c) {
-                        yp[c] = make_float2(y[c][2 * jj], y[c][2 * jj + 1]);
-                    }
-                    if constexpr (MODE == kMode3M) {
-                        acc[0][i][jj] = __ffma2_rn(xb[0], yp[0], acc[0][i][jj]);
-                        acc[1][i][jj] = __ffma2_rn(xb[1], yp[1], acc[1][i][jj]);
-                        acc[2][i][jj] = __ffma2_rn(xb[2], yp[2], acc[2][i][jj]);
-                    } else {
-                        acc[0][i][jj] = __ffma2_rn(xb[0], yp[0], acc[0][i][jj]);  // Ar.Br
-                        acc[1][i][jj] = __ffma2_rn(xb[1], yp[1], acc[1][i][jj]);  // Ai.Bi
-                        acc[2][i][jj] = __ffma2_rn(xb[0], yp[1], acc[2][i][jj]);  // Ar.Bi
-                        acc[3][i][jj] = __ffma2_rn(xb[1], yp[0], acc[3][i][jj]);  // Ai.Br
-                    }
-                }
-            }
+        const float2* stage = ring + slot * G::STAGE;
+        if (conj) {
+            k_block<BM, BN, MODE, true, UNROLL>(stage + t.x, stage + BK * G::PA + t.y, sa, sb, acc);
+        } else {
+            k_block<BM, BN, MODE, false, UNROLL>(stage + t.x, stage + BK * G::PA + t.y, 1.0f, 1.0f, acc);
         }
+        slot = slot + 1 == STAGES ? 0 : slot + 1;
+        refill = refill + 1 == STAGES ? 0 : refill + 1;
     }
     cp_async_wait<0>();  // only empty groups can remain; keep the count at zero between tasks
 }
 
-template <int BM, int BN, int MODE>
-__device__ void run_task(const BProblem& prob, int tile, int part, float2* raw, float* planes, float* partials,
-                         uint32_t* counters, int* last_flag)
+template <int BM, int BN, int MODE, int UNROLL>
+__device__ __forceinline__ void run_task(const BProblem& p, int m0, int n0, int tile, int part, float2* ring,
+                                         float* partials, uint32_t* counters, int* last_flag)
 {
     using G = Cfg<BM, BN, MODE>;
-    const BProblem p = prob;  // registers: no reloads after barriers
-    const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
-    const int m0 = tm * BM, n0 = tn * BN;
     const int kbeg = part * p.span;
     const int kend = min(p.k, kbeg + p.span);
     const int klen = kend > kbeg ? kend - kbeg : 0;
-    const int tx = thread_tx(), ty = thread_ty();
-    AccTile<BM, BN, MODE> acc;
-    accumulate<BM, BN, MODE, kRawElems, kPlaneFloats>(p, m0, n0, kbeg, klen, raw, planes, acc);
+    const int2 t = thread_xy<BM, BN, MODE>();
+    Acc<BM, BN, MODE> acc;
+    accumulate<BM, BN, MODE, kStages, UNROLL>(p, m0, n0, kbeg, klen, ring, acc);
 
-    // Output (i, j) of this thread: row m0 + (i / VA)*16*VA + tx*VA + i % VA,
-    // column n0 + (j / VB)*16*VB + ty*VB + j % VB.
     if (p.parts == 1) {
-#pragma unroll
-        for (int j = 0; j < G::NT; ++j) {
-            const int col = n0 + (j / G::VB) * 16 * G::VB + ty * G::VB + j % G::VB;
-#pragma unroll
-            for (int i = 0; i < G::MT; ++i) {
-                const int row = m0 + (i / G::VA) * 16 * G::VA + tx * G::VA + i % G::VA;
+        if (p.k == 0) {
+            for (int e = threadIdx.x; e < BM * BN; e += G::THREADS) {
+                const int row = m0 + e % BM, col = n0 + e / BM;
                 if (row < p.m && col < p.n) {
                     float2* cp = p.C + (size_t)col * p.ldc + row;
-                    if (p.k == 0) {
-                        *cp = beta_scaled(p.epi, cp);
-                    } else {
-                        float2 v = acc_product<BM, BN, MODE>(acc, i, j);
-                        if (p.repair && !finite2(v)) {
-                            v = repair_product(p, row, col);
-                        }
-                        *cp = epilogue_value(v.x, v.y, p.epi, cp);
-                    }
+                    *cp = beta_scaled(p.epi, cp);
                 }
             }
+        } else {
+            store_tile<BM, BN, MODE>(p, m0, n0, t, acc);
         }
         return;
     }
@@ -433,10 +501,10 @@ __device__ void run_task(const BProblem& prob, int tile, int part, float2* raw, 
     const size_t plane = (size_t)p.ppitch * p.n;
 #pragma unroll
     for (int j = 0; j < G::NT; ++j) {
-        const int col = n0 + (j / G::VB) * 16 * G::VB + ty * G::VB + j % G::VB;
+        const int col = n0 + t.y + G::TN * j;
 #pragma unroll
         for (int i = 0; i < G::MT; ++i) {
-            const int row = m0 + (i / G::VA) * 16 * G::VA + tx * G::VA + i % G::VA;
+            const int row = m0 + t.x + G::TM * i;
             if (row < p.m && col < p.n) {
                 const size_t o = (size_t)col * p.ppitch + row;
                 const float2 v = acc_product<BM, BN, MODE>(acc, i, j);
@@ -507,35 +575,45 @@ __device__ void run_task(const BProblem& prob, int tile, int part, float2* raw, 
     }
 }
 
-template <int MODE>
-__device__ __forceinline__ void dispatch_task(const BProblem& p, int tile, int part, float2* raw, float* planes,
-                                              float* partials, uint32_t* counters, int* last_flag)
+// One task of the tile shape: tile 0 walks its 64x64 tiles (unsplit along K, so
+// without counters), the others are one tile.
+template <int TILE, int MODE, int UNROLL>
+__device__ __forceinline__ void tile_task(const BProblem& p, int tile, int part, float2* ring, float* partials,
+                                          uint32_t* counters, int* last_flag)
 {
-    switch (p.tile) {
-        case 0:
-            if constexpr (MODE == kMode3M) {
-                run_task<128, 64, MODE>(p, tile, part, raw, planes, partials, counters, last_flag);
-            }
-            break;
-        case 1: run_task<64, 64, MODE>(p, tile, part, raw, planes, partials, counters, last_flag); break;
-        case 2: run_task<128, 32, MODE>(p, tile, part, raw, planes, partials, counters, last_flag); break;
-        case 3: run_task<32, 128, MODE>(p, tile, part, raw, planes, partials, counters, last_flag); break;
-        case 4: run_task<64, 32, MODE>(p, tile, part, raw, planes, partials, counters, last_flag); break;
-        default: run_task<32, 32, MODE>(p, tile, part, raw, planes, partials, counters, last_flag); break;
+    constexpr int BM = TILE == 0 ? 64 : tile_bm(TILE), BN = tile_bn(TILE);
+    const int m0 = (tile % p.tiles_m) * tile_bm(TILE), n0 = (tile / p.tiles_m) * BN;
+    for (int m = m0; m < min(p.m, m0 + tile_bm(TILE)); m += BM) {
+        if (TILE == 0 && m != m0) {
+            __syncthreads();  // the previous tile's shared-memory reads are done
+        }
+        run_task<BM, BN, MODE, UNROLL>(p, m, n0, tile, part, ring, partials, counters, last_flag);
     }
 }
 
+// Out of line in the heterogeneous kernel, so that each tile shape's loop gets
+// the registers to itself; the strided kernel is instantiated per tile (all
+// shapes inlined side by side spilled: 200 us instead of 185 on 64 problems of
+// 256 x 192 x 320).
+template <int TILE>
+__device__ __noinline__ void tile_task_call(const BProblem& p, int tile, int part, float2* ring, float* partials,
+                                            uint32_t* counters, int* last_flag)
+{
+    tile_task<TILE, kMode3M, kUnrollMixed>(p, tile, part, ring, partials, counters, last_flag);
+}
+
 // Heterogeneous batch: tasks from a device list (problem, tile, partition).
-__global__ void __launch_bounds__(kThreads) batched_kernel(const BProblem* __restrict__ problems,
-                                                           const BTask* __restrict__ tasks, int ntasks,
-                                                           int* __restrict__ next, float* partials,
-                                                           uint32_t* counters)
+__global__ void __launch_bounds__(kThreads, 3) batched_kernel(const BProblem* __restrict__ problems,
+                                                              const BTask* __restrict__ tasks, int ntasks,
+                                                              int* __restrict__ next, float* partials,
+                                                              uint32_t* counters)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* raw = reinterpret_cast<float2*>(smem_raw);
-    float* planes = reinterpret_cast<float*>(smem_raw + (size_t)kStages * kRawElems * sizeof(float2));
+    float2* ring = reinterpret_cast<float2*>(smem_raw);
     __shared__ int task_id;
     __shared__ int last_flag;
+    __shared__ BProblem cur;  // the task's problem: its fields are read where they are used
+    static_assert(sizeof(BProblem) % 4 == 0 && sizeof(BProblem) / 4 <= kThreads, "one word per thread");
     for (;;) {
         __syncthreads();  // the previous task's shared-memory reads are done
         if (threadIdx.x == 0) {
@@ -547,7 +625,18 @@ __global__ void __launch_bounds__(kThreads) batched_kernel(const BProblem* __res
             return;
         }
         const BTask tk = tasks[t];
-        dispatch_task<kMode3M>(problems[tk.problem], tk.tile, tk.part, raw, planes, partials, counters, &last_flag);
+        if (threadIdx.x < sizeof(BProblem) / 4) {
+            reinterpret_cast<uint32_t*>(&cur)[threadIdx.x] =
+                reinterpret_cast<const uint32_t*>(problems + tk.problem)[threadIdx.x];
+        }
+        __syncthreads();
+        switch (cur.tile) {
+            case 1: tile_task_call<1>(cur, tk.tile, tk.part, ring, partials, counters, &last_flag); break;
+            case 2: tile_task_call<2>(cur, tk.tile, tk.part, ring, partials, counters, &last_flag); break;
+            case 3: tile_task_call<3>(cur, tk.tile, tk.part, ring, partials, counters, &last_flag); break;
+            case 4: tile_task_call<4>(cur, tk.tile, tk.part, ring, partials, counters, &last_flag); break;
+            default: tile_task_call<5>(cur, tk.tile, tk.part, ring, partials, counters, &last_flag); break;
+        }
     }
 }
 
@@ -555,16 +644,28 @@ __global__ void __launch_bounds__(kThreads) batched_kernel(const BProblem* __res
 // A + b*sA, B + b*sB, C + b*sC and its own partial / counter ranges; task t
 // is (b, tile, part) = (t / per_batch, (t % per_batch) / parts, t % parts).
 // counters[0] is the task counter; tile counters follow.
-template <int MODE>
-__global__ void __launch_bounds__(kThreads) strided_kernel(BProblem proto, long long sA, long long sB, long long sC,
-                                                           int batch, size_t partial_stride, float* partials,
-                                                           uint32_t* counters)
+// Geometry of the strided kernel's tile (tile 0 walks 64 x 64 tiles).
+template <int MODE, int TILE>
+using StridedCfg = Cfg<TILE == 0 ? 64 : tile_bm(TILE), tile_bn(TILE), MODE>;
+// Blocks per SM the registers allow: 96 accumulators a thread leave room for
+// three, the four-product mode's 128 for two.
+template <int MODE, int TILE>
+constexpr int kStridedBlocks = StridedCfg<MODE, TILE>::AREA >= 4096   ? (MODE == kMode3M ? 3 : 2)
+                               : StridedCfg<MODE, TILE>::AREA >= 2048 ? 4
+                                                                      : 5;
+template <int MODE, int TILE>
+constexpr size_t kStridedSmem = (size_t)kStages * StridedCfg<MODE, TILE>::STAGE * sizeof(float2);
+
+template <int MODE, int TILE>
+__global__ void __launch_bounds__(kThreads, (kStridedBlocks<MODE, TILE>))
+    strided_kernel(const __grid_constant__ BProblem proto, long long sA, long long sB, long long sC, int batch, size_t partial_stride,
+                   float* partials, uint32_t* counters)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* raw = reinterpret_cast<float2*>(smem_raw);
-    float* planes = reinterpret_cast<float*>(smem_raw + (size_t)kStages * kRawElems * sizeof(float2));
+    float2* ring = reinterpret_cast<float2*>(smem_raw);
     __shared__ int task_id;
     __shared__ int last_flag;
+    __shared__ BProblem cur;  // the task's problem: its fields are read where they are used
     const int tiles = proto.tiles_m * proto.tiles_n;
     const int per_batch = tiles * proto.parts;
     const long long ntasks = (long long)per_batch * batch;
@@ -579,13 +680,16 @@ __global__ void __launch_bounds__(kThreads) strided_kernel(BProblem proto, long 
             return;
         }
         const int b = t / per_batch, r = t - b * per_batch;
-        BProblem p = proto;
-        p.A = proto.A + (long long)b * sA;
-        p.B = proto.B + (long long)b * sB;
-        p.C = proto.C + (long long)b * sC;
-        p.partial_off = (size_t)b * partial_stride;
-        p.counter_off = 1 + (size_t)b * tiles;
-        dispatch_task<MODE>(p, r / proto.parts, r % proto.parts, raw, planes, partials, counters, &last_flag);
+        if (threadIdx.x == 0) {
+            cur = proto;
+            cur.A = proto.A + (long long)b * sA;
+            cur.B = proto.B + (long long)b * sB;
+            cur.C = proto.C + (long long)b * sC;
+            cur.partial_off = (size_t)b * partial_stride;
+            cur.counter_off = 1 + (size_t)b * tiles;
+        }
+        __syncthreads();
+tile_task<TILE, MODE, kUnroll>(cur, r / proto.parts, r % proto.parts, ring, partials, counters, &last_flag);
     }
 }
 
@@ -604,11 +708,14 @@ __global__ void __launch_bounds__(kThreads) strided_kernel(BProblem proto, long 
 // barriers are reached by every thread of every block (no early exits).
 template <int BM, int BN, int MODE>
 struct SingleCfg {
-    static constexpr int RAWS = (BM + BN) * BK;  // elements per raw slot
-    static constexpr int PLS = Cfg<BM, BN, MODE>::A_FLOATS + Cfg<BM, BN, MODE>::B_FLOATS;
-    static constexpr size_t SMEM = (size_t)kStages * RAWS * sizeof(float2) + 2 * (size_t)PLS * sizeof(float);
-    static_assert((size_t)2 * BM * BN * sizeof(float) <= (size_t)kStages * RAWS * sizeof(float2),
-                  "partials exceed the raw slots");
+    using G = Cfg<BM, BN, MODE>;
+    static constexpr int STAGES = 4;
+    static constexpr size_t SMEM = (size_t)STAGES * G::STAGE * sizeof(float2);
+    // blocks per SM the registers allow (65536 / threads / registers of the micro-kernel)
+    static constexpr int BLOCKS = G::THREADS == 256 ? 1 : G::AREA >= 4096 ? (MODE == kMode3M ? 3 : 2)
+                                                      : G::AREA >= 2048   ? 4
+                                                                          : 5;
+    static_assert((size_t)2 * BM * BN * sizeof(float) <= SMEM, "partials exceed the ring");
 };
 
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr)
@@ -621,55 +728,40 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t addr)
 constexpr int kMaxClusterParts = 8;  // portable cluster size
 
 template <int BM, int BN, int MODE>
-__global__ void __launch_bounds__(kThreads) single_kernel(const BProblem p)
+__global__ void __launch_bounds__(Cfg<BM, BN, MODE>::THREADS, SingleCfg<BM, BN, MODE>::BLOCKS)
+    single_kernel(const BProblem p)
 {
     using G = Cfg<BM, BN, MODE>;
     using S = SingleCfg<BM, BN, MODE>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2* raw = reinterpret_cast<float2*>(smem_raw);
-    float* planes = reinterpret_cast<float*>(smem_raw + (size_t)kStages * S::RAWS * sizeof(float2));
+    float2* ring = reinterpret_cast<float2*>(smem_raw);
     const int tile = blockIdx.x, part = blockIdx.y;
     const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
     const int m0 = tm * BM, n0 = tn * BN;
     const int kbeg = part * p.span;
     const int kend = min(p.k, kbeg + p.span);
     const int klen = kend > kbeg ? kend - kbeg : 0;
-    const int tx = thread_tx(), ty = thread_ty();
-    AccTile<BM, BN, MODE> acc;
-    accumulate<BM, BN, MODE, S::RAWS, S::PLS>(p, m0, n0, kbeg, klen, raw, planes, acc);
+    const int2 t = thread_xy<BM, BN, MODE>();
+    Acc<BM, BN, MODE> acc;
+    accumulate<BM, BN, MODE, S::STAGES, kUnroll>(p, m0, n0, kbeg, klen, ring, acc);
 
     if (p.parts == 1) {
-#pragma unroll
-        for (int j = 0; j < G::NT; ++j) {
-            const int col = n0 + (j / G::VB) * 16 * G::VB + ty * G::VB + j % G::VB;
-#pragma unroll
-            for (int i = 0; i < G::MT; ++i) {
-                const int row = m0 + (i / G::VA) * 16 * G::VA + tx * G::VA + i % G::VA;
-                if (row < p.m && col < p.n) {
-                    float2 v =
-                        acc_product<BM, BN, MODE>(acc, i, j);
-                    if (p.repair && !finite2(v)) {
-                        v = repair_product(p, row, col);
-                    }
-                    float2* cp = p.C + (size_t)col * p.ldc + row;
-                    *cp = epilogue_value(v.x, v.y, p.epi, cp);
-                }
-            }
-        }
+        store_tile<BM, BN, MODE>(p, m0, n0, t, acc);
         return;
     }
 
     // This partition's (Re, Im) at part_re[e], part_im[e], e = c*BM + r (tile
-    // coordinates), over the raw slots: every thread's copies have landed and
-    // been converted before the K loop's last barrier.
-    float* part_re = reinterpret_cast<float*>(raw);
+    // coordinates), over the ring: every copy has landed, and the barrier puts
+    // every thread past its last read.
+    __syncthreads();
+    float* part_re = reinterpret_cast<float*>(ring);
     float* part_im = part_re + BM * BN;
 #pragma unroll
     for (int j = 0; j < G::NT; ++j) {
-        const int c = (j / G::VB) * 16 * G::VB + ty * G::VB + j % G::VB;
+        const int c = t.y + G::TN * j;
 #pragma unroll
         for (int i = 0; i < G::MT; ++i) {
-            const int r = (i / G::VA) * 16 * G::VA + tx * G::VA + i % G::VA;
+            const int r = t.x + G::TM * i;
             const float2 v = acc_product<BM, BN, MODE>(acc, i, j);
             part_re[c * BM + r] = v.x;
             part_im[c * BM + r] = v.y;
@@ -680,7 +772,7 @@ __global__ void __launch_bounds__(kThreads) single_kernel(const BProblem p)
     const uint32_t im_local = static_cast<uint32_t>(__cvta_generic_to_shared(part_im));
     const int per = (BM * BN + p.parts - 1) / p.parts;  // outputs merged by each block
     const int e_end = min(BM * BN, (part + 1) * per);
-    for (int e = part * per + (int)threadIdx.x; e < e_end; e += kThreads) {
+    for (int e = part * per + (int)threadIdx.x; e < e_end; e += G::THREADS) {
         const int r = e % BM, c = e / BM;
         const int row = m0 + r, col = n0 + c;
         float tr[kMaxClusterParts], ti[kMaxClusterParts];
@@ -714,14 +806,14 @@ __global__ void __launch_bounds__(kThreads) single_kernel(const BProblem p)
 template <int MODE>
 cudaError_t launch_single_tile(cudaStream_t s, const BProblem& bp, int tile)
 {
-    auto run = [&](auto kernel, size_t smem) -> cudaError_t {
+    auto run = [&](auto kernel, int threads, size_t smem) -> cudaError_t {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) {
             return e;
         }
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(bp.tiles_m * bp.tiles_n), (unsigned)bp.parts, 1);
-        cfg.blockDim = dim3(kThreads, 1, 1);
+        cfg.blockDim = dim3((unsigned)threads, 1, 1);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = s;
         cudaLaunchAttribute attr[1];
@@ -733,17 +825,22 @@ cudaError_t launch_single_tile(cudaStream_t s, const BProblem& bp, int tile)
         cfg.numAttrs = 1;
         return cudaLaunchKernelEx(&cfg, kernel, bp);
     };
+    auto launch_tile = [&](auto bm, auto bn) -> cudaError_t {
+        constexpr int BM = decltype(bm)::value, BN = decltype(bn)::value;
+        return run(single_kernel<BM, BN, MODE>, Cfg<BM, BN, MODE>::THREADS, SingleCfg<BM, BN, MODE>::SMEM);
+    };
+    using std::integral_constant;
     switch (tile) {
         case 0:
             if constexpr (MODE == kMode3M) {
-                return run(single_kernel<128, 64, MODE>, SingleCfg<128, 64, MODE>::SMEM);
+                return launch_tile(integral_constant<int, 128>{}, integral_constant<int, 64>{});
             }
             return cudaErrorInvalidValue;
-        case 1: return run(single_kernel<64, 64, MODE>, SingleCfg<64, 64, MODE>::SMEM);
-        case 2: return run(single_kernel<128, 32, MODE>, SingleCfg<128, 32, MODE>::SMEM);
-        case 3: return run(single_kernel<32, 128, MODE>, SingleCfg<32, 128, MODE>::SMEM);
-        case 4: return run(single_kernel<64, 32, MODE>, SingleCfg<64, 32, MODE>::SMEM);
-        default: return run(single_kernel<32, 32, MODE>, SingleCfg<32, 32, MODE>::SMEM);
+        case 1: return launch_tile(integral_constant<int, 64>{}, integral_constant<int, 64>{});
+        case 2: return launch_tile(integral_constant<int, 128>{}, integral_constant<int, 32>{});
+        case 3: return launch_tile(integral_constant<int, 32>{}, integral_constant<int, 128>{});
+        case 4: return launch_tile(integral_constant<int, 64>{}, integral_constant<int, 32>{});
+        default: return launch_tile(integral_constant<int, 32>{}, integral_constant<int, 32>{});
     }
 }
 
@@ -794,12 +891,14 @@ struct Policy {
     int split_cap;
 };
 
-constexpr Policy kPolicies[] = {{8192, 1}, {8192, 2}, {8192, 4}, {8192, 8}, {4096, 1},
-                                {4096, 2}, {4096, 4}, {4096, 8}, {2048, 1}, {2048, 4}};
-constexpr Policy kDefaultPolicy = {8192, 4};
+constexpr Policy kPolicies[] = {{4096, 1}, {4096, 2}, {4096, 4}, {4096, 8}, {2048, 1},
+                                {2048, 2}, {2048, 4}, {1024, 1}, {1024, 2}, {1024, 4}};
+constexpr Policy kDefaultPolicy = {4096, 4};
 
-// Relative FFMA efficiency of each tile shape (per output-element-term).
-constexpr double kTileEfficiency[kTileCount] = {1.0, 0.85, 0.8, 0.8, 0.65, 0.45};
+// Relative FFMA efficiency of each tile shape (per output-element-term), from
+// the per-term cost of blocks sharing an SM (kSingleCost below): the narrower
+// tiles load more shared memory per FMA.
+constexpr double kTileEfficiency[kTileCount] = {1.0, 1.0, 0.93, 0.88, 0.87, 0.75};
 
 int span_for(int k, int parts) { return ceil_div(ceil_div(k, 16), parts) * 16; }
 
@@ -810,7 +909,7 @@ double choose_tile(BProblem& p, int max_area, int mode)
     int best = kTileCount - 1;
     double best_cost = 1e300;
     for (int t = 0; t < kTileCount; ++t) {
-        if (tile_bm(t) * tile_bn(t) > max_area || (mode == kMode4M && t == 0)) {
+        if (t == 0 || tile_bm(t) * tile_bn(t) > max_area) {
             continue;
         }
         const double work =
@@ -1027,17 +1126,89 @@ Policy autotune(cg3mBatchPlan* plan, cudaStream_t s)
 
 namespace cg3m {
 
+int single_tile_bm(int tile) { return tile_bm(tile); }
+int single_tile_bn(int tile) { return tile_bn(tile); }
+
+// Time model of the one-launch kernel (three-product mode), in microseconds,
+// fitted on B200 to 2500 timed (shape, tile, partitions) launches (median
+// error 2-4 % per tile; the tile and split it picks cost a mean 2 % over the
+// best of each shape).  Clusters of `parts` blocks run in waves of as many
+// clusters as fit at once; a wave costs a fixed part and span x the per-term
+// time a block needs by itself.  Blocks that share an SM add a per-term cost
+// for every layer of clusters: one layer holds as many as fit with one block
+// per SM, which is fewer than sm_count / parts (GPC boundaries), so a split
+// of 7 or 8 starts its second layer at 105 or 120 blocks.
+namespace {
+struct SingleCost {
+    double base_us, fixed_us, term_ns, shared_term_ns, merge_us;
+};
+constexpr SingleCost kSingleCost[kTileCount] = {{3.396, 3.006, 0.0, 167.65, 0.031},  {6.203, 0.0, 25.64, 70.90, 0.0},
+                                                {4.231, 2.119, 18.57, 76.50, 0.0},   {3.417, 2.711, 16.39, 80.99, 0.135},
+                                                {3.483, 0.0, 17.18, 40.77, 0.131},   {1.719, 0.927, 13.61, 23.63, 0.150}};
+// Blocks per SM of each tile (SingleCfg::BLOCKS), three and four products.
+constexpr int kSingleOcc[2][kTileCount] = {{1, 3, 3, 3, 4, 5}, {1, 2, 2, 2, 4, 5}};
+// Clusters resident at once on 148 SMs (cudaOccupancyMaxActiveClusters), by
+// blocks per SM (1..5) and cluster size (1..8).
+constexpr int kClusterCap[5][kMaxClusterParts] = {{148, 74, 45, 33, 26, 22, 15, 15},
+                                                  {296, 148, 93, 71, 56, 45, 37, 33},
+                                                  {444, 222, 142, 104, 82, 71, 56, 48},
+                                                  {592, 296, 187, 142, 112, 93, 78, 71},
+                                                  {740, 370, 235, 175, 142, 116, 97, 86}};
+}  // namespace
+
+// A K split in the strided kernel: its last block's merge, and per output of a
+// task the partials written and read.
+constexpr double kSplitLaunchUs = 3.0, kSplitUsPerOutput = 0.6e-3;
+
 bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, StridedPlan* out)
 {
     if (batch <= 0 || p.m <= 0 || p.n <= 0 || p.k <= 0 || (mode != kMode3M && mode != kMode4M)) {
         return false;
     }
+    // The tile and K split with the least estimated time: the one-launch
+    // kernel's model (kSingleCost) without clusters -- a task is a block of its
+    // own -- plus the partials a split leaves in L2 and its last block merges.
     BProblem bp{};
     bp.m = p.m;
     bp.n = p.n;
     bp.k = p.k;
-    const double one = choose_tile(bp, 8192, mode);
-    choose_parts(bp, 4, one * batch / std::max(sm_count, 1));
+    const long long sms = std::max(sm_count, 1);
+    double best = 1e300;
+    for (int t = 1; t < kTileCount; ++t) {
+        const int tm = ceil_div(p.m, tile_bm(t)), tn = ceil_div(p.n, tile_bn(t));
+        const int occ = kSingleOcc[mode == kMode4M ? 1 : 0][t];
+        const SingleCost& c = kSingleCost[t];
+        for (int q = 1; q <= 8; ++q) {
+            const int span = q == 1 ? p.k : span_for(p.k, q);
+            if (q > 1 && (span < 48 || (q - 1) * span >= p.k)) {
+                continue;
+            }
+            const long long tasks = (long long)tm * tn * batch * q;
+            const long long waves = (tasks + sms * occ - 1) / (sms * occ), load = (tasks + sms - 1) / sms;
+            const double fma = (mode == kMode4M ? 4.0 / 3.0 : 1.0) * (load > 1 ? 1.07 : 1.0);
+            double us = c.base_us + (double)waves * c.fixed_us +
+                        span * 1e-3 * fma * ((double)waves * c.term_ns + (double)load * c.shared_term_ns);
+            if (q > 1) {
+                us += kSplitLaunchUs + (double)load * tile_bm(t) * tile_bn(t) * kSplitUsPerOutput;
+            }
+            if (us < best) {
+                best = us;
+                bp.tile = t;
+                bp.tiles_m = tm;
+                bp.tiles_n = tn;
+                bp.parts = q;
+                bp.span = span;
+            }
+        }
+    }
+    // Two tiles per task once every block has many of them: half the trips to
+    // the task counter, and the pair shares op(B)'s columns.
+    const long long rounds =
+        (long long)bp.tiles_m * bp.tiles_n * batch / (3LL * std::max(sm_count, 1));
+    if (mode == kMode3M && bp.tile == 1 && bp.parts == 1 && rounds >= 16) {
+        bp.tile = 0;
+        bp.tiles_m = ceil_div(p.m, tile_bm(0));
+    }
     StridedPlan pl{};
     pl.tile = bp.tile;
     pl.tile_m = tile_bm(bp.tile);
@@ -1053,31 +1224,6 @@ bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, Stri
     *out = pl;
     return true;
 }
-
-int single_tile_bm(int tile) { return tile_bm(tile); }
-int single_tile_bn(int tile) { return tile_bn(tile); }
-
-// Time model of the one-launch kernel (three-product mode), in microseconds,
-// fitted on B200 to 1100 timed (shape, tile, partitions) launches (median
-// error 1.5 %).  Clusters of `parts` blocks run in waves of as many clusters
-// as fit at once (cudaOccupancyMaxActiveClusters on a 148-SM B200, scaled for
-// other SM counts); each wave costs the tile's fixed part (first copies,
-// epilogue) plus span x its per-term time, and tiles that share an SM (64 x 32:
-// two blocks, 32 x 32: three) add a per-term cost for every block on the
-// busiest SM.  The cluster merge costs a little per partition.
-namespace {
-struct SingleCost {
-    double fixed_us, term_ns, shared_term_ns;
-};
-constexpr SingleCost kSingleCost[kTileCount] = {{4.96, 183.8, 0.0},  {3.55, 129.2, 0.0}, {3.31, 176.6, 0.0},
-                                                {3.29, 118.7, 0.0},  {2.99, 51.4, 59.7}, {2.26, 15.3, 43.7}};
-constexpr int kSingleOcc[kTileCount] = {1, 1, 1, 1, 2, 3};
-// Clusters resident at once on 148 SMs, by blocks per SM (1..3) and cluster size (1..8).
-constexpr int kClusterCap[3][kMaxClusterParts] = {{148, 74, 45, 33, 26, 22, 15, 15},
-                                                  {296, 148, 93, 71, 56, 45, 37, 33},
-                                                  {444, 222, 142, 104, 82, 71, 56, 48}};
-constexpr double kSingleMergePerPartUs = 0.146;
-}  // namespace
 
 double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile, int forced_parts, int* tile,
                    int* parts)
@@ -1098,18 +1244,20 @@ double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile,
             if (q > 1 && (q - 1) * span >= k) {
                 continue;
             }
-            const long long cap =
-                std::max<long long>(1, (long long)kClusterCap[kSingleOcc[t] - 1][q - 1] * sm_count / 148);
+            const int occ = kSingleOcc[mode == kMode4M ? 1 : 0][t];
+            const long long cap = std::max<long long>(1, (long long)kClusterCap[occ - 1][q - 1] * sm_count / 148);
+            const long long layer = std::max<long long>(1, (long long)kClusterCap[0][q - 1] * sm_count / 148);
             const long long waves = (tiles + cap - 1) / cap;
-            const long long load = (tiles * q + sm_count - 1) / sm_count;
+            const long long load = (tiles + layer - 1) / layer;
             const SingleCost& c = kSingleCost[t];
             // Four-product mode: four FFMA per output and K term instead of
             // three (the per-term costs scaled by that ratio, not fitted).
-            const double fma = mode == kMode4M ? 4.0 / 3.0 : 1.0;
-            double us = (double)waves * c.fixed_us +
+            // Shared SMs run 7 % above the linear fit, which single layers dominate.
+            const double fma = (mode == kMode4M ? 4.0 / 3.0 : 1.0) * (load > 1 ? 1.07 : 1.0);
+            double us = c.base_us + (double)waves * c.fixed_us +
                         span * 1e-3 * fma * ((double)waves * c.term_ns + (double)load * c.shared_term_ns);
             if (q > 1) {
-                us += kSingleMergePerPartUs * q;
+                us += c.merge_us * q;
             }
             if (us < best) {
                 best = us;
@@ -1197,22 +1345,33 @@ cudaError_t launch_strided(cudaStream_t s, const Problem& p, int mode, int repai
         return e;
     }
     const long long ntasks = (long long)plan.tiles * plan.parts * batch;
-    const int grid = (int)std::min<long long>(ntasks, (long long)std::max(sm_count, 1));
-    if (mode == kMode3M) {
-        e = cudaFuncSetAttribute(strided_kernel<kMode3M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSmemBytes);
-        if (e == cudaSuccess) {
-            strided_kernel<kMode3M><<<grid, kThreads, kSmemBytes, s>>>(proto, sA, sB, sC, batch, plan.partial_stride,
-                                                                       partials, counters);
+    auto run = [&](auto mode_c, auto tile_c) -> cudaError_t {
+        constexpr int M = decltype(mode_c)::value, T = decltype(tile_c)::value;
+        auto kernel = strided_kernel<M, T>;
+        const size_t smem = kStridedSmem<M, T>;
+        const int grid = (int)std::min<long long>(ntasks, (long long)std::max(sm_count, 1) * kStridedBlocks<M, T>);
+        const cudaError_t attr = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (attr == cudaSuccess) {
+            kernel<<<grid, kThreads, smem, s>>>(proto, sA, sB, sC, batch, plan.partial_stride, partials, counters);
         }
-    } else {
-        e = cudaFuncSetAttribute(strided_kernel<kMode4M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSmemBytes);
-        if (e == cudaSuccess) {
-            strided_kernel<kMode4M><<<grid, kThreads, kSmemBytes, s>>>(proto, sA, sB, sC, batch, plan.partial_stride,
-                                                                       partials, counters);
+        return attr;
+    };
+    using std::integral_constant;
+    auto run_mode = [&](auto mode_c) -> cudaError_t {
+        switch (plan.tile) {
+            case 0:
+                if constexpr (decltype(mode_c)::value == kMode3M) {
+                    return run(mode_c, integral_constant<int, 0>{});
+                }
+                return cudaErrorInvalidValue;
+            case 1: return run(mode_c, integral_constant<int, 1>{});
+            case 2: return run(mode_c, integral_constant<int, 2>{});
+            case 3: return run(mode_c, integral_constant<int, 3>{});
+            case 4: return run(mode_c, integral_constant<int, 4>{});
+            default: return run(mode_c, integral_constant<int, 5>{});
         }
-    }
+    };
+    e = mode == kMode3M ? run_mode(integral_constant<int, kMode3M>{}) : run_mode(integral_constant<int, kMode4M>{});
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 

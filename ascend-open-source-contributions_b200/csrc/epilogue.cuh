@@ -51,7 +51,8 @@ __device__ __forceinline__ float2 repair_four_product(const float2* A, int lda, 
 
 // alpha == 1 and beta == 0 store (re, im) unchanged (the reference's fused
 // path writes the merged products directly); beta == 0 never reads C.
-__device__ __forceinline__ float2 epilogue_value(float re, float im, const EpiParams& e, const float2* cptr)
+// `c` is C's value, unused when unit or beta_zero.
+__device__ __forceinline__ float2 epilogue_with(float re, float im, const EpiParams& e, float2 c)
 {
     if (e.unit) {
         return make_float2(re, im);
@@ -59,11 +60,14 @@ __device__ __forceinline__ float2 epilogue_value(float re, float im, const EpiPa
     float xr = __fsub_rn(__fmul_rn(e.ar, re), __fmul_rn(e.ai, im));
     float xi = __fadd_rn(__fmul_rn(e.ar, im), __fmul_rn(e.ai, re));
     if (!e.beta_zero) {
-        const float2 c = *cptr;
         xr = __fadd_rn(xr, __fsub_rn(__fmul_rn(e.br, c.x), __fmul_rn(e.bi, c.y)));
         xi = __fadd_rn(xi, __fadd_rn(__fmul_rn(e.br, c.y), __fmul_rn(e.bi, c.x)));
     }
     return make_float2(xr, xi);
+}
+__device__ __forceinline__ float2 epilogue_value(float re, float im, const EpiParams& e, const float2* cptr)
+{
+    return epilogue_with(re, im, e, e.unit || e.beta_zero ? make_float2(0.0f, 0.0f) : *cptr);
 }
 
 // The epilogue of output (row, col) with the non-finite repair applied first

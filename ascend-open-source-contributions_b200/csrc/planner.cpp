@@ -88,11 +88,11 @@ struct TileChoice {
 // planner splits K over 128 x 64 tiles instead (512^3: 64 x 32 x 3 parts
 // 62.9 us, 128 x 64 x 4 parts 38.8 us; 1024^3: 306 vs 174 us).
 const TileChoice kFp32Tiles[] = {{128, 64, 1}};
-// Cost of one wave of 128 x 64 FP32 tiles in K terms of that tile (0.133 us
-// per term): a fixed part of about 38 terms (pipeline fill, epilogue, wave
-// launch; fitted on 512^3 .. 2048^3) plus the span; the split-K merge costs
-// about 30 terms plus the partial planes it reads.
-constexpr uint64_t kFp32WaveFixed = 38;
+// Cost of one wave of 128 x 64 FP32 tiles in K terms of that tile (0.111 us
+// per term): a fixed part of about 56 terms (pipeline fill, epilogue, wave
+// launch; fitted with the microsecond model below) plus the span; the split-K
+// merge costs about 30 terms plus the partial planes it reads.
+constexpr uint64_t kFp32WaveFixed = 56;
 constexpr uint64_t kMergeFixed = 30;
 constexpr uint64_t kMergeFloatsPerTerm = 41500;
 // With 2..8 partitions the partitions of a tile form one thread-block cluster
@@ -112,13 +112,16 @@ uint64_t fp32_waves(uint64_t tiles, int parts, int sm_count)
     return (tiles * parts + sm_count - 1) / sm_count;
 }
 // The same costs in microseconds for the whole packed call (pack kernel over
-// op(A) and op(B) -- 8 bytes read, 12 written per element -- GEMM waves, merge
-// kernel), fitted on B200 to 28 timed shapes (median error 3.3 %).
-constexpr double kPackedFixedUs = 1.64;
-constexpr double kPackedUsPerMB = 0.199;
-constexpr double kPackedUsPerTerm = 0.1205;
-constexpr double kMergeLaunchUs = 3.53;
-constexpr double kMergeUsPerTerm = 0.0;
+// op(A) and op(B) -- 8 bytes read, 12 written per element -- GEMM waves, merge),
+// fitted on B200 to 460 timed (shape, partitions) calls (median error 1.5 %).
+constexpr double kPackedFixedUs = 2.91;
+constexpr double kPackedUsPerMB = 0.1323;
+constexpr double kPackedUsPerTerm = 0.1113;
+constexpr double kPackedUsPerPart = 0.0857;
+constexpr double kMergeLaunchUs = 2.5;
+// The one-launch engine has to look faster by this much: its model errs by up
+// to 10 % where the two engines meet, the packed one's by 3 %.
+constexpr double kSingleMargin = 1.06;
 // Tensor-core kernel tile (gemm_tc.cu): 128 x 128, one CTA per SM (TMEM).
 const TileChoice kTcTiles[] = {{128, 128, 1}};
 
@@ -150,9 +153,9 @@ double packed_time_us(const Problem& p, int parts, int span, uint64_t tiles, int
     const double bytes = ((double)p.m * p.k + (double)p.k * p.n) * 20.0;
     double us = kPackedFixedUs + kPackedUsPerMB * bytes * 1e-6 + kPackedUsPerTerm * (double)waves * (span + kFp32WaveFixed);
     if (parts > kClusterMergeMax) {
-        us += kMergeLaunchUs + kMergeUsPerTerm * (kMergeFixed + (double)(2 * parts + 2) * p.m * p.n / kMergeFloatsPerTerm);
+        us += kMergeLaunchUs;
     } else if (parts > 1) {
-        us += kPackedUsPerTerm * parts;
+        us += kPackedUsPerPart * parts;
     }
     return us;
 }
@@ -236,7 +239,7 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
         // FP32: waves of 128 x 64 tiles at (span + fixed) each, plus the merge
         // (EstimateCgemmCoreWork's busiest-core work with measured B200 costs).
         uint64_t best = std::numeric_limits<uint64_t>::max();
-        for (int parts = 1; parts <= 32; ++parts) {
+        for (int parts = 1; parts <= 64; ++parts) {
             const int span = k_span(p.k, parts, granule);
             if ((parts - 1) * span >= p.k || (parts > 1 && span < 64)) {
                 continue;
@@ -315,7 +318,7 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
         int tile = 0, parts = 0;
         const double single = plan_single(p.m, p.n, p.k, 0, sm_count, -1, forced, &tile, &parts);
         out.est_us = packed_time_us(p, out.parts, out.span, default_tiles, sm_count);
-        if (single < out.est_us) {
+        if (single * kSingleMargin < out.est_us) {
             out.est_us = single;
             out.engine = 2;
             out.onchip_tile = tile;
