@@ -83,6 +83,8 @@ SIGNATURES = {
                       ctypes.POINTER(cg3mCallInfo)],
     "cg3mCgemm3mStridedBatched": [_P, _I, _I, _I, _I, _I, _CP, _P, _I, ctypes.c_int64, _P, _I, ctypes.c_int64, _CP,
                                   _P, _I, ctypes.c_int64, _I],
+    "cg3mCgemm3mStridedBatchedEx": [_P, _I, _I, _I, _I, _I, _CP, _P, _I, ctypes.c_int64, _P, _I, ctypes.c_int64, _CP,
+                                    _P, _I, ctypes.c_int64, _I, ctypes.POINTER(cg3mOptions)],
     "cg3mCgemm": [_P, _I, _I, _I, _I, _I, _CP, _P, _I, _P, _I, _CP, _P, _I],
     "aclblasCgemm": [_P, _I, _I, _I, _I, _I, _CP, _P, _I, _P, _I, _CP, _P, _I],
     "cg3mCgemm3mHost": [_P, _I, _I, _I, _I, _I, _CP, _P, _I, _P, _I, _CP, _P, _I, ctypes.POINTER(cg3mOptions), _I,
@@ -387,6 +389,42 @@ def default_handle():
     return h
 
 
+def _op_shape(A, B, ta, tb):
+    """(m, n, k) of opt(A) @ opt(B) for the last two dimensions of torch tensors."""
+    (ar, ac), (br, bc) = A.shape[-2:], B.shape[-2:]
+    m, k = (ar, ac) if ta in (0, 3) else (ac, ar)
+    k2, n = (br, bc) if tb in (0, 3) else (bc, br)
+    if k != k2:
+        raise ValueError("inner dimensions differ")
+    return m, n, k
+
+
+def cgemm3m_batched(A, B, transa="N", transb="N", form="fp32"):
+    """``opt(A[i]) @ opt(B[i])`` for complex64 CUDA tensors (batch, rows, cols),
+    without the rounding pass; the whole batch in one launch where that is the
+    faster way (cg3mCgemm3mStridedBatchedEx)."""
+    import torch
+
+    if not (A.is_cuda and B.is_cuda):
+        raise ValueError("cg3m runs on CUDA tensors only")
+    if A.dim() != 3 or B.dim() != 3 or A.shape[0] != B.shape[0]:
+        raise ValueError("expected two 3-D tensors of one batch size")
+    A = A.contiguous()
+    B = B.contiguous()
+    ta, tb = _op(transa), _op(transb)
+    m, n, k = _op_shape(A, B, ta, tb)
+    C = torch.empty((A.shape[0], m, n), dtype=torch.complex64, device=A.device)
+    al, be = cx(1.0), cx(0.0)
+    opts = cg3mOptions(FORM[form] if isinstance(form, str) else form, ROUNDING["off"], 0, 0, 0, 0)
+    h = default_handle()
+    # operands swapped as in cgemm3m: column-major C^T = op(B)^T op(A)^T
+    _check(_lib.cg3mCgemm3mStridedBatchedEx(h.h, tb, ta, n, m, k, ctypes.byref(al), ptr(B), B.shape[2],
+                                            B.shape[1] * B.shape[2], ptr(A), A.shape[2], A.shape[1] * A.shape[2],
+                                            ctypes.byref(be), ptr(C), n, m * n, A.shape[0], ctypes.byref(opts)),
+           "cg3mCgemm3mStridedBatchedEx")
+    return C
+
+
 def cgemm3m(A, B, transa="N", transb="N", alpha=1.0, beta=0.0, C=None, form="fp32", rounding="auto"):
     """Convenience wrapper on torch complex64 tensors in *row-major torch* shape.
 
@@ -402,12 +440,8 @@ def cgemm3m(A, B, transa="N", transb="N", alpha=1.0, beta=0.0, C=None, form="fp3
     A = A.contiguous()
     B = B.contiguous()
     ta, tb = _op(transa), _op(transb)
-    ar, ac = A.shape
-    br, bc = B.shape
-    m, k = (ar, ac) if ta in (0, 3) else (ac, ar)
-    k2, n = (br, bc) if tb in (0, 3) else (bc, br)
-    if k != k2:
-        raise ValueError("inner dimensions differ")
+    (_, ac), (_, bc) = A.shape, B.shape
+    m, n, k = _op_shape(A, B, ta, tb)
     # torch row-major (rows, cols) == column-major (cols, rows): compute
     # C^T = op(B)^T op(A)^T, i.e. swap the operands (the reference's C^T
     # convention, gemm_host_common.h:69-74).

@@ -20,6 +20,7 @@ from __future__ import annotations
 import torch
 
 from . import cgemm3m as _cgemm3m
+from . import cgemm3m_batched as _cgemm3m_batched
 
 _BITS = {"N": (0, 0), "T": (1, 0), "C": (1, 1), "R": (0, 1)}
 _NAMES = {v: k for k, v in _BITS.items()}
@@ -44,6 +45,8 @@ def _mm(X, Y, tx, ty, form):
     """opt(X) @ opt(Y) for 2-D or batched 3-D complex64 tensors."""
     if X.dim() == 2:
         return _cgemm3m(X, Y, tx, ty, form=form, rounding="off")
+    if X.is_cuda and X.dtype == Y.dtype == torch.complex64 and Y.dim() == 3 and X.shape[0] == Y.shape[0] > 0:
+        return _cgemm3m_batched(X, Y, tx, ty, form)
     return torch.stack([_cgemm3m(X[i], Y[i], tx, ty, form=form, rounding="off") for i in range(X.shape[0])])
 
 

@@ -105,6 +105,9 @@ cg3mStatus_t workspace(cg3mContext* h, size_t bytes, void** out)
     return CG3M_STATUS_SUCCESS;
 }
 
+// Operand planes one batched tensor-core launch may hold in the workspace.
+constexpr size_t kBatchPlaneBytes = size_t(1) << 30;
+
 // Options of cg3mCgemm's three-product case: the FP32 drop-in arithmetic, no
 // rounding pass.
 cg3mOptions cgemm_unit_options()
@@ -477,6 +480,123 @@ cg3mStatus_t cg3mCgemm3mStridedBatched(cg3mHandle_t h, cg3mOperation_t transa, c
                                                                per_launch, plan, ws, h->sm_count);
         if (e != cudaSuccess) {
             return to_status(e);
+        }
+    }
+    return CG3M_STATUS_SUCCESS;
+}
+
+cg3mStatus_t cg3mCgemm3mStridedBatchedEx(cg3mHandle_t h, cg3mOperation_t transa, cg3mOperation_t transb, int m,
+                                         int n, int k, const cg3mComplex* alpha, const cg3mComplex* A, int lda,
+                                         int64_t strideA, const cg3mComplex* B, int ldb, int64_t strideB,
+                                         const cg3mComplex* beta, cg3mComplex* C, int ldc, int64_t strideC,
+                                         int batch_count, const cg3mOptions* opts_in)
+{
+    if (h == nullptr) {
+        return CG3M_STATUS_HANDLE_IS_NULLPTR;
+    }
+    if (batch_count < 0) {
+        return CG3M_STATUS_INVALID_VALUE;
+    }
+    if (batch_count == 0) {
+        return CG3M_STATUS_SUCCESS;
+    }
+    cg3mOptions opts{};
+    if (opts_in != nullptr) {
+        opts = *opts_in;
+    }
+    int action = 0;
+    const cg3mStatus_t st =
+        validate(transa, transb, m, n, k, alpha, A, lda, B, ldb, beta, C, ldc, true, &action);
+    if (st != CG3M_STATUS_SUCCESS || action == 0) {
+        return st;
+    }
+    if (opts.form < CG3M_FORM_FP32 || opts.form > CG3M_FORM_BF16X9) {
+        return CG3M_STATUS_INVALID_VALUE;
+    }
+    const cg3mStatus_t bs = bind_device(h);
+    if (bs != CG3M_STATUS_SUCCESS) {
+        return bs;
+    }
+    // One launch for the batch when the calls would run the planner's plain
+    // choice (no forced split or engine, no rounding pass) and the outputs do
+    // not overlap; of that launch and the calls one by one, the faster by the
+    // planner's estimates.
+    const long long span_c = (long long)(n - 1) * ldc + m;
+    const bool apart = (strideC < 0 ? -strideC : strideC) >= span_c;
+    Problem p{transa, transb, m, n, k, alpha->real, alpha->imag, beta->real, beta->imag, A, lda, B, ldb, C, ldc};
+    Plan one;
+    const bool tc = opts.form != CG3M_FORM_FP32;
+    if (batch_count > 1 && action == 2 && apart && opts.k_partitions == 0 &&
+        (opts.engine == 0 || (tc && opts.engine == 1)) && h->stage_event_count == 0 &&
+        make_plan(p, opts, h->sm_count, &one) && !one.rounding) {
+        double best = one.est_us * batch_count;
+        StridedPlan strided;
+        const bool onchip = opts.engine == 0 && make_strided_plan(p, 0, batch_count, h->sm_count, &strided) &&
+                            strided.est_us * (tc ? 1.1 : 1.0) < best;
+        if (onchip) {
+            best = strided.est_us * (tc ? 1.1 : 1.0);
+        }
+        if (tc && m > 128 && batch_tc_time_us(p, opts.form, h->sm_count, batch_count) < best) {
+            // As many problems per launch as fit kBatchPlaneBytes of planes (at
+            // least one), in even chunks; fewer when the device has no room.
+            Plan plan;
+            int chunk = std::min(batch_count, 32768);  // a grid dimension
+            if (!batch_tc_plan(p, opts, h->sm_count, 1, &plan)) {
+                return CG3M_STATUS_INVALID_VALUE;
+            }
+            const size_t room = kBatchPlaneBytes / std::max<size_t>(plan.total, 1);
+            if ((size_t)chunk > std::max<size_t>(room, 1)) {
+                const int chunks = ceil_div(batch_count, (int)std::max<size_t>(room, 1));
+                chunk = ceil_div(batch_count, chunks);
+            }
+            void* ws = nullptr;
+            cg3mStatus_t wst = CG3M_STATUS_ALLOC_FAILED;
+            for (;; chunk = (chunk + 1) / 2) {
+                if (!batch_tc_plan(p, opts, h->sm_count, chunk, &plan)) {
+                    return CG3M_STATUS_INVALID_VALUE;
+                }
+                wst = workspace(h, plan.total, &ws);
+                if (wst != CG3M_STATUS_ALLOC_FAILED || chunk == 1) {
+                    break;
+                }
+                cudaGetLastError();
+            }
+            if (wst != CG3M_STATUS_SUCCESS) {
+                return wst;
+            }
+            h->round_stats = nullptr;
+            for (int i = 0; i < batch_count; i += chunk) {
+                const BatchStrides bst{std::min(chunk, batch_count - i), strideA, strideB, strideC};
+                Problem pi = p;
+                pi.A = A + i * strideA;
+                pi.B = B + i * strideB;
+                pi.C = C + i * strideC;
+                cudaError_t e = launch_pack(h->stream, pi, plan, ws, nullptr, nullptr, bst);
+                if (e == cudaSuccess) {
+                    e = launch_gemm_tc_batch(h->stream, pi, plan, ws, h->status, bst);
+                }
+                if (e != cudaSuccess) {
+                    return to_status(e);
+                }
+            }
+            return CG3M_STATUS_SUCCESS;
+        }
+        if (onchip) {
+            void* ws = nullptr;
+            const cg3mStatus_t wst = workspace(h, strided.bytes, &ws);
+            if (wst != CG3M_STATUS_SUCCESS) {
+                return wst;
+            }
+            h->round_stats = nullptr;
+            return to_status(launch_strided(h->stream, p, 0, 0, strideA, strideB, strideC, batch_count, strided, ws,
+                                            h->sm_count));
+        }
+    }
+    for (int i = 0; i < batch_count; ++i) {
+        const cg3mStatus_t s = run_one(h, transa, transb, m, n, k, alpha, A + i * strideA, lda, B + i * strideB, ldb,
+                                       beta, C + i * strideC, ldc, opts, true, nullptr);
+        if (s != CG3M_STATUS_SUCCESS) {
+            return s;
         }
     }
     return CG3M_STATUS_SUCCESS;

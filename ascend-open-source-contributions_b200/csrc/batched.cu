@@ -1213,6 +1213,7 @@ bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, Stri
     pl.tile = bp.tile;
     pl.tile_m = tile_bm(bp.tile);
     pl.tile_n = tile_bn(bp.tile);
+    pl.est_us = best;
     pl.parts = bp.parts;
     pl.span = bp.span;
     pl.tiles = bp.tiles_m * bp.tiles_n;

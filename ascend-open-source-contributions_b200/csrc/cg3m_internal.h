@@ -36,6 +36,13 @@ namespace cg3m {
 constexpr size_t kDefaultWorkspaceBytes = size_t(32) << 20;  // cann_ops_blas.h:33-35
 constexpr size_t kRegionAlign = 512;                          // cgemm_host.cpp:33 (16 x 32 B)
 
+// Equal problems of one launch at element strides a, b, c (operand planes of
+// problem i follow those of problem i - 1).
+struct BatchStrides {
+    int count = 1;
+    long long a = 0, b = 0, c = 0;
+};
+
 // Which plane layout a GEMM kernel consumes.
 enum class Layout { MnMajor, KMajor };
 
@@ -54,7 +61,7 @@ struct Plan {
     int onchip_tile = 0;     // engine 2: tile index of the on-chip family (0 128x64 .. 5 32x32)
     bool cluster_merge = false;  // FP32 packed engine: the K partitions (2..8) merge inside their cluster
     bool repair = false;         // cg3mCgemm, alpha = 1, beta = 0: non-finite outputs repaired in the epilogue
-    double est_us = 0.0;         // FP32 plans: the planner's time estimate (microseconds)
+    double est_us = 0.0;         // the planner's time estimate (microseconds; without the rounding pass)
     // workspace layout (byte offsets from the workspace base)
     size_t planes_a_off = 0, planes_b_off = 0, partial_off = 0, round_off = 0, total = 0;
     int pitch_a = 0, pitch_b = 0;  // elements per plane row
@@ -96,9 +103,19 @@ cudaError_t launch_beta_scale(cudaStream_t s, int m, int n, float br, float bi, 
 // packed rows did not (all but the leading term of re and im), and only for the
 // 256-row bands of op(A) rows / op(B) columns whose byte is nonzero.
 cudaError_t launch_pack(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const uint8_t* band_a = nullptr,
-                        const uint8_t* band_b = nullptr);
+                        const uint8_t* band_b = nullptr, const BatchStrides& batch = BatchStrides{});
 cudaError_t launch_gemm_fp32(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status);
 cudaError_t launch_gemm_tc(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status);
+// `batch` equal problems on the CTA-pair kernel in one launch (m > 128, unsplit
+// along K), planes packed by launch_pack with the same strides; the plan is
+// batch_tc_plan's.
+cudaError_t launch_gemm_tc_batch(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status,
+                                 const BatchStrides& batch);
+// The tensor-core plan of `count` equal problems in one launch (workspace laid
+// out for all of them), and its estimated time in microseconds; false when the
+// shape has one 128-row tile only.
+bool batch_tc_plan(const Problem& p, const cg3mOptions& opts, int sm_count, int count, Plan* plan);
+double batch_tc_time_us(const Problem& p, int form, int sm_count, int count);
 cudaError_t launch_merge(cudaStream_t s, const Problem& p, const Plan& plan, void* ws);
 // The rounding-correction pass.  Tensor-core forms start the call with the
 // packed rows, which also write the leading split planes the risk-plane GEMM
@@ -208,6 +225,7 @@ struct StridedPlan {
     size_t counters = 0;        // task counter + tile counters (uint32)
     size_t partial_off = 0;     // byte offset of the partials in the workspace
     size_t bytes = 0;           // workspace bytes
+    double est_us = 0.0;        // estimated time
 };
 bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, StridedPlan* out);
 // One problem in one launch of the on-chip family: grid (tiles, parts), the

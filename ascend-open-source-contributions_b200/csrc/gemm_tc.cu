@@ -174,6 +174,7 @@ struct TcParams {
     int* status;
     int seg_blocks;  // K-blocks per accumulation segment
     int cluster_merge;  // pair kernel: the `parts` pairs of a tile form one cluster and merge on chip
+    long long c_batch;  // pair kernel: blockIdx.z is the problem of a batch, its C at c_batch elements each
     // pair kernel in the rounding pass: the per-16 x 16 flagged counts; pair
     // tiles inside a 256 x 256 tile the exact recompute takes are skipped
     const uint32_t* skip_count;
@@ -908,6 +909,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int kblocks = (kend - kbeg + Cfg::BK - 1) / Cfg::BK;
     const int seg_blocks = p.seg_blocks;
     const int segments = (kblocks + seg_blocks - 1) / seg_blocks;
+    const int z0 = (int)blockIdx.z * 3 * Cfg::ZS;  // first plane of this problem
+    float2* const C = p.C + (long long)blockIdx.z * p.c_batch;
 
     if (p.skip_count != nullptr) {
         // Rounding pass: the exact recompute writes every output of the
@@ -980,9 +983,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                         if (leader) {
                             mbar_arrive_expect_tx(&full[s], 2 * STAGE_BYTES);
                         }
-                        tma_load_3d_pair(st, &tmA, bar, kbeg + kb * Cfg::BK, m0, c * Cfg::ZS);
+                        tma_load_3d_pair(st, &tmA, bar, kbeg + kb * Cfg::BK, m0, z0 + c * Cfg::ZS);
                         tma_load_3d_pair(st + Cfg::S * A_PLANE, &tmB, bar, kbeg + kb * Cfg::BK,
-                                         n0 + (int)rank * PAIR_BHALF, c * Cfg::ZS);
+                                         n0 + (int)rank * PAIR_BHALF, z0 + c * Cfg::ZS);
                     }
                 }
             }
@@ -1139,7 +1142,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 const int col = n0 + group * COLS + j;
                 if (col < p.n) {
                     if (p.parts == 1) {
-                        float2* cp = p.C + (size_t)col * p.ldc + row;
+                        float2* cp = C + (size_t)col * p.ldc + row;
                         *cp = epilogue_value(re[j], im[j], p.epi, cp);
                     } else {
                         const size_t o = (size_t)col * p.ppitch + row;
@@ -1182,7 +1185,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     vre = __fadd_rn(vre, ld_dsmem_f32(mapa_shared(re_local + 4u * e, peer)));
                     vim = __fadd_rn(vim, ld_dsmem_f32(mapa_shared(im_local + 4u * e, peer)));
                 }
-                float2* cp = p.C + (size_t)col * p.ldc + row;
+                float2* cp = C + (size_t)col * p.ldc + row;
                 *cp = epilogue_value(vre, vim, p.epi, cp);
             }
         }
@@ -1196,7 +1199,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 template <int FORM>
 cudaError_t launch_pair(cudaStream_t stream, const Problem& pr, const Plan& plan, void* ws, int* status,
-                        const uint32_t* skip_count = nullptr)
+                        const uint32_t* skip_count = nullptr, const BatchStrides& batch = BatchStrides{})
 {
     using Cfg = TcCfg<FORM>;
     using G = PairGeom<FORM>;
@@ -1206,7 +1209,7 @@ cudaError_t launch_pair(cudaStream_t stream, const Problem& pr, const Plan& plan
     CUtensorMap ta, tb;
     const CUtensorMapDataType dt = bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
     {
-        const uint64_t dims[3] = {(uint64_t)pr.k, (uint64_t)pr.m, (uint64_t)(3 * Cfg::ZS)};
+        const uint64_t dims[3] = {(uint64_t)pr.k, (uint64_t)pr.m, (uint64_t)batch.count * 3 * Cfg::ZS};
         const uint64_t strides[2] = {(uint64_t)plan.pitch_a * elem, (uint64_t)plan.plane_a_elems * elem};
         const uint32_t box[3] = {(uint32_t)Cfg::BK, (uint32_t)TILE_M, (uint32_t)Cfg::S};
         if (!encode_tensor_map(&ta, dt, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, w + plan.planes_a_off)) {
@@ -1214,7 +1217,7 @@ cudaError_t launch_pair(cudaStream_t stream, const Problem& pr, const Plan& plan
         }
     }
     {
-        const uint64_t dims[3] = {(uint64_t)pr.k, (uint64_t)pr.n, (uint64_t)(3 * Cfg::ZS)};
+        const uint64_t dims[3] = {(uint64_t)pr.k, (uint64_t)pr.n, (uint64_t)batch.count * 3 * Cfg::ZS};
         const uint64_t strides[2] = {(uint64_t)plan.pitch_b * elem, (uint64_t)plan.plane_b_elems * elem};
         const uint32_t box[3] = {(uint32_t)Cfg::BK, (uint32_t)PAIR_BHALF, (uint32_t)Cfg::S};
         if (!encode_tensor_map(&tb, dt, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, w + plan.planes_b_off)) {
@@ -1241,6 +1244,7 @@ cudaError_t launch_pair(cudaStream_t stream, const Problem& pr, const Plan& plan
         p.seg_blocks = 1;
     }
     p.skip_count = skip_count;
+    p.c_batch = batch.c;
     p.cluster_merge = plan.cluster_merge ? 1 : 0;
     if (p.cluster_merge && (plan.parts < 2 || plan.parts > 4)) {
         return cudaErrorInvalidValue;  // clusters of at most 8 CTAs: up to 4 pairs
@@ -1253,7 +1257,7 @@ cudaError_t launch_pair(cudaStream_t stream, const Problem& pr, const Plan& plan
         return err;
     }
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(2 * p.tiles_m * p.tiles_n), (unsigned)plan.parts);
+    cfg.gridDim = dim3((unsigned)(2 * p.tiles_m * p.tiles_n), (unsigned)plan.parts, (unsigned)batch.count);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = G::SMEM;
     cfg.stream = stream;
@@ -1402,6 +1406,20 @@ cudaError_t launch_gemm_tc(cudaStream_t stream, const Problem& pr, const Plan& p
         case CG3M_FORM_TF32X3: return launch_form<CG3M_FORM_TF32X3, 128>(stream, pr, plan, ws, status);
         case CG3M_FORM_BF16X6: return launch_form<CG3M_FORM_BF16X6, 128>(stream, pr, plan, ws, status);
         case CG3M_FORM_BF16X9: return launch_form<CG3M_FORM_BF16X9, 128>(stream, pr, plan, ws, status);
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+cudaError_t launch_gemm_tc_batch(cudaStream_t stream, const Problem& pr, const Plan& plan, void* ws, int* status,
+                                 const BatchStrides& batch)
+{
+    if (pr.m <= TILE_M || plan.parts != 1 || plan.cluster_merge) {
+        return cudaErrorInvalidValue;
+    }
+    switch (plan.form) {
+        case CG3M_FORM_TF32X3: return launch_pair<CG3M_FORM_TF32X3>(stream, pr, plan, ws, status, nullptr, batch);
+        case CG3M_FORM_BF16X6: return launch_pair<CG3M_FORM_BF16X6>(stream, pr, plan, ws, status, nullptr, batch);
+        case CG3M_FORM_BF16X9: return launch_pair<CG3M_FORM_BF16X9>(stream, pr, plan, ws, status, nullptr, batch);
         default: return cudaErrorInvalidValue;
     }
 }

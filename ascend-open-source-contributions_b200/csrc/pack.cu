@@ -38,6 +38,10 @@ struct PackSide {
     void* lead;
     int lead_pitch;
     size_t lead_plane_elems;
+    // Equal problems of one launch (blockIdx.y): strides of the source in
+    // elements and of the planes in bytes.
+    long long src_batch;
+    size_t out_batch;
     // The rest of the planes (same pass): per 256-row band of the plane rows,
     // nonzero when a 256 x 256 tile of that band is left to the form's products.
     const uint8_t* band_need;
@@ -129,7 +133,9 @@ __global__ void __launch_bounds__(TILE* ROWS) pack_kernel(PackSide a, PackSide b
     // launches no blocks over the other side's extent.  The full packs launch
     // one block per tile; the rest of the planes in the rounding pass uses a
     // smaller grid, as most of its tiles may lie in bands it skips.
-    const PackSide& s = blockIdx.z == 0 ? a : b;
+    PackSide s = blockIdx.z == 0 ? a : b;
+    s.src += (long long)blockIdx.y * s.src_batch;
+    s.out = static_cast<uint8_t*>(s.out) + blockIdx.y * s.out_batch;
     const int tiles_r = (s.rows + TILE - 1) / TILE;
     const long long tiles = (long long)tiles_r * ((s.cols + TILE - 1) / TILE);
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -234,9 +240,10 @@ cudaError_t launch_pack_rows(cudaStream_t stream, const Problem& p, void* rows_a
 }
 
 cudaError_t launch_pack(cudaStream_t stream, const Problem& p, const Plan& plan, void* ws, const uint8_t* band_a,
-                        const uint8_t* band_b)
+                        const uint8_t* band_b, const BatchStrides& batch)
 {
     const bool kmajor = plan.form != CG3M_FORM_FP32;
+    const size_t elem = plan.form == CG3M_FORM_BF16X6 || plan.form == CG3M_FORM_BF16X9 ? 2 : 4;
     auto side = [&](bool isA) {
         PackSide s{};
         const int op = isA ? p.transa : p.transb;
@@ -257,10 +264,12 @@ cudaError_t launch_pack(cudaStream_t stream, const Problem& p, const Plan& plan,
         s.pitch = isA ? plan.pitch_a : plan.pitch_b;
         s.plane_elems = isA ? plan.plane_a_elems : plan.plane_b_elems;
         s.band_need = isA ? band_a : band_b;
+        s.src_batch = isA ? batch.a : batch.b;
+        s.out_batch = (size_t)plan.planes * s.plane_elems * elem;
         return s;
     };
     const PackSide a = side(true), b = side(false);
-    const dim3 grid(pack_blocks(a, b), 1, 2), block(TILE, ROWS);
+    const dim3 grid(pack_blocks(a, b), (unsigned)batch.count, 2), block(TILE, ROWS);
     if (band_a != nullptr) {
         // the rest of the tensor-core planes, for the bands the form's products read
         const dim3 rest_grid(grid.x < 148u * 8u ? grid.x : 148u * 8u, 1, 2);

@@ -16,6 +16,7 @@
 // with how few tiles there are, since a 148-SM part needs far more
 // independent tasks than a 1-4-way split of a handful of tiles provides.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <limits>
 
@@ -178,6 +179,37 @@ double tc_time_us(const Problem& p, int form, int parts, int span, int sm_count)
 
 }  // namespace
 
+// One launch of `count` equal problems on the CTA-pair kernel: the pack at
+// 5.5 TB/s, then waves of sm_count / 2 pair tiles (256 x 128) whose time per K
+// term is that of full waves at 3072^3 and 4096^3 (bound by L2 and the power
+// limit).
+double batch_tc_time_us(const Problem& p, int form, int sm_count, int count)
+{
+    const double pairs = std::max(1, sm_count / 2);
+    const double tiles = (double)ceil_div(p.m, 256) * ceil_div(p.n, 128) * count;
+    const double elems = ((double)p.m * p.k + (double)p.k * p.n) * count;
+    const double bytes = form == CG3M_FORM_TF32X3 ? 32.0 : 26.0;
+    const double term = form == CG3M_FORM_TF32X3 ? 0.058 : form == CG3M_FORM_BF16X9 ? 0.078 : 0.057;
+    return 14.0 + elems * bytes / 5.5e6 + std::ceil(tiles / pairs) * ((double)align_up((size_t)p.k, 64) * term + 4.0);
+}
+
+bool batch_tc_plan(const Problem& p, const cg3mOptions& opts, int sm_count, int count, Plan* plan)
+{
+    cg3mOptions o = opts;
+    o.engine = 1;
+    o.k_partitions = 1;
+    o.rounding = CG3M_ROUNDING_OFF;
+    if (p.m <= 128 || opts.form == CG3M_FORM_FP32 || !make_plan(p, o, sm_count, plan)) {
+        return false;
+    }
+    const size_t elem = opts.form == CG3M_FORM_TF32X3 ? 4 : 2;
+    plan->planes_a_off = 0;
+    plan->planes_b_off = align_up(plan->plane_a_elems * elem * plan->planes * count, kRegionAlign);
+    plan->total = align_up(plan->planes_b_off + plan->plane_b_elems * elem * plan->planes * count, kRegionAlign);
+    plan->guards = 0;
+    return true;
+}
+
 bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* plan)
 {
     Plan out{};
@@ -339,13 +371,15 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
     // model), the call runs that plan in plain FP32 -- its error is the plain
     // form's, which every form promises not to exceed -- and reports form
     // FP32.  engine 1 (or a forced K split) keeps the tensor-core path.
+    if (tc) {
+        out.est_us = tc_time_us(p, opts.form, out.parts, out.span, sm_count);
+    }
     if (tc && !out.rounding && opts.engine == 0 && opts.k_partitions <= 0) {
         cg3mOptions fo = opts;
         fo.form = CG3M_FORM_FP32;
         fo.rounding = CG3M_ROUNDING_OFF;
         Plan fp;
-        if (make_plan(p, fo, sm_count, &fp) && fp.est_us * 1.1 < tc_time_us(p, opts.form, out.parts, out.span,
-                                                                              sm_count)) {
+        if (make_plan(p, fo, sm_count, &fp) && fp.est_us * 1.1 < out.est_us) {
             *plan = fp;
             return true;
         }

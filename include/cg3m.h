@@ -189,6 +189,22 @@ cg3mStatus_t cg3mCgemm3mStridedBatched(cg3mHandle_t handle, cg3mOperation_t tran
                                        const cg3mComplex* beta, cg3mComplex* C, int ldc, int64_t strideC,
                                        int batch_count);
 
+/* batch_count calls of cg3mCgemm3mEx on equal shapes, X_i = X + i*strideX
+ * (complex elements), with the extended entry points' options and op codes (R
+ * included) and without the non-finite repair of the strided API above.  When
+ * the outputs do not overlap and no split, engine or rounding pass is asked
+ * for, the batch runs as one launch (tensor-core forms: one pack and one GEMM
+ * over all problems, unsplit along K, the operand planes of at most 1 GiB of
+ * problems at a time; or one launch of the on-chip FP32 family) where the
+ * planner estimates that faster than the calls one by one; the K split, and
+ * with it the last bits, may then differ from the single call's.  Validated
+ * once, with the first matrices. */
+cg3mStatus_t cg3mCgemm3mStridedBatchedEx(cg3mHandle_t handle, cg3mOperation_t transa, cg3mOperation_t transb, int m,
+                                         int n, int k, const cg3mComplex* alpha, const cg3mComplex* A, int lda,
+                                         int64_t strideA, const cg3mComplex* B, int ldb, int64_t strideB,
+                                         const cg3mComplex* beta, cg3mComplex* C, int ldc, int64_t strideC,
+                                         int batch_count, const cg3mOptions* opts);
+
 /* One problem of a heterogeneous batch (device pointers, host scalars). */
 typedef struct {
     int transa, transb;
