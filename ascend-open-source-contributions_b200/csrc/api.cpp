@@ -208,8 +208,10 @@ cudaError_t device_malloc(void** p, size_t bytes)
 }
 
 cudaError_t enqueue(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status, int* kernels,
-                    const cudaEvent_t* events, int nevents)
+                    const cudaEvent_t* events, int nevents, const ColPanel* panel)
 {
+    const ColPanel whole{0, p.n, 0};
+    const ColPanel& cols = panel != nullptr ? *panel : whole;
     auto record = [&](int idx, cudaStream_t st) {
         if (events != nullptr && idx >= 0 && idx < nevents && events[idx] != nullptr) {
             cudaEventRecord(events[idx], st);
@@ -254,14 +256,14 @@ cudaError_t enqueue(cudaStream_t s, const Problem& p, const Plan& plan, void* ws
         auto mark = run_marks(0, main_len, s);
         if (tc_round) {
             // the rest of the planes is packed after the selection
-            err = launch_rounding_pack(s, p, plan, ws, [&]() { mark(++count); });
+            err = launch_rounding_pack(s, p, plan, ws, cols, [&]() { mark(++count); });
         } else {
             err = launch_pack(s, p, plan, ws);
             mark(++count);
         }
         if (err == cudaSuccess) {
             if (plan.rounding) {
-                err = launch_gemm_with_path(s, p, plan, ws, status);
+                err = launch_gemm_with_path(s, p, plan, ws, cols, status);
             } else {
                 err = plan.form == CG3M_FORM_FP32 ? launch_gemm_fp32(s, p, plan, ws, status)
                                                   : launch_gemm_tc(s, p, plan, ws, status);
@@ -274,11 +276,11 @@ cudaError_t enqueue(cudaStream_t s, const Problem& p, const Plan& plan, void* ws
         }
     }
     if (err == cudaSuccess && plan.rounding) {
-        err = launch_rounding_prep(s, p, plan, ws, &prep_launched, run_marks(count, prep_len, s));
+        err = launch_rounding_prep(s, p, plan, ws, cols, &prep_launched, run_marks(count, prep_len, s));
         count += prep_launched;
         if (err == cudaSuccess) {
             int launched = 0;
-            err = launch_rounding_finish(s, p, plan, ws, status, &launched, run_marks(count, 64, s));
+            err = launch_rounding_finish(s, p, plan, ws, cols, status, &launched, run_marks(count, 64, s));
             count += launched;
         }
     }
@@ -703,6 +705,7 @@ cg3mStatus_t cg3mCgemm3mHost(cg3mHandle_t h, cg3mOperation_t transa, cg3mOperati
     // Panel width: whole output tiles of the whole problem's plan, with the
     // whole problem's K split for every panel (same bits as one call).
     int tile_n = 64;
+    Plan pass;  // tensor-core forms with the rounding pass: the whole problem's plan, run panel by panel
     if (product) {
         Problem whole{transa, transb, m, n, k, alpha->real, alpha->imag, beta->real, beta->imag, A, lda, B, ldb, C,
                       ldc};
@@ -715,8 +718,10 @@ cg3mStatus_t cg3mCgemm3mHost(cg3mHandle_t h, cg3mOperation_t transa, cg3mOperati
         }
         o.form = static_cast<cg3mForm_t>(plan.form);  // a small tensor-core call may run as plain FP32
         tile_n = plan.tile_n;
-        if (plan.rounding) {
+        if (plan.rounding && plan.form == CG3M_FORM_FP32) {
             panels = 1;
+        } else if (plan.rounding) {
+            pass = plan;
         }
     }
     if (panels <= 0) {
@@ -724,7 +729,11 @@ cg3mStatus_t cg3mCgemm3mHost(cg3mHandle_t h, cg3mOperation_t transa, cg3mOperati
         panels = ceil_div(n, per);
     }
     panels = std::max(1, std::min(panels, n));
-    const int nb = ceil_div(n, panels);
+    int nb = ceil_div(n, panels);
+    if (pass.rounding) {
+        // Whole exact tiles, two to a panel at least: the exact products pair them.
+        nb = std::max(std::min(2 * kOzakiTile, n), ceil_div(nb, kOzakiTile) * kOzakiTile);
+    }
     panels = ceil_div(n, nb);
 
     // Device copies with the caller's leading dimensions.
@@ -788,6 +797,10 @@ cg3mStatus_t cg3mCgemm3mHost(cg3mHandle_t h, cg3mOperation_t transa, cg3mOperati
     }
     cg3mStatus_t result = to_status(err);
     int kernels = 0;
+    void* pass_ws = nullptr;
+    if (pass.rounding && result == CG3M_STATUS_SUCCESS) {
+        result = workspace(h, pass.total, &pass_ws);
+    }
     for (int j = 0; j < panels && result == CG3M_STATUS_SUCCESS; ++j) {
         const int j0 = j * nb, w = std::min(nb, n - j0);
         err = cudaStreamWaitEvent(h->stream, ev_a, 0);
@@ -798,8 +811,25 @@ cg3mStatus_t cg3mCgemm3mHost(cg3mHandle_t h, cg3mOperation_t transa, cg3mOperati
         }
         cg3mCallInfo pi{};
         const cg3mComplex* bj = product ? (b_normal ? dB + (size_t)j0 * ldb : dB + j0) : nullptr;
-        result = run_one(h, transa, transb, m, w, k, alpha, product ? dA : nullptr, lda, bj, ldb, beta,
+        if (pass.rounding) {
+            const Problem dev{transa, transb, m, n, k, alpha->real, alpha->imag, beta->real, beta->imag, dA, lda, dB,
+                              ldb, dC, ldc};
+            const ColPanel cols{j0, j0 + w, j};
+            result = to_status(enqueue(h->stream, dev, pass, pass_ws, h->status, &pi.kernels,
+                                       j == 0 ? h->stage_events : nullptr, j == 0 ? h->stage_event_count : 0, &cols));
+            pi.path = 2;
+            pi.form = pass.form;
+            pi.tile_m = pass.tile_m;
+            pi.tile_n = pass.tile_n;
+            pi.k_partitions = pass.parts;
+            pi.k_span = pass.span;
+            pi.rounding = 1;
+            pi.workspace_bytes = pass.total;
+            h->round_stats = rounding_stats_ptr(pass, pass_ws, n);
+        } else {
+            result = run_one(h, transa, transb, m, w, k, alpha, product ? dA : nullptr, lda, bj, ldb, beta,
                          dC + (size_t)j0 * ldc, ldc, o, true, &pi);
+        }
         if (result != CG3M_STATUS_SUCCESS) {
             break;
         }

@@ -43,6 +43,16 @@ struct BatchStrides {
     long long a = 0, b = 0, c = 0;
 };
 
+// Output columns [j0, j1) of a call in the tensor-core forms' rounding pass,
+// which decides and recomputes every output by itself: the host-buffer entry
+// point runs it panel by panel while the next panel uploads.  j0 is a multiple
+// of kOzakiTile, and so is j1 unless it is the last column; panels run in order,
+// panel 0 also prepares op(A).
+constexpr int kMaxPanels = 16;
+struct ColPanel {
+    int j0, j1, index;
+};
+
 // Which plane layout a GEMM kernel consumes.
 enum class Layout { MnMajor, KMajor };
 
@@ -103,7 +113,8 @@ cudaError_t launch_beta_scale(cudaStream_t s, int m, int n, float br, float bi, 
 // packed rows did not (all but the leading term of re and im), and only for the
 // 256-row bands of op(A) rows / op(B) columns whose byte is nonzero.
 cudaError_t launch_pack(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const uint8_t* band_a = nullptr,
-                        const uint8_t* band_b = nullptr, const BatchStrides& batch = BatchStrides{});
+                        const uint8_t* band_b = nullptr, const BatchStrides& batch = BatchStrides{},
+                        const ColPanel* panel = nullptr);
 cudaError_t launch_gemm_fp32(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status);
 cudaError_t launch_gemm_tc(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status);
 // `batch` equal problems on the CTA-pair kernel in one launch (m > 128, unsplit
@@ -127,7 +138,7 @@ cudaError_t launch_merge(cudaStream_t s, const Problem& p, const Plan& plan, voi
 // epilogue, and they pack the rest of their planes in the finish, for the
 // bands whose tiles the exact recompute leaves to the form).  mark(i) is
 // called after the i-th kernel of each half (1-based) is enqueued.
-cudaError_t launch_rounding_pack(cudaStream_t s, const Problem& p, const Plan& plan, void* ws,
+cudaError_t launch_rounding_pack(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const ColPanel& panel,
                                  const std::function<void()>& mark);
 // The tensor-core forms' risk-plane GEMM applies the selection in its
 // epilogue: these are the selection's inputs and outputs.
@@ -139,19 +150,21 @@ struct LeadSelect {
     uint32_t* stats;
 };
 int rounding_prep_kernels(int form);
-cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* launched,
-                                 const std::function<void(int)>& mark);
-cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status,
-                                   int* launched, const std::function<void(int)>& mark);
+cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const ColPanel& panel,
+                                 int* launched, const std::function<void(int)>& mark);
+cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan& plan, void* ws,
+                                   const ColPanel& panel, int* status, int* launched,
+                                   const std::function<void(int)>& mark);
 // GEMM that also writes the risk plane used by the rounding-correction pass
 // (the tensor-core forms: one pass over the leading split planes, whose C the
 // pass then replaces everywhere).
-cudaError_t launch_gemm_with_path(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status);
+cudaError_t launch_gemm_with_path(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const ColPanel& panel,
+                                  int* status);
 // Tensor-core forms in the rounding pass: the form's own products on every
 // 256 x 128 pair tile outside the tiles the exact recompute takes (tile_count:
 // the pass's per-16 x 16 flagged counts).
-cudaError_t launch_gemm_tc_tiles(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status,
-                                 const uint32_t* tile_count);
+cudaError_t launch_gemm_tc_tiles(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const ColPanel& panel,
+                                 int* status, const uint32_t* tile_count);
 // Rounding pass: a 16 x 16 tile with more flagged outputs than this is
 // recomputed as part of a tile; sparser tiles have each flagged output
 // recomputed on its own.  Counters it leaves beside the flags:
@@ -190,13 +203,17 @@ struct OzLayout {
 };
 OzLayout oz_layout(int n, uint8_t* base, std::vector<size_t>* guards = nullptr);
 // Residues of op(A) rows and op(B) columns (needs only the packed rows).
-cudaError_t launch_ozaki_split(cudaStream_t s, int n, int pitch, const float2* rows_a, const float2* rows_b,
-                               const OzLayout& L);
+cudaError_t launch_ozaki_split(cudaStream_t s, int n, int pitch, const ColPanel& panel, const float2* rows_a,
+                               const float2* rows_b, const OzLayout& L);
 // The exact products of every tile marked in L.tile_ran and their
 // reconstruction into every output of those tiles; outputs it cannot certify
 // are marked in fallback_bits.  Two launches; mark(i) after the i-th (1-based).
-cudaError_t launch_ozaki_tiles(cudaStream_t s, int n, const OzLayout& L, uint32_t* stats, uint32_t* fallback_bits,
-                               float2* C, int* status, int* launched, const std::function<void(int)>& mark);
+cudaError_t launch_ozaki_tiles(cudaStream_t s, int n, const ColPanel& panel, const OzLayout& L, uint32_t* stats,
+                               uint32_t* fallback_bits, float2* C, int* status, int* launched,
+                               const std::function<void(int)>& mark);
+// Row r of 2 n (op(A) rows, then op(B) columns) that block b of a per-row kernel
+// takes when it covers `rows_a` op(A) rows and the panel's columns.
+__host__ __device__ inline int panel_row(int b, int rows_a, int n, int j0) { return b < rows_a ? b : n + j0 + b - rows_a; }
 // Bytes of the rounding-correction region for a square problem of order n.
 size_t rounding_bytes(int n, int form, std::vector<size_t>* guards = nullptr);
 // Device address of the pass's counters (flagged, recomputed as tiles, one by
@@ -246,9 +263,10 @@ cudaError_t launch_strided(cudaStream_t s, const Problem& p, int mode, int repai
 // Enqueue a fully planned call (pack + GEMM [+ merge] [+ rounding]); when
 // `events` is non-null, kernel j (in the order the call info names them) is
 // bracketed by events[2j] and events[2j + 1], recorded on the stream it runs
-// on (entries past nevents are skipped).
+// on (entries past nevents are skipped).  `panel`: only these output columns
+// (tensor-core forms with the rounding pass).
 cudaError_t enqueue(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status, int* kernels,
-                    const cudaEvent_t* events = nullptr, int nevents = 0);
+                    const cudaEvent_t* events = nullptr, int nevents = 0, const ColPanel* panel = nullptr);
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 

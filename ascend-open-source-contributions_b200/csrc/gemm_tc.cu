@@ -174,6 +174,7 @@ struct TcParams {
     int* status;
     int seg_blocks;  // K-blocks per accumulation segment
     int cluster_merge;  // pair kernel: the `parts` pairs of a tile form one cluster and merge on chip
+    int tn0;            // first tile column (a panel of the rounding pass; else 0)
     long long c_batch;  // pair kernel: blockIdx.z is the problem of a batch, its C at c_batch elements each
     // pair kernel in the rounding pass: the per-16 x 16 flagged counts; pair
     // tiles inside a 256 x 256 tile the exact recompute takes are skipped
@@ -595,7 +596,7 @@ __global__ void __launch_bounds__(kLeadThreads, 1)
     const int first_m = (pid / in_group) * GM;
     const int gsz = min(p.tiles_m - first_m, GM);
     const int tm = first_m + (pid % in_group) % gsz;
-    const int tn = (pid % in_group) / gsz;
+    const int tn = p.tn0 + (pid % in_group) / gsz;
     const int m0 = tm * TILE_M, n0 = tn * kLeadBN;
     const int kblocks = (p.k + Cfg::BK - 1) / Cfg::BK;
     const int seg_blocks = p.seg_blocks;
@@ -900,7 +901,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int first_m = (pid / in_group) * GM;
     const int gsz = min(tiles_m2 - first_m, GM);
     const int tm = first_m + (pid % in_group) % gsz;
-    const int tn = (pid % in_group) / gsz;
+    const int tn = p.tn0 + (pid % in_group) / gsz;
     const int m0 = tm * 2 * TILE_M + (int)rank * TILE_M;  // this CTA's rows
     const int n0 = tn * BN;
     const int part = blockIdx.y;
@@ -1199,7 +1200,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 template <int FORM>
 cudaError_t launch_pair(cudaStream_t stream, const Problem& pr, const Plan& plan, void* ws, int* status,
-                        const uint32_t* skip_count = nullptr, const BatchStrides& batch = BatchStrides{})
+                        const uint32_t* skip_count = nullptr, const BatchStrides& batch = BatchStrides{},
+                        const ColPanel* panel = nullptr)
 {
     using Cfg = TcCfg<FORM>;
     using G = PairGeom<FORM>;
@@ -1245,6 +1247,10 @@ cudaError_t launch_pair(cudaStream_t stream, const Problem& pr, const Plan& plan
     }
     p.skip_count = skip_count;
     p.c_batch = batch.c;
+    if (panel != nullptr) {
+        p.tn0 = panel->j0 / PAIR_BN;
+        p.tiles_n = ceil_div(panel->j1 - panel->j0, PAIR_BN);
+    }
     p.cluster_merge = plan.cluster_merge ? 1 : 0;
     if (p.cluster_merge && (plan.parts < 2 || plan.parts > 4)) {
         return cudaErrorInvalidValue;  // clusters of at most 8 CTAs: up to 4 pairs
@@ -1329,7 +1335,7 @@ cudaError_t launch_form(cudaStream_t stream, const Problem& pr, const Plan& plan
 
 template <int LEAD>
 cudaError_t launch_lead_path(cudaStream_t stream, const Problem& pr, const Plan& plan, void* ws, int* status,
-                             const LeadSelect& sel)
+                             const LeadSelect& sel, const ColPanel& panel)
 {
     using Cfg = TcCfg<LEAD>;
     const bool bf16 = Cfg::FMT == 1;
@@ -1360,7 +1366,8 @@ cudaError_t launch_lead_path(cudaStream_t stream, const Problem& pr, const Plan&
     p.span = pr.k;
     p.parts = 1;
     p.tiles_m = ceil_div(pr.m, TILE_M);
-    p.tiles_n = ceil_div(pr.n, kLeadBN);
+    p.tn0 = panel.j0 / kLeadBN;
+    p.tiles_n = ceil_div(panel.j1 - panel.j0, kLeadBN);
     p.epi = EpiParams{pr.ar, pr.ai, pr.br, pr.bi, plan.unit ? 1 : 0, plan.beta_zero ? 1 : 0};
     p.C = static_cast<float2*>(pr.C);
     p.ldc = pr.ldc;
@@ -1425,26 +1432,30 @@ cudaError_t launch_gemm_tc_batch(cudaStream_t stream, const Problem& pr, const P
 }
 
 cudaError_t launch_gemm_tc_path(cudaStream_t stream, const Problem& pr, const Plan& plan, void* ws,
-                                const LeadSelect& sel, int* status)
+                                const LeadSelect& sel, const ColPanel& panel, int* status)
 {
     switch (plan.form) {
-        case CG3M_FORM_TF32X3: return launch_lead_path<kLeadTf32>(stream, pr, plan, ws, status, sel);
+        case CG3M_FORM_TF32X3: return launch_lead_path<kLeadTf32>(stream, pr, plan, ws, status, sel, panel);
         case CG3M_FORM_BF16X6:
-        case CG3M_FORM_BF16X9: return launch_lead_path<kLeadBf16>(stream, pr, plan, ws, status, sel);
+        case CG3M_FORM_BF16X9: return launch_lead_path<kLeadBf16>(stream, pr, plan, ws, status, sel, panel);
         default: return cudaErrorInvalidValue;
     }
 }
 
-cudaError_t launch_gemm_tc_tiles(cudaStream_t stream, const Problem& pr, const Plan& plan, void* ws, int* status,
-                                 const uint32_t* tile_count)
+cudaError_t launch_gemm_tc_tiles(cudaStream_t stream, const Problem& pr, const Plan& plan, void* ws,
+                                 const ColPanel& panel, int* status, const uint32_t* tile_count)
 {
+    const BatchStrides one;
     if (!CG3M_TC_PAIR || pr.m <= TILE_M || plan.parts != 1 || tile_count == nullptr) {
         return cudaErrorInvalidValue;  // the rounding pass's orders (2048..4096) always have two row tiles
     }
     switch (plan.form) {
-        case CG3M_FORM_TF32X3: return launch_pair<CG3M_FORM_TF32X3>(stream, pr, plan, ws, status, tile_count);
-        case CG3M_FORM_BF16X6: return launch_pair<CG3M_FORM_BF16X6>(stream, pr, plan, ws, status, tile_count);
-        case CG3M_FORM_BF16X9: return launch_pair<CG3M_FORM_BF16X9>(stream, pr, plan, ws, status, tile_count);
+        case CG3M_FORM_TF32X3: return launch_pair<CG3M_FORM_TF32X3>(stream, pr, plan, ws, status, tile_count, one,
+                                                                   &panel);
+        case CG3M_FORM_BF16X6: return launch_pair<CG3M_FORM_BF16X6>(stream, pr, plan, ws, status, tile_count, one,
+                                                                   &panel);
+        case CG3M_FORM_BF16X9: return launch_pair<CG3M_FORM_BF16X9>(stream, pr, plan, ws, status, tile_count, one,
+                                                                   &panel);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -153,6 +153,7 @@ struct OzCrt {
 struct OzParams {
     int kblocks;             // 128-byte K blocks
     int tiles;               // tiles per side
+    int tn0, tn1;            // tile columns of this launch
     const uint8_t* tile_ran; // per tile (tn * tiles + tm): 1 when the exact products run there
     uint8_t* residues;       // [kOzPlanes][y_pad / 16][y_pad][16]
     int y_pad;
@@ -166,6 +167,7 @@ struct OzParams {
 struct OzFinish {
     int n;
     int tiles;
+    int strip0;              // first 16-column strip of this launch
     const int* E;            // op(A) row exponents
     const int* F;            // op(B) column exponents
     const int* CA;           // rounded parts per op(A) row
@@ -246,7 +248,7 @@ __device__ __forceinline__ void store_images(const float2 (*re)[3], const float2
     }
 }
 
-// One block per op(A) row (blockIdx.x < n) or op(B) column.  Plane layout:
+// One block per op(A) row (the first nrows_a) or op(B) column of the panel.  Plane layout:
 // [2m + {0 plus, 1 minus}][row][kpitch] int8 for both operands.
 //
 // All FP32: the 47-bit parts go through 16-bit limbs, so a residue is a few
@@ -255,12 +257,13 @@ __device__ __forceinline__ void store_images(const float2 (*re)[3], const float2
 __global__ void __launch_bounds__(256)
     ozaki_split_kernel(int n, int pitch, const float2* __restrict__ rows_a, const float2* __restrict__ rows_b,
                        int8_t* __restrict__ pa, int8_t* __restrict__ pb, int kpitch, size_t plane_bytes,
-                       int* __restrict__ E, int* __restrict__ F, int* __restrict__ CA, int* __restrict__ CB)
+                       int* __restrict__ E, int* __restrict__ F, int* __restrict__ CA, int* __restrict__ CB, int nrows_a,
+                       int j0)
 {
     __shared__ float wmax[8];
     __shared__ int wbad[8];
     __shared__ int wcnt[8];
-    const int r = blockIdx.x;
+    const int r = panel_row(blockIdx.x, nrows_a, n, j0);
     const bool is_a = r < n;
     const int row = is_a ? r : r - n;
     const float2* src = (is_a ? rows_a : rows_b) + (size_t)row * pitch;
@@ -415,7 +418,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     if (warp == 0) {
         uint32_t mask = 0;
         if (lane < p.tiles) {
-            for (int tn = 0; tn < p.tiles; ++tn) {
+            for (int tn = p.tn0; tn < p.tn1; ++tn) {
                 mask |= (p.tile_ran[(size_t)tn * p.tiles + lane] ? 1u : 0u) << tn;
             }
         }
@@ -670,15 +673,16 @@ __global__ void __launch_bounds__(256, 4) ozaki_crt_kernel(const __grid_constant
 {
     const int pair = threadIdx.x & 7;
     const int row = blockIdx.y * kCrtRows + (threadIdx.x >> 3);
-    const int col0 = blockIdx.x * 16 + pair * 2;
+    const int strip = f.strip0 + blockIdx.x;
+    const int col0 = strip * 16 + pair * 2;
     const int n = f.n;
-    const int tm = (blockIdx.y * kCrtRows) / OZ_TILE_M, tn = (blockIdx.x * 16) / OZ_TN;
+    const int tm = (blockIdx.y * kCrtRows) / OZ_TILE_M, tn = (strip * 16) / OZ_TN;
     if (!f.tile_ran[(size_t)tn * f.tiles + tm] || row >= n || col0 >= n) {
         return;
     }
     // Every output of a tile that ran is written here, flagged or not: the
     // form's own products skipped these tiles.
-    const uint8_t* src = f.residues + ((size_t)blockIdx.x * f.y_pad + row) * 16 + pair * 2;
+    const uint8_t* src = f.residues + ((size_t)strip * f.y_pad + row) * 16 + pair * 2;
     double xr[2], xi[2];
     {
         double s[2][2][3];  // [part][output][limb]
@@ -849,20 +853,22 @@ static const OzCrt& crt_constants()
     return crt;
 }
 
-cudaError_t launch_ozaki_split(cudaStream_t s, int n, int pitch, const float2* rows_a, const float2* rows_b,
-                               const OzLayout& L)
+cudaError_t launch_ozaki_split(cudaStream_t s, int n, int pitch, const ColPanel& panel, const float2* rows_a,
+                               const float2* rows_b, const OzLayout& L)
 {
     static const bool range_ok = crt_range_ok();
     if (n > kOzMaxN || !range_ok) {
         return cudaErrorInvalidValue;  // the moduli cover the exact products up to order kOzMaxN
     }
-    ozaki_split_kernel<<<2 * n, 256, 0, s>>>(n, pitch, rows_a, rows_b, L.planes_a, L.planes_b, L.kpitch,
-                                              L.plane_bytes, L.E, L.F, L.CA, L.CB);
+    const int nrows_a = panel.index == 0 ? n : 0;
+    ozaki_split_kernel<<<nrows_a + panel.j1 - panel.j0, 256, 0, s>>>(n, pitch, rows_a, rows_b, L.planes_a, L.planes_b, L.kpitch,
+                                              L.plane_bytes, L.E, L.F, L.CA, L.CB, nrows_a, panel.j0);
     return cudaGetLastError();
 }
 
-cudaError_t launch_ozaki_tiles(cudaStream_t s, int n, const OzLayout& L, uint32_t* stats, uint32_t* fallback_bits,
-                               float2* C, int* status, int* launched, const std::function<void(int)>& mark)
+cudaError_t launch_ozaki_tiles(cudaStream_t s, int n, const ColPanel& panel, const OzLayout& L, uint32_t* stats,
+                               uint32_t* fallback_bits, float2* C, int* status, int* launched,
+                               const std::function<void(int)>& mark)
 {
     const OzCrt& crt = crt_constants();
     int count = 0;
@@ -888,6 +894,8 @@ cudaError_t launch_ozaki_tiles(cudaStream_t s, int n, const OzLayout& L, uint32_
         OzParams p{};
         p.kblocks = (n + OZ_BK - 1) / OZ_BK;
         p.tiles = tiles;
+        p.tn0 = panel.j0 / OZ_TN;
+        p.tn1 = ceil_div(panel.j1, OZ_TN);
         p.tile_ran = L.tile_ran;
         p.residues = L.residues;
         p.y_pad = L.y_pad;
@@ -933,6 +941,7 @@ cudaError_t launch_ozaki_tiles(cudaStream_t s, int n, const OzLayout& L, uint32_
         OzFinish f{};
         f.n = n;
         f.tiles = tiles;
+        f.strip0 = panel.j0 / 16;
         f.E = L.E;
         f.F = L.F;
         f.CA = L.CA;
@@ -945,7 +954,8 @@ cudaError_t launch_ozaki_tiles(cudaStream_t s, int n, const OzLayout& L, uint32_
         f.fallback_bits = fallback_bits;
         f.C = C;
         f.crt = crt;
-        ozaki_crt_kernel<<<dim3((unsigned)(L.y_pad / 16), (unsigned)(L.y_pad / kCrtRows)), 256, 0, s>>>(f);
+        const int strips = ceil_div(panel.j1, 16) - f.strip0;
+        ozaki_crt_kernel<<<dim3((unsigned)strips, (unsigned)(L.y_pad / kCrtRows)), 256, 0, s>>>(f);
         err = cudaGetLastError();
         mark(++count);
     }

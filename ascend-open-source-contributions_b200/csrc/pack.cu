@@ -199,8 +199,22 @@ unsigned pack_blocks(const PackSide& a, const PackSide& b)
 
 }  // namespace
 
+namespace {
+
+// Narrows op(B)'s side to the panel's columns: they are stored columns when the
+// source is k x n and stored rows otherwise, and plane rows either way
+// (K-major planes of `elem` bytes an element).
+void narrow_to_panel(PackSide& s, const ColPanel& panel, bool normal, size_t elem)
+{
+    s.src += (size_t)panel.j0 * (normal ? s.ld : 1);
+    (normal ? s.cols : s.rows) = panel.j1 - panel.j0;
+    s.out = static_cast<uint8_t*>(s.out) + (size_t)panel.j0 * s.pitch * elem;
+}
+
+}  // namespace
+
 cudaError_t launch_pack_rows(cudaStream_t stream, const Problem& p, void* rows_a, void* rows_b, int pitch,
-                             const Plan* lead_plan, void* ws)
+                             const Plan* lead_plan, void* ws, const ColPanel* panel)
 {
     auto side = [&](bool isA) {
         PackSide s{};
@@ -225,6 +239,13 @@ cudaError_t launch_pack_rows(cudaStream_t stream, const Problem& p, void* rows_a
             s.lead_pitch = isA ? lead_plan->pitch_a : lead_plan->pitch_b;
             s.lead_plane_elems = isA ? lead_plan->plane_a_elems : lead_plan->plane_b_elems;
         }
+        if (panel != nullptr && !isA) {
+            narrow_to_panel(s, *panel, normal, sizeof(float2));
+            const size_t elem = lead_plan->form == CG3M_FORM_TF32X3 ? 4 : 2;
+            s.lead = static_cast<uint8_t*>(s.lead) + (size_t)panel->j0 * s.lead_pitch * elem;
+        } else if (panel != nullptr && panel->index > 0) {
+            s.rows = 0;  // packed with the first panel
+        }
         return s;
     };
     const PackSide a = side(true), b = side(false);
@@ -240,7 +261,7 @@ cudaError_t launch_pack_rows(cudaStream_t stream, const Problem& p, void* rows_a
 }
 
 cudaError_t launch_pack(cudaStream_t stream, const Problem& p, const Plan& plan, void* ws, const uint8_t* band_a,
-                        const uint8_t* band_b, const BatchStrides& batch)
+                        const uint8_t* band_b, const BatchStrides& batch, const ColPanel* panel)
 {
     const bool kmajor = plan.form != CG3M_FORM_FP32;
     const size_t elem = plan.form == CG3M_FORM_BF16X6 || plan.form == CG3M_FORM_BF16X9 ? 2 : 4;
@@ -266,6 +287,10 @@ cudaError_t launch_pack(cudaStream_t stream, const Problem& p, const Plan& plan,
         s.band_need = isA ? band_a : band_b;
         s.src_batch = isA ? batch.a : batch.b;
         s.out_batch = (size_t)plan.planes * s.plane_elems * elem;
+        if (panel != nullptr && !isA) {
+            narrow_to_panel(s, *panel, normal, elem);
+            s.band_need += panel->j0 / 256;
+        }
         return s;
     };
     const PackSide a = side(true), b = side(false);

@@ -39,14 +39,15 @@
 namespace cg3m {
 
 cudaError_t launch_pack_rows(cudaStream_t stream, const Problem& p, void* rows_a, void* rows_b, int pitch,
-                             const Plan* lead_plan = nullptr, void* ws = nullptr);
+                             const Plan* lead_plan = nullptr, void* ws = nullptr, const ColPanel* panel = nullptr);
 cudaError_t launch_gemm_fp32_path(cudaStream_t stream, const Problem& pr, const Plan& plan, void* ws, float* path,
                                   int* status);
 cudaError_t launch_gemm_tc_path(cudaStream_t stream, const Problem& pr, const Plan& plan, void* ws,
-                                const LeadSelect& sel, int* status);
+                                const LeadSelect& sel, const ColPanel& panel, int* status);
 
 namespace {
 
+constexpr int kMaxBands = 16;         // 256-row bands of the largest gated order, 4096
 constexpr int kLanes = 64;
 constexpr int kTile = 16;             // flag granule: 16 x 16 outputs
 constexpr int kMaxSpan = 65;          // ceil(4096/64) | 1
@@ -56,10 +57,10 @@ constexpr float kConfidence = 3.75f;  // CGEMM_ROUNDING_CONFIDENCE, cgemm_host.c
 
 __global__ void __launch_bounds__(kLanes) energy_kernel(const float2* __restrict__ rows_a,
                                                         const float2* __restrict__ rows_b, int n, int pitch,
-                                                        int span, float* __restrict__ energy)
+                                                        int span, float* __restrict__ energy, int nrows_a, int j0)
 {
     __shared__ float lanes[kLanes];
-    const int r = blockIdx.x;
+    const int r = panel_row(blockIdx.x, nrows_a, n, j0);
     const float2* src = r < n ? rows_a + (size_t)r * pitch : rows_b + (size_t)(r - n) * pitch;
     // Each lane reads its own span of consecutive terms straight from global
     // memory (no staged row, so many rows are in flight per SM); the sector a
@@ -163,26 +164,36 @@ __global__ void select_kernel(int n, const float2* __restrict__ C, const float* 
 // that row band of op(A) and column band of op(B), so both bands are marked
 // for the rest of the pack.
 static_assert(kOzakiTile / kTile == 16, "16 x 16 count tiles per exact tile");
-__global__ void __launch_bounds__(256) band_need_kernel(int n, const uint32_t* __restrict__ tile_count,
+// The planes of an op(A) band packed for an earlier panel stay: band_a holds one
+// array of kMaxBands per panel, and a band is marked in the first that needs it.
+__global__ void __launch_bounds__(256) band_need_kernel(int n, int band0, int panel,
+                                                         const uint32_t* __restrict__ tile_count,
                                                          uint8_t* __restrict__ band_a, uint8_t* __restrict__ band_b,
                                                          uint8_t* __restrict__ tile_ran, uint32_t* __restrict__ stats)
 {
+    const int bj = band0 + blockIdx.y;
     const int g16 = (n + kTile - 1) / kTile;
     const int gi = blockIdx.x * 16 + threadIdx.x % 16;
-    const int gj = blockIdx.y * 16 + threadIdx.x / 16;
+    const int gj = bj * 16 + threadIdx.x / 16;
     const uint32_t count = gi < g16 && gj < g16 ? tile_count[(size_t)gj * g16 + gi] : 0u;
     const bool run = __syncthreads_or(count > kSparseMax);
     if (threadIdx.x == 0) {
-        tile_ran[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = run ? 1 : 0;
+        tile_ran[(size_t)bj * gridDim.x + blockIdx.x] = run ? 1 : 0;
         if (run) {
             atomicAdd(&stats[kStatExactTiles], 1u);
             // output positions of the tile inside the matrix (the roofline's work)
             const int rows = min(kOzakiTile, n - (int)blockIdx.x * kOzakiTile);
-            const int cols = min(kOzakiTile, n - (int)blockIdx.y * kOzakiTile);
+            const int cols = min(kOzakiTile, n - bj * kOzakiTile);
             atomicAdd(&stats[kStatExactOutputs], (uint32_t)(rows * cols));
         } else {
-            band_a[blockIdx.x] = 1;
-            band_b[blockIdx.y] = 1;
+            bool packed = false;
+            for (int q = 0; q < panel; ++q) {
+                packed |= band_a[q * kMaxBands + blockIdx.x] != 0;
+            }
+            if (!packed) {
+                band_a[panel * kMaxBands + blockIdx.x] = 1;
+            }
+            band_b[bj] = 1;
         }
     }
     if (run) {
@@ -552,12 +563,12 @@ __global__ void __launch_bounds__(512) recompute_fp32_tiled(const __grid_constan
 __global__ void __launch_bounds__(256) lane_major_kernel(int n, int pitch, int span, const float2* __restrict__ rows_a,
                                                          const float2* __restrict__ rows_b,
                                                          float2* __restrict__ lanes_a, float2* __restrict__ lanes_b,
-                                                         const uint8_t* __restrict__ need)
+                                                         uint8_t* __restrict__ need, int j0)
 {
     extern __shared__ float2 row[];
-    const int r = blockIdx.x;
-    if (!need[r]) {
-        return;  // no output the per-output kernels recompute lies in this row or column
+    const int r = panel_row(blockIdx.x, n, n, j0);
+    if (need[r] != 1) {
+        return;  // no output the per-output kernels recompute lies in this row or column, or it was copied
     }
     const size_t width = (size_t)kLanes * span;
     const float2* src = r < n ? rows_a + (size_t)r * pitch : rows_b + (size_t)(r - n) * pitch;
@@ -566,6 +577,9 @@ __global__ void __launch_bounds__(256) lane_major_kernel(int n, int pitch, int s
         row[k] = src[k];
     }
     __syncthreads();
+    if (threadIdx.x == 0) {
+        need[r] = 2;  // copied: a later panel need not
+    }
     for (int f = threadIdx.x; f < (int)width; f += blockDim.x) {
         const int sidx = f / kLanes, l = f % kLanes;
         const int k = l * span + sidx;
@@ -583,11 +597,12 @@ __global__ void __launch_bounds__(256) lanes_needed_kernel(int n, int tc, const 
                                                            const uint32_t* __restrict__ fallback_bits,
                                                            const uint32_t* __restrict__ tile_count,
                                                            const uint8_t* __restrict__ tile_ran, int exact_tiles,
-                                                           uint8_t* __restrict__ need)
+                                                           uint8_t* __restrict__ need, int j0, int j1)
 {
-    const size_t words = ((size_t)n * n + 31) / 32;
+    // panels start on whole words (j0 is a multiple of 256)
+    const size_t words = ((size_t)j1 * n + 31) / 32;
     const int tiles16 = (n + kTile - 1) / kTile;
-    for (size_t w = (size_t)blockIdx.x * blockDim.x + threadIdx.x; w < words; w += (size_t)gridDim.x * blockDim.x) {
+    for (size_t w = (size_t)j0 * n / 32 + (size_t)blockIdx.x * blockDim.x + threadIdx.x; w < words; w += (size_t)gridDim.x * blockDim.x) {
         const uint32_t fb = tc ? fallback_bits[w] : 0u;
         uint32_t bits = flag_bits[w] | fb;
         // Fast path: a word inside one column and one tile row band whose tile
@@ -623,7 +638,9 @@ __global__ void __launch_bounds__(256) lanes_needed_kernel(int n, int tc, const 
                           : tile_count[(size_t)(j / kTile) * tiles16 + i / kTile] <= kSparseMax;
             }
             if (want) {
-                need[i] = 1;
+                if (need[i] == 0) {  // 2: an earlier panel copied it
+                    need[i] = 1;
+                }
                 need[n + j] = 1;
             }
         }
@@ -655,7 +672,8 @@ __global__ void __launch_bounds__(kLanes) recompute_sparse(int n, int span,
                                                           const uint32_t* __restrict__ bits,
                                                           const uint32_t* __restrict__ tile_count,
                                                           uint32_t* __restrict__ stats, float2* __restrict__ C,
-                                                          const uint8_t* __restrict__ tile_ran, int exact_tiles)
+                                                          const uint8_t* __restrict__ tile_ran, int exact_tiles,
+                                                          int gj0, int gjn)
 {
     constexpr bool FP64 = MODE != kSparseFp32;
     __shared__ float sr[kLanes], si[kLanes], tr[kLanes], ti[kLanes];
@@ -668,9 +686,9 @@ __global__ void __launch_bounds__(kLanes) recompute_sparse(int n, int span,
     // band's columns go by, so each staged row comes from L2, not HBM.
     constexpr int kSparseBand = 64;
     const int tiles = (n + kTile - 1) / kTile;
-    const int band = blockIdx.x / (kSparseBand * tiles), first = band * kSparseBand;
-    const int rows_in_band = min(kSparseBand, tiles - first), in_band = blockIdx.x - band * kSparseBand * tiles;
-    const int gi = first + in_band % rows_in_band, gj = in_band / rows_in_band;
+    const int band = blockIdx.x / (kSparseBand * gjn), first = band * kSparseBand;
+    const int rows_in_band = min(kSparseBand, tiles - first), in_band = blockIdx.x - band * kSparseBand * gjn;
+    const int gi = first + in_band % rows_in_band, gj = gj0 + in_band / rows_in_band;
     const uint32_t count = tile_count[(size_t)gj * tiles + gi];
     if (count == 0) {
         return;
@@ -897,16 +915,15 @@ struct RoundLayout {
     uint32_t* stats;
     uint32_t* fallback_bits;
     uint8_t* need;      // rows of op(A), then columns of op(B), the per-output kernels read
-    uint8_t* band;      // [kMaxBands] op(A) row bands, then [kMaxBands] op(B) column bands, of 256
-                        // whose tiles the form's products read (tensor-core forms)
+    uint8_t* band;      // [kMaxBands] op(B) column bands, then per panel [kMaxBands] op(A) row bands, of
+                        // 256 whose tiles the form's products read (tensor-core forms)
     size_t zero_bytes;  // tile_count + stats + fallback_bits + need + band, one memset
     OzLayout oz;
 };
 
 static size_t flag_words(int n) { return ((size_t)n * n + 31) / 32; }
 static size_t need_words(int n) { return ((size_t)2 * n + 3) / 4; }
-constexpr int kMaxBands = 16;  // 256-row bands of the largest gated order, 4096
-static size_t band_words() { return (size_t)2 * kMaxBands / 4; }
+static size_t band_words() { return (size_t)(kMaxPanels + 1) * kMaxBands / 4; }
 static size_t tile_words(int n)
 {
     const size_t t = (size_t)(n + kTile - 1) / kTile;
@@ -987,7 +1004,8 @@ uint32_t* rounding_stats_ptr(const Plan& plan, void* ws, int n) { return round_l
 
 size_t rounding_bytes(int n, int form, std::vector<size_t>* guards) { return round_offsets(n, form, guards).end; }
 
-cudaError_t launch_gemm_with_path(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status)
+cudaError_t launch_gemm_with_path(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const ColPanel& panel,
+                                  int* status)
 {
     const RoundLayout L = round_layout(plan, ws, p.n);
     if (plan.form == CG3M_FORM_FP32) {
@@ -995,7 +1013,7 @@ cudaError_t launch_gemm_with_path(cudaStream_t s, const Problem& p, const Plan& 
     }
     const LeadSelect sel{L.energy, bridge_term(p.n), kConfidence * kConfidence, L.flag_bits,
                          L.tile_count, L.stats};
-    return launch_gemm_tc_path(s, p, plan, ws, sel, status);
+    return launch_gemm_tc_path(s, p, plan, ws, sel, panel, status);
 }
 
 // The replay's staging copies: op(A) rows or op(B) columns as an n x n array of
@@ -1047,28 +1065,33 @@ int rounding_prep_kernels(int form)
 // take per-bit atomics when n is not a multiple of 32), then the packed rows
 // with the leading planes and the energies, all before the risk-plane GEMM
 // that applies the selection.
-cudaError_t launch_rounding_pack(cudaStream_t s, const Problem& p, const Plan& plan, void* ws,
+cudaError_t launch_rounding_pack(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const ColPanel& panel,
                                  const std::function<void()>& mark)
 {
     const int n = p.n;
     const RoundLayout L = round_layout(plan, ws, n);
     const int pitch = row_pitch(n);
-    cudaError_t err = cudaMemsetAsync(L.flag_bits, 0, L.zero_bytes + flag_words(n) * 4, s);
+    cudaError_t err = cudaSuccess;
+    if (panel.index == 0) {
+        err = cudaMemsetAsync(L.flag_bits, 0, L.zero_bytes + flag_words(n) * 4, s);
+    }
     if (err == cudaSuccess) {
-        err = launch_pack_rows(s, p, L.rows_a, L.rows_b, pitch, &plan, ws);
+        err = launch_pack_rows(s, p, L.rows_a, L.rows_b, pitch, &plan, ws, &panel);
         mark();
     }
     if (err == cudaSuccess) {
         const int span = ((n + kLanes - 1) / kLanes) | 1;
-        energy_kernel<<<2 * n, kLanes, 0, s>>>(L.rows_a, L.rows_b, n, pitch, span, L.energy);
+        const int nrows_a = panel.index == 0 ? n : 0;
+        energy_kernel<<<nrows_a + panel.j1 - panel.j0, kLanes, 0, s>>>(L.rows_a, L.rows_b, n, pitch, span, L.energy,
+                                                                       nrows_a, panel.j0);
         err = cudaGetLastError();
         mark();
     }
     return err;
 }
 
-cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* launched,
-                                 const std::function<void(int)>& mark)
+cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const ColPanel& panel,
+                                 int* launched, const std::function<void(int)>& mark)
 {
     const int n = p.n;
     const int pitch = row_pitch(n);
@@ -1081,13 +1104,12 @@ cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& p
         mark(++count);
     }
     if (err == cudaSuccess && plan.form == CG3M_FORM_FP32) {
-        energy_kernel<<<2 * n, kLanes, 0, s>>>(L.rows_a, L.rows_b, n, pitch, span,
-                                                                        L.energy);
+        energy_kernel<<<2 * n, kLanes, 0, s>>>(L.rows_a, L.rows_b, n, pitch, span, L.energy, n, 0);
         err = cudaGetLastError();
         mark(++count);
     }
     if (err == cudaSuccess && plan.form != CG3M_FORM_FP32) {
-        err = launch_ozaki_split(s, n, pitch, L.rows_a, L.rows_b, L.oz);
+        err = launch_ozaki_split(s, n, pitch, panel, L.rows_a, L.rows_b, L.oz);
         mark(++count);
     }
     if (launched != nullptr) {
@@ -1096,8 +1118,9 @@ cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& p
     return err;
 }
 
-cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* status,
-                                   int* launched, const std::function<void(int)>& mark)
+cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan& plan, void* ws,
+                                   const ColPanel& panel, int* status, int* launched,
+                                   const std::function<void(int)>& mark)
 {
     const int n = p.n;
     const RoundLayout L = round_layout(plan, ws, n);
@@ -1123,12 +1146,13 @@ cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan&
     auto lanes = [&]() {
         const bool tc = plan.form != CG3M_FORM_FP32;
         lanes_needed_kernel<<<148 * 4, 256, 0, s>>>(n, tc ? 1 : 0, L.flag_bits, L.fallback_bits, L.tile_count,
-                                                    tc ? L.oz.tile_ran : nullptr, L.oz.y_pad / kOzakiTile, L.need);
+                                                    tc ? L.oz.tile_ran : nullptr, L.oz.y_pad / kOzakiTile, L.need,
+                                                    panel.j0, panel.j1);
         cudaError_t e = cudaGetLastError();
         mark(++count);
         if (e == cudaSuccess) {
-            lane_major_kernel<<<2 * n, 256, (size_t)n * sizeof(float2), s>>>(n, pitch, span, L.rows_a, L.rows_b,
-                                                                             L.lanes_a, L.lanes_b, L.need);
+            lane_major_kernel<<<n + panel.j1 - panel.j0, 256, (size_t)n * sizeof(float2), s>>>(
+                n, pitch, span, L.rows_a, L.rows_b, L.lanes_a, L.lanes_b, L.need, panel.j0);
             e = cudaGetLastError();
             mark(++count);
         }
@@ -1138,8 +1162,9 @@ cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan&
         // one block per 16 x 16 tile: several tiles per block (4, or a grid-
         // stride walk) saved ~0.02 ms of block launches where no tile has work
         // but made the reference's data (~7 flagged outputs per tile) 1.6-2.5x slower
-        kernel<<<tiles16 * tiles16, kLanes, 0, s>>>(n, span, L.lanes_a, L.lanes_b, bits, L.tile_count, L.stats, C,
-                                                    L.oz.tile_ran, L.oz.y_pad / kOzakiTile);
+        const int gj0 = panel.j0 / kTile, gjn = ceil_div(panel.j1, kTile) - gj0;
+        kernel<<<tiles16 * gjn, kLanes, 0, s>>>(n, span, L.lanes_a, L.lanes_b, bits, L.tile_count, L.stats, C,
+                                                L.oz.tile_ran, L.oz.y_pad / kOzakiTile, gj0, gjn);
         const cudaError_t e = cudaGetLastError();
         mark(++count);
         return e;
@@ -1161,27 +1186,30 @@ cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan&
         // not take, and the exact recompute writes every output of its tiles.
         // The rest of the form's planes is packed for the bands those tiles read.
         const int bands = (n + kOzakiTile - 1) / kOzakiTile;
-        if (err == cudaSuccess && bands > kMaxBands) {
+        const int band0 = panel.j0 / kOzakiTile, panel_bands = ceil_div(panel.j1, kOzakiTile) - band0;
+        uint8_t* const band_b = L.band;
+        uint8_t* const band_a = L.band + kMaxBands;
+        if (err == cudaSuccess && (bands > kMaxBands || panel.index >= kMaxPanels)) {
             err = cudaErrorInvalidValue;  // beyond the gated orders
         }
         if (err == cudaSuccess) {
-            band_need_kernel<<<dim3(bands, bands), 256, 0, s>>>(n, L.tile_count, L.band, L.band + kMaxBands,
-                                                            L.oz.tile_ran, L.stats);
+            band_need_kernel<<<dim3(bands, panel_bands), 256, 0, s>>>(n, band0, panel.index, L.tile_count, band_a,
+                                                                     band_b, L.oz.tile_ran, L.stats);
             err = cudaGetLastError();
             mark(++count);
         }
         if (err == cudaSuccess) {
-            err = launch_pack(s, p, plan, ws, L.band, L.band + kMaxBands);
+            err = launch_pack(s, p, plan, ws, band_a + panel.index * kMaxBands, band_b, BatchStrides{}, &panel);
             mark(++count);
         }
         if (err == cudaSuccess) {
-            err = launch_gemm_tc_tiles(s, p, plan, ws, status, L.tile_count);
+            err = launch_gemm_tc_tiles(s, p, plan, ws, panel, status, L.tile_count);
             mark(++count);
         }
         if (err == cudaSuccess) {
             int oz_launched = 0;
             const int before = count;
-            err = launch_ozaki_tiles(s, n, L.oz, L.stats, L.fallback_bits, C, status, &oz_launched,
+            err = launch_ozaki_tiles(s, n, panel, L.oz, L.stats, L.fallback_bits, C, status, &oz_launched,
                                      [&](int i) { mark(before + i); });
             count += oz_launched;
         }

@@ -320,7 +320,9 @@ cg3mStatus_t cg3mCgemm3mNoAlloc(void* stream, cg3mOperation_t transa, cg3mOperat
  * host.  Every panel is the cg3mCgemm3mEx call on device copies that keep the
  * caller's leading dimensions, with the K split of the whole problem, so C
  * holds the bits the device call on the whole problem would give.  When the
- * rounding-correction pass applies to the whole problem it runs as one panel.
+ * rounding-correction pass applies to the whole problem, the tensor-core forms
+ * run it panel by panel (panels of whole 256-column tiles, at least two of
+ * them), the FP32 form as one panel.
  * `panels` <= 0 picks the count (about 8 panels of whole tiles); the device
  * copies are kept in the handle for later calls.  op code R is accepted.
  * C rows past m (padding) are neither read nor written. */
