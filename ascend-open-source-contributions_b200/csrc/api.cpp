@@ -538,7 +538,7 @@ cg3mStatus_t cg3mCgemm3mStridedBatchedEx(cg3mHandle_t h, cg3mOperation_t transa,
         if (onchip) {
             best = strided.est_us * (tc ? 1.1 : 1.0);
         }
-        if (tc && m > 128 && batch_tc_time_us(p, opts.form, h->sm_count, batch_count) < best) {
+        if (tc && m > 128 && batch_tc_time_us(p, opts, h->sm_count, batch_count) < best) {
             // As many problems per launch as fit kBatchPlaneBytes of planes (at
             // least one), in even chunks; fewer when the device has no room.
             Plan plan;

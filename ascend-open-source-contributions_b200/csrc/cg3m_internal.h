@@ -126,7 +126,7 @@ cudaError_t launch_gemm_tc_batch(cudaStream_t s, const Problem& p, const Plan& p
 // out for all of them), and its estimated time in microseconds; false when the
 // shape has one 128-row tile only.
 bool batch_tc_plan(const Problem& p, const cg3mOptions& opts, int sm_count, int count, Plan* plan);
-double batch_tc_time_us(const Problem& p, int form, int sm_count, int count);
+double batch_tc_time_us(const Problem& p, const cg3mOptions& opts, int sm_count, int count);
 cudaError_t launch_merge(cudaStream_t s, const Problem& p, const Plan& plan, void* ws);
 // The rounding-correction pass.  Tensor-core forms start the call with the
 // packed rows, which also write the leading split planes the risk-plane GEMM

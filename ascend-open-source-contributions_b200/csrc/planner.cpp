@@ -126,19 +126,6 @@ constexpr double kSingleMargin = 1.06;
 // Tensor-core kernel tile (gemm_tc.cu): 128 x 128, one CTA per SM (TMEM).
 const TileChoice kTcTiles[] = {{128, 128, 1}};
 
-// Busiest-SM work for `tiles` output tiles split into `parts` K partitions
-// (EstimateCgemmCoreWork, cgemm_host.cpp:145-156, with SM slots as cores).
-uint64_t core_work(const TileChoice& t, int m, int n, int parts, int sm_count)
-{
-    const uint64_t tiles = (uint64_t)ceil_div(m, t.bm) * ceil_div(n, t.bn);
-    const uint64_t slots = (uint64_t)sm_count * t.slots_per_sm;
-    const uint64_t waves = (tiles * parts + slots - 1) / slots;
-    // Work per wave: one tile's multiply-adds per K term, scaled by how many of
-    // the SM's slots share its FP32 pipe.
-    const uint64_t rows = std::min(m, t.bm), cols = std::min(n, t.bn);
-    return waves * rows * cols * (uint64_t)t.slots_per_sm;
-}
-
 // kSpan = ceil(ceil(k/g)/parts)*g (cgemm_host.cpp:274-275 with g = 16).  The
 // granule g is the GEMM kernel's K-tile so that only the last partition has a
 // ragged tail: 16 for the FP32 kernel, 64 elements (one 128-byte row of the
@@ -161,36 +148,67 @@ double packed_time_us(const Problem& p, int parts, int span, uint64_t tiles, int
     return us;
 }
 
-// Tensor-core call in microseconds (pack of the split planes, waves of CTA-pair
-// tiles, merge), fitted on B200 to the 200 performance shapes (graph replay;
-// median error 13-19 %, hence the margin where it is compared).
-double tc_time_us(const Problem& p, int form, int parts, int span, int sm_count)
+// Tensor-core call in microseconds, fitted on B200 to 600 timed (shape, form,
+// K split) calls of up to 3000 x 3000 x 4000 (median error 2 %; the split it
+// picks, or plain FP32, costs a mean 0.1 % over the best of each shape): the
+// pack per 5.5 MB it moves, waves of CTA-pair tiles (256 x 128 on two SMs; 128 x
+// 128 on one for a single row tile) at a fixed part and a time per K term that
+// depends on the accumulation segment, and the merge, in the tile's cluster or
+// per 10 MB of partials and output.
+struct TcCost {
+    double base_us, pack_us, wave_us, cluster_us, merge_us, term_us[3];  // segments of >= 128, 64, 32 terms
+};
+constexpr TcCost kTcCost[3] = {{3.85, 1.131, 5.81, 2.96, 0.929, {0.0409, 0.0521, 0.0711}},   // 3xTF32
+                               {3.57, 1.132, 6.82, 2.24, 0.947, {0.0394, 0.0523, 0.0523}},   // split-BF16 x6
+                               {4.32, 1.162, 6.40, 2.16, 0.990, {0.0563, 0.0632, 0.0632}}};  // split-BF16 x9
+
+uint64_t tc_tiles(const Problem& p)
 {
-    const uint64_t tiles = p.m > 128 ? (uint64_t)ceil_div(p.m, 256) * ceil_div(p.n, 128)
-                                     : (uint64_t)ceil_div(p.n, 128);
-    const double waves = (double)((tiles * parts + sm_count - 1) / sm_count);
-    const double elems = (double)p.m * p.k + (double)p.k * p.n;
-    if (form == CG3M_FORM_TF32X3) {
-        return 11.80 + 0.1374 * elems * 32e-6 + 0.11003 * waves * span + (parts > 1 ? 1.25 : 0.0);
+    return p.m > 128 ? (uint64_t)ceil_div(p.m, 256) * ceil_div(p.n, 128) : (uint64_t)ceil_div(p.n, 128);
+}
+
+// K splits merged on chip: only when every cluster of 2 x parts CTAs is
+// resident at once.  A grid that one wave holds as loose CTAs but not as
+// clusters runs a second wave, which costs more than the merge launch it saves
+// (1.3-1.6x on 128..144-CTA grids).
+bool tc_cluster_merge(const Problem& p, int parts, int sm_count)
+{
+    if (p.m <= 128 || parts < 2 || parts > 4) {
+        return false;
     }
-    const double terms = form == CG3M_FORM_BF16X9 ? 1.5 : 1.0;  // nine products instead of six
-    return 13.27 + 0.1055 * elems * 44e-6 + 0.08315 * terms * waves * span;
+    const uint64_t cap = std::max<uint64_t>(1, kClusterCapOneBlock[2 * parts - 1] * (uint64_t)sm_count / 148);
+    return tc_tiles(p) <= cap;
+}
+
+double tc_time_us(const Problem& p, int form, int segment, int parts, int span, int sm_count, int count = 1)
+{
+    const TcCost& c = kTcCost[form - CG3M_FORM_TF32X3];
+    const uint64_t slots = std::max(1, p.m > 128 ? sm_count / 2 : sm_count);
+    const bool merged = tc_cluster_merge(p, parts, sm_count) && count == 1;
+    const double waves = merged ? 1.0 : (double)((tc_tiles(p) * parts * count + slots - 1) / slots);
+    const double mb = ((double)p.m * p.k + (double)p.k * p.n) * count * (form == CG3M_FORM_TF32X3 ? 32e-6 : 26e-6);
+    const double terms = (double)align_up((size_t)span, 64);
+    double us = c.base_us + c.pack_us * mb / 5.5 +
+                waves * (c.wave_us + terms * c.term_us[segment >= 128 ? 0 : segment >= 64 ? 1 : 2]);
+    if (merged) {
+        us += c.cluster_us;
+    } else if (parts > 1) {
+        us += c.merge_us * (double)(16 * parts + 16) * p.m * p.n * 1e-7;
+    }
+    return us;
+}
+
+// K terms accumulated in TMEM between round-to-nearest merges.
+int tc_segment(const cg3mOptions& opts, int k)
+{
+    return opts.tc_segment > 0 ? opts.tc_segment : (k >= 2048 ? 128 : k > 1024 ? 64 : 32);
 }
 
 }  // namespace
 
-// One launch of `count` equal problems on the CTA-pair kernel: the pack at
-// 5.5 TB/s, then waves of sm_count / 2 pair tiles (256 x 128) whose time per K
-// term is that of full waves at 3072^3 and 4096^3 (bound by L2 and the power
-// limit).
-double batch_tc_time_us(const Problem& p, int form, int sm_count, int count)
+double batch_tc_time_us(const Problem& p, const cg3mOptions& opts, int sm_count, int count)
 {
-    const double pairs = std::max(1, sm_count / 2);
-    const double tiles = (double)ceil_div(p.m, 256) * ceil_div(p.n, 128) * count;
-    const double elems = ((double)p.m * p.k + (double)p.k * p.n) * count;
-    const double bytes = form == CG3M_FORM_TF32X3 ? 32.0 : 26.0;
-    const double term = form == CG3M_FORM_TF32X3 ? 0.058 : form == CG3M_FORM_BF16X9 ? 0.078 : 0.057;
-    return 14.0 + elems * bytes / 5.5e6 + std::ceil(tiles / pairs) * ((double)align_up((size_t)p.k, 64) * term + 4.0);
+    return tc_time_us(p, opts.form, tc_segment(opts, p.k), 1, p.k, sm_count, count);
 }
 
 bool batch_tc_plan(const Problem& p, const cg3mOptions& opts, int sm_count, int count, Plan* plan)
@@ -222,7 +240,7 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
     // error grows with sqrt(K); these lengths keep the tensor-core error at or
     // below the plain form's (measured on data with a 2^16 dynamic range in the
     // imaginary parts), at the cost of more merges for short K.
-    out.tc_segment = opts.tc_segment > 0 ? opts.tc_segment : (p.k >= 2048 ? 128 : p.k > 1024 ? 64 : 32);
+    out.tc_segment = tc_segment(opts, p.k);
     out.beta_zero = p.br == 0.0f && p.bi == 0.0f;
     if (sm_count <= 0) {
         sm_count = 148;
@@ -261,7 +279,6 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
     // ---- tile x K-partition search -------------------------------------------
     const TileChoice* tiles = tc ? kTcTiles : kFp32Tiles;
     const int granule = tc ? 64 : 16;
-    const int ntiles = 1;
     const uint64_t default_tiles = (uint64_t)ceil_div(p.m, tiles[0].bm) * ceil_div(p.n, tiles[0].bn);
     TileChoice best_tile = tiles[0];
     int best_parts = 1;
@@ -287,34 +304,21 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
                 best_parts = parts;
             }
         }
-    } else if (default_tiles < (uint64_t)sm_count * tiles[0].slots_per_sm && !out.rounding) {
-        // Few tiles: search jointly (SelectCgemm3mDecomposition, :174-200).
-        // Partitions are bounded by what can still fill the machine: at most
-        // 4-way as in the reference when tiles are plentiful, deeper only while
-        // tiles x parts stays within two waves of SM slots and every partition
-        // keeps >= 256 K terms.
-        uint64_t best = std::numeric_limits<uint64_t>::max();
-        for (int t = 0; t < ntiles; ++t) {
-            const uint64_t nt = (uint64_t)ceil_div(p.m, tiles[t].bm) * ceil_div(p.n, tiles[t].bn);
-            const uint64_t slots = (uint64_t)sm_count * tiles[t].slots_per_sm;
-            int max_parts = (int)std::max<uint64_t>(4, (2 * slots) / std::max<uint64_t>(nt, 1));
-            max_parts = std::min(max_parts, 64);
-            for (int parts = 1; parts <= max_parts; ++parts) {
-                const int span = k_span(p.k, parts, granule);
-                if ((parts - 1) * span >= p.k) {
-                    continue;
-                }
-                if (parts > 4 && span < 256) {
-                    continue;
-                }
-                const uint64_t work = core_work(tiles[t], p.m, p.n, parts, sm_count) * (uint64_t)(span + 16);
-                // Charge the partial-output traffic of the merge: 2 planes per part.
-                const uint64_t merge = parts > 1 ? (uint64_t)parts * p.m * p.n / sm_count : 0;
-                if (work + merge < best) {
-                    best = work + merge;
-                    best_tile = tiles[t];
-                    best_parts = parts;
-                }
+    } else if (!out.rounding) {
+        // Tensor-core forms: the split with the least estimated time
+        // (SelectCgemm3mDecomposition's joint search, :174-200, over one tile).
+        // Partitions keep >= 128 K terms, >= 256 beyond the reference's four.
+        double best = std::numeric_limits<double>::max();
+        for (int parts = 1; parts <= 64; ++parts) {
+            const int span = k_span(p.k, parts, granule);
+            if (parts > 1 && ((parts - 1) * span >= p.k || span < (parts > 4 ? 256 : 128))) {
+                continue;
+            }
+            const double us =
+                tc_time_us(p, opts.form, out.tc_segment, parts, parts > 1 ? span : p.k, sm_count);
+            if (us < best) {
+                best = us;
+                best_parts = parts;
             }
         }
     }
@@ -372,14 +376,14 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
     // form's, which every form promises not to exceed -- and reports form
     // FP32.  engine 1 (or a forced K split) keeps the tensor-core path.
     if (tc) {
-        out.est_us = tc_time_us(p, opts.form, out.parts, out.span, sm_count);
+        out.est_us = tc_time_us(p, opts.form, out.tc_segment, out.parts, out.span, sm_count);
     }
     if (tc && !out.rounding && opts.engine == 0 && opts.k_partitions <= 0) {
         cg3mOptions fo = opts;
         fo.form = CG3M_FORM_FP32;
         fo.rounding = CG3M_ROUNDING_OFF;
         Plan fp;
-        if (make_plan(p, fo, sm_count, &fp) && fp.est_us * 1.1 < out.est_us) {
+        if (make_plan(p, fo, sm_count, &fp) && fp.est_us * 1.05 < out.est_us) {
             *plan = fp;
             return true;
         }
@@ -418,20 +422,9 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
     out.partial_pitch = (int)align_up((size_t)p.m, 32);
     out.partial_plane_elems = (size_t)out.partial_pitch * p.n;
     // K splits merged on chip through the tile's cluster: the FP32 GEMM (up to 8
-    // partitions) and the tensor-core CTA-pair kernel (used for m > 128; up to 4
-    // partitions, two CTAs each).  The pair kernel merges on chip only when all
-    // of its clusters of 2 x parts CTAs are resident at once: a grid that one
-    // wave holds as loose CTAs but not as clusters runs a second wave, which
-    // costs more than the merge launch it saves (1.3-1.6x on 128..144-CTA grids).
-    bool tc_merge = false;
-    if (tc && p.m > 128 && out.parts <= 4) {
-        const uint64_t pair_tiles = (uint64_t)ceil_div(p.m, 256) * ceil_div(p.n, 128);
-        const uint64_t cap =
-            std::max<uint64_t>(1, kClusterCapOneBlock[2 * out.parts - 1] * (uint64_t)sm_count / 148);
-        tc_merge = pair_tiles <= cap;
-    }
+    // partitions) and the tensor-core CTA-pair kernel (up to 4, two CTAs each).
     out.cluster_merge = !out.rounding && out.parts > 1 &&
-                        (tc ? tc_merge
+                        (tc ? tc_cluster_merge(p, out.parts, sm_count)
                             : (out.parts <= kClusterMergeMax && out.tile_m == 128 && out.tile_n == 64));
     out.partial_off = off;
     if (out.parts > 1 && !out.cluster_merge) {
