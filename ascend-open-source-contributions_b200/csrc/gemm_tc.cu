@@ -349,6 +349,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();  // the pack kernel's planes
 
     // Work order (producer and MMA issuer walk it identically): for each K
     // segment, for each component c in {re, im, sum}, for each K-block of the
@@ -955,6 +956,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     cluster_sync();  // both CTAs' barriers initialised, TMEM allocated in both
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();  // the pack kernel's planes
 
     if (warp == 0) {
         // ---------------- TMA producer (both CTAs) ----------------
@@ -1267,13 +1269,17 @@ cudaError_t launch_pair(cudaStream_t stream, const Problem& pr, const Plan& plan
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = G::SMEM;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = p.cluster_merge ? (unsigned)plan.parts : 1u;
     attr[0].val.clusterDim.z = 1;
+    // Straight after the pack kernel.  Not in the rounding pass, where blocks of
+    // taken tiles return without waiting for it.
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = skip_count == nullptr ? 2 : 1;
     err = cudaLaunchKernelEx(&cfg, kernel, ta, tb, p);
     return err != cudaSuccess ? err : cudaGetLastError();
 }
@@ -1328,9 +1334,18 @@ cudaError_t launch_form(cudaStream_t stream, const Problem& pr, const Plan& plan
     if (err != cudaSuccess) {
         return err;
     }
-    const dim3 grid((unsigned)(p.tiles_m * p.tiles_n), (unsigned)plan.parts);
-    kernel<<<grid, kThreads, G::SMEM, stream>>>(ta, tb, p);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(p.tiles_m * p.tiles_n), (unsigned)plan.parts);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = G::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // after the pack kernel
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    err = cudaLaunchKernelEx(&cfg, kernel, ta, tb, p);
+    return err != cudaSuccess ? err : cudaGetLastError();
 }
 
 template <int LEAD>

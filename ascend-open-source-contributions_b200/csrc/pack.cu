@@ -21,6 +21,7 @@
 #include <cuda_bf16.h>
 
 #include "cg3m_internal.h"
+#include "ptx.cuh"
 
 namespace cg3m {
 namespace {
@@ -128,6 +129,9 @@ template <int FORM, bool REST = false>
 __global__ void __launch_bounds__(TILE* ROWS) pack_kernel(PackSide a, PackSide b)
 {
     __shared__ float2 tile[TILE][TILE + 1];
+    // The GEMM's blocks set up (barriers, TMEM, tensor maps) on the SMs this
+    // kernel's last blocks leave free; they wait for its end before they read.
+    pdl_launch_dependents();
     // Block x of side z covers tiles x, x + gridDim.x, ... of that side's own
     // tile grid (tile t at (t mod tiles_r, t / tiles_r)), so a long-K shape
     // launches no blocks over the other side's extent.  The full packs launch

@@ -311,6 +311,16 @@ __device__ __forceinline__ bool elect_one()
 // the abort flag, made the same for all lanes before the warp branches on them.
 __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffffu, ok); }
 
+// ---- programmatic dependent launch ---------------------------------------------
+
+// In a kernel launched with programmatic stream serialization: waits until the
+// kernel before it has completed and its writes are visible.  Every thread of
+// the grid calls it, so the kernel completes after its predecessor.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// In the kernel before: the next one's blocks may start once every block of
+// this one has got here.
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- CTA pairs (cluster of 2, cta_group::2) -----------------------------------
 
 __device__ __forceinline__ uint32_t cluster_ctarank()
