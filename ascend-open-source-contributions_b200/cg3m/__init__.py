@@ -356,9 +356,9 @@ def stage_names(info):
                      "lane_major", "replay_outputs"]
         else:
             # packed rows with the leading planes and the energies first; the
-            # risk-plane GEMM selects; the rest of the planes only for the bands
-            # the form's products read
-            names = ["pack_rows", "energy", "gemm_path", "exact_split", "band_need", "pack_rest",
+            # risk-plane GEMM selects; the residues and the rest of the planes
+            # only for the bands the exact and the form's products read
+            names = ["pack_rows", "energy", "gemm_path", "band_need", "exact_split", "pack_rest",
                      "gemm_form_tiles", "exact_tiles", "exact_crt", "lanes_needed", "lane_major",
                      "recompute_fp64_outputs", "fallback_fp64"]
     else:

@@ -183,11 +183,14 @@ enum : int {
 // tile with more than kSparseMax flagged outputs.
 constexpr int kOzakiTile = 256;
 
+constexpr int kOzNonFinite = 1 << 20;  // exponent marker: the row or column holds Inf/NaN
+constexpr int kOzZero = -(1 << 20);    // exponent marker: the row or column is all zero
+
 // Exponents, rounding counts, residue planes and product residues of the
 // tensor-core forms' exact recompute (ozaki.cu), carved from the rounding
 // region.
 struct OzLayout {
-    int* E = nullptr;            // op(A) row exponents
+    int* E = nullptr;            // op(A) row exponents (written with the energies)
     int* F = nullptr;            // op(B) column exponents
     int* CA = nullptr;           // rounded parts per op(A) row
     int* CB = nullptr;           // rounded parts per op(B) column
@@ -202,9 +205,11 @@ struct OzLayout {
     size_t bytes = 0;
 };
 OzLayout oz_layout(int n, uint8_t* base, std::vector<size_t>* guards = nullptr);
-// Residues of op(A) rows and op(B) columns (needs only the packed rows).
+// Residues of the op(A) rows and op(B) columns in the 256-row bands marked
+// (needs the packed rows and the exponents).
 cudaError_t launch_ozaki_split(cudaStream_t s, int n, int pitch, const ColPanel& panel, const float2* rows_a,
-                               const float2* rows_b, const OzLayout& L);
+                               const float2* rows_b, const OzLayout& L, const uint8_t* band_a,
+                               const uint8_t* band_b);
 // The exact products of every tile marked in L.tile_ran and their
 // reconstruction into every output of those tiles; outputs it cannot certify
 // are marked in fallback_bits.  Two launches; mark(i) after the i-th (1-based).

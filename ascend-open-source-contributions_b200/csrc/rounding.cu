@@ -55,25 +55,51 @@ constexpr float kConfidence = 3.75f;  // CGEMM_ROUNDING_CONFIDENCE, cgemm_host.c
 
 // ---- 2. energies ----------------------------------------------------------------
 
+// EXP (the tensor-core forms): also the exponent of the exact recompute, e with
+// 2^(e-1) <= the row's largest part < 2^e, to E (op(A) rows) and F (op(B)
+// columns), or a marker for an all-zero row or one that holds Inf/NaN.
+template <bool EXP>
 __global__ void __launch_bounds__(kLanes) energy_kernel(const float2* __restrict__ rows_a,
                                                         const float2* __restrict__ rows_b, int n, int pitch,
-                                                        int span, float* __restrict__ energy, int nrows_a, int j0)
+                                                        int span, float* __restrict__ energy, int nrows_a, int j0,
+                                                        int* __restrict__ E, int* __restrict__ F)
 {
     __shared__ float lanes[kLanes];
+    __shared__ float wmax[2];
     const int r = panel_row(blockIdx.x, nrows_a, n, j0);
     const float2* src = r < n ? rows_a + (size_t)r * pitch : rows_b + (size_t)(r - n) * pitch;
     // Each lane reads its own span of consecutive terms straight from global
     // memory (no staged row, so many rows are in flight per SM); the sector a
     // thread fetches serves its next terms from L1.
     const int l = threadIdx.x;
-    float e = 0.0f;
+    float e = 0.0f, top = 0.0f;
+    bool bad = false;
     const int k0 = l * span, k1 = min(n, k0 + span);
     for (int k = k0; k < k1; ++k) {
         const float2 x = __ldg(src + k);
         e = __fmaf_rn(x.x, x.x, e);
         e = __fmaf_rn(x.y, x.y, e);
+        if constexpr (EXP) {
+            top = fmaxf(top, fmaxf(fabsf(x.x), fabsf(x.y)));  // fmaxf drops a NaN
+            bad |= x.x != x.x || x.y != x.y;
+        }
     }
     lanes[l] = e;
+    if constexpr (EXP) {
+#pragma unroll
+        for (int off = 16; off >= 1; off /= 2) {
+            top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+        }
+        if ((l & 31) == 0) {
+            wmax[l >> 5] = top;
+        }
+        bad = __syncthreads_or(bad);
+        if (l == 0) {
+            top = fmaxf(wmax[0], wmax[1]);
+            const int ex = bad || isinf(top) ? kOzNonFinite : top > 0.0f ? ilogbf(top) + 1 : kOzZero;
+            (r < n ? E : F)[r < n ? r : r - n] = ex;
+        }
+    }
     __syncthreads();
     for (int stride = kLanes / 2; stride >= 1; stride /= 2) {
         if (l < stride) {
@@ -162,13 +188,19 @@ __global__ void select_kernel(int n, const float2* __restrict__ C, const float* 
 // tiles holds more than kSparseMax flagged outputs.  Otherwise the form's
 // products run there (the pair kernel's own test of the same counts) and read
 // that row band of op(A) and column band of op(B), so both bands are marked
-// for the rest of the pack.
+// for the rest of the pack; a taken tile marks them for the residues.
 static_assert(kOzakiTile / kTile == 16, "16 x 16 count tiles per exact tile");
-// The planes of an op(A) band packed for an earlier panel stay: band_a holds one
-// array of kMaxBands per panel, and a band is marked in the first that needs it.
+// What an op(A) band got for an earlier panel stays: its marks are one array of
+// kMaxBands per panel, and a band is marked in the first that needs it.  Marks
+// (BandMarks): op(B) bands, then the op(A) arrays.
+struct BandMarks {
+    uint8_t* rest;  // the rest of the planes
+    uint8_t* ran;   // the residues
+    __host__ __device__ static size_t bytes() { return (size_t)(kMaxPanels + 1) * kMaxBands; }
+    __host__ __device__ static uint8_t* a(uint8_t* marks, int panel) { return marks + (panel + 1) * kMaxBands; }
+};
 __global__ void __launch_bounds__(256) band_need_kernel(int n, int band0, int panel,
-                                                         const uint32_t* __restrict__ tile_count,
-                                                         uint8_t* __restrict__ band_a, uint8_t* __restrict__ band_b,
+                                                         const uint32_t* __restrict__ tile_count, BandMarks marks,
                                                          uint8_t* __restrict__ tile_ran, uint32_t* __restrict__ stats)
 {
     const int bj = band0 + blockIdx.y;
@@ -185,16 +217,16 @@ __global__ void __launch_bounds__(256) band_need_kernel(int n, int band0, int pa
             const int rows = min(kOzakiTile, n - (int)blockIdx.x * kOzakiTile);
             const int cols = min(kOzakiTile, n - bj * kOzakiTile);
             atomicAdd(&stats[kStatExactOutputs], (uint32_t)(rows * cols));
-        } else {
-            bool packed = false;
-            for (int q = 0; q < panel; ++q) {
-                packed |= band_a[q * kMaxBands + blockIdx.x] != 0;
-            }
-            if (!packed) {
-                band_a[panel * kMaxBands + blockIdx.x] = 1;
-            }
-            band_b[bj] = 1;
         }
+        uint8_t* const m = run ? marks.ran : marks.rest;
+        bool done = false;
+        for (int q = 0; q < panel; ++q) {
+            done |= BandMarks::a(m, q)[blockIdx.x] != 0;
+        }
+        if (!done) {
+            BandMarks::a(m, panel)[blockIdx.x] = 1;
+        }
+        m[bj] = 1;
     }
     if (run) {
         const uint32_t flagged = __reduce_add_sync(0xffffffffu, count);
@@ -567,7 +599,8 @@ __global__ void __launch_bounds__(256) lane_major_kernel(int n, int pitch, int s
 {
     extern __shared__ float2 row[];
     const int r = panel_row(blockIdx.x, n, n, j0);
-    if (need[r] != 1) {
+    // need[2n + r]: op(A) row r was copied for an earlier panel
+    if (!need[r] || (r < n && need[2 * n + r])) {
         return;  // no output the per-output kernels recompute lies in this row or column, or it was copied
     }
     const size_t width = (size_t)kLanes * span;
@@ -577,8 +610,8 @@ __global__ void __launch_bounds__(256) lane_major_kernel(int n, int pitch, int s
         row[k] = src[k];
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        need[r] = 2;  // copied: a later panel need not
+    if (threadIdx.x == 0 && r < n) {
+        need[2 * n + r] = 1;
     }
     for (int f = threadIdx.x; f < (int)width; f += blockDim.x) {
         const int sidx = f / kLanes, l = f % kLanes;
@@ -638,9 +671,7 @@ __global__ void __launch_bounds__(256) lanes_needed_kernel(int n, int tc, const 
                           : tile_count[(size_t)(j / kTile) * tiles16 + i / kTile] <= kSparseMax;
             }
             if (want) {
-                if (need[i] == 0) {  // 2: an earlier panel copied it
-                    need[i] = 1;
-                }
+                need[i] = 1;
                 need[n + j] = 1;
             }
         }
@@ -914,16 +945,16 @@ struct RoundLayout {
     uint32_t* tile_count;
     uint32_t* stats;
     uint32_t* fallback_bits;
-    uint8_t* need;      // rows of op(A), then columns of op(B), the per-output kernels read
-    uint8_t* band;      // [kMaxBands] op(B) column bands, then per panel [kMaxBands] op(A) row bands, of
-                        // 256 whose tiles the form's products read (tensor-core forms)
+    uint8_t* need;      // rows of op(A), then columns of op(B), the per-output kernels read; then the op(A)
+                        // rows whose lane-major copy is made
+    BandMarks marks;    // 256-row bands whose tiles the form's products, the residues read (tensor-core forms)
     size_t zero_bytes;  // tile_count + stats + fallback_bits + need + band, one memset
     OzLayout oz;
 };
 
 static size_t flag_words(int n) { return ((size_t)n * n + 31) / 32; }
-static size_t need_words(int n) { return ((size_t)2 * n + 3) / 4; }
-static size_t band_words() { return (size_t)(kMaxPanels + 1) * kMaxBands / 4; }
+static size_t need_words(int n) { return ((size_t)3 * n + 3) / 4; }
+static size_t band_words() { return 2 * BandMarks::bytes() / 4; }
 static size_t tile_words(int n)
 {
     const size_t t = (size_t)(n + kTile - 1) / kTile;
@@ -992,7 +1023,8 @@ static RoundLayout round_layout(const Plan& plan, void* ws, int n)
     L.stats = L.tile_count + tile_words(n);
     L.fallback_bits = L.stats + kStatWords;
     L.need = reinterpret_cast<uint8_t*>(L.fallback_bits + flag_words(n));
-    L.band = L.need + need_words(n) * 4;
+    L.marks.rest = L.need + need_words(n) * 4;
+    L.marks.ran = L.marks.rest + BandMarks::bytes();
     L.zero_bytes = (tile_words(n) + kStatWords + flag_words(n) + need_words(n) + band_words()) * 4;
     if (plan.form != CG3M_FORM_FP32) {
         L.oz = oz_layout(n, b + o.oz);
@@ -1058,7 +1090,7 @@ static cudaError_t launch_replay(cudaStream_t s, int n, int span, const RoundLay
 
 int rounding_prep_kernels(int form)
 {
-    return form == CG3M_FORM_FP32 ? 2 : 1;  // FP32: packed rows, energies; tensor-core forms: residues
+    return form == CG3M_FORM_FP32 ? 2 : 0;  // FP32: packed rows, energies
 }
 
 // Tensor-core forms: zero the selection's outputs (its flag words too, which
@@ -1082,8 +1114,8 @@ cudaError_t launch_rounding_pack(cudaStream_t s, const Problem& p, const Plan& p
     if (err == cudaSuccess) {
         const int span = ((n + kLanes - 1) / kLanes) | 1;
         const int nrows_a = panel.index == 0 ? n : 0;
-        energy_kernel<<<nrows_a + panel.j1 - panel.j0, kLanes, 0, s>>>(L.rows_a, L.rows_b, n, pitch, span, L.energy,
-                                                                       nrows_a, panel.j0);
+        energy_kernel<true><<<nrows_a + panel.j1 - panel.j0, kLanes, 0, s>>>(
+            L.rows_a, L.rows_b, n, pitch, span, L.energy, nrows_a, panel.j0, L.oz.E, L.oz.F);
         err = cudaGetLastError();
         mark();
     }
@@ -1099,17 +1131,15 @@ cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& p
     const int span = ((n + kLanes - 1) / kLanes) | 1;
     int count = 0;
     cudaError_t err = cudaSuccess;
+    (void)panel;  // only the FP32 form prepares anything here
     if (plan.form == CG3M_FORM_FP32) {  // the tensor-core forms packed their rows and energies first
         err = launch_pack_rows(s, p, L.rows_a, L.rows_b, pitch);
         mark(++count);
     }
     if (err == cudaSuccess && plan.form == CG3M_FORM_FP32) {
-        energy_kernel<<<2 * n, kLanes, 0, s>>>(L.rows_a, L.rows_b, n, pitch, span, L.energy, n, 0);
+        energy_kernel<false><<<2 * n, kLanes, 0, s>>>(L.rows_a, L.rows_b, n, pitch, span, L.energy, n, 0, nullptr,
+                                                      nullptr);
         err = cudaGetLastError();
-        mark(++count);
-    }
-    if (err == cudaSuccess && plan.form != CG3M_FORM_FP32) {
-        err = launch_ozaki_split(s, n, pitch, panel, L.rows_a, L.rows_b, L.oz);
         mark(++count);
     }
     if (launched != nullptr) {
@@ -1187,19 +1217,23 @@ cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan&
         // The rest of the form's planes is packed for the bands those tiles read.
         const int bands = (n + kOzakiTile - 1) / kOzakiTile;
         const int band0 = panel.j0 / kOzakiTile, panel_bands = ceil_div(panel.j1, kOzakiTile) - band0;
-        uint8_t* const band_b = L.band;
-        uint8_t* const band_a = L.band + kMaxBands;
         if (err == cudaSuccess && (bands > kMaxBands || panel.index >= kMaxPanels)) {
             err = cudaErrorInvalidValue;  // beyond the gated orders
         }
         if (err == cudaSuccess) {
-            band_need_kernel<<<dim3(bands, panel_bands), 256, 0, s>>>(n, band0, panel.index, L.tile_count, band_a,
-                                                                     band_b, L.oz.tile_ran, L.stats);
+            band_need_kernel<<<dim3(bands, panel_bands), 256, 0, s>>>(n, band0, panel.index, L.tile_count, L.marks,
+                                                                     L.oz.tile_ran, L.stats);
             err = cudaGetLastError();
             mark(++count);
         }
         if (err == cudaSuccess) {
-            err = launch_pack(s, p, plan, ws, band_a + panel.index * kMaxBands, band_b, BatchStrides{}, &panel);
+            err = launch_ozaki_split(s, n, pitch, panel, L.rows_a, L.rows_b, L.oz,
+                                     BandMarks::a(L.marks.ran, panel.index), L.marks.ran);
+            mark(++count);
+        }
+        if (err == cudaSuccess) {
+            err = launch_pack(s, p, plan, ws, BandMarks::a(L.marks.rest, panel.index), L.marks.rest, BatchStrides{},
+                              &panel);
             mark(++count);
         }
         if (err == cudaSuccess) {
