@@ -21,7 +21,6 @@
 #include <cuda_bf16.h>
 
 #include "cg3m_internal.h"
-#include "ptx.cuh"
 
 namespace cg3m {
 namespace {
@@ -58,14 +57,14 @@ __device__ __forceinline__ float tf32_rna(float x)
 // Writes the planes of one component value v (component c in 0..2).  REST:
 // all but the leading split term of re and im (written with the packed rows).
 template <int FORM, bool REST = false>
-__device__ __forceinline__ void put(const PackSide& s, int c, size_t idx, float v)
+__device__ __forceinline__ void put(const PackSide& s, void* out, int c, size_t idx, float v)
 {
     if constexpr (FORM == CG3M_FORM_FP32) {
-        static_cast<float*>(s.out)[c * s.plane_elems + idx] = v;
+        static_cast<float*>(out)[c * s.plane_elems + idx] = v;
     } else if constexpr (FORM == CG3M_FORM_TF32X3) {
         const float hi = tf32_rna(v);
         const float lo = tf32_rna(v - hi);
-        float* o = static_cast<float*>(s.out);
+        float* o = static_cast<float*>(out);
         if (!REST || c == 2) {
             o[(2 * c) * s.plane_elems + idx] = hi;
         }
@@ -76,7 +75,7 @@ __device__ __forceinline__ void put(const PackSide& s, int c, size_t idx, float 
         const __nv_bfloat16 b1 = __float2bfloat16_rn(r1);
         const float r2 = r1 - __bfloat162float(b1);
         const __nv_bfloat16 b2 = __float2bfloat16_rn(r2);
-        __nv_bfloat16* o = static_cast<__nv_bfloat16*>(s.out);
+        __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
         if (!REST || c == 2) {
             o[(3 * c) * s.plane_elems + idx] = b0;
         }
@@ -98,12 +97,12 @@ constexpr int kFormRowsBf16 = 102;
 
 // One element of op(X) at plane row prow, plane column pcol.
 template <int FORM, bool REST = false>
-__device__ __forceinline__ void put_all(const PackSide& s, int prow, int pcol, float2 v)
+__device__ __forceinline__ void put_all(const PackSide& s, void* out, int prow, int pcol, float2 v)
 {
     const float re = v.x;
     const float im = v.y * s.conj;
     if constexpr (FORM == kFormRows || FORM == kFormRowsTf32 || FORM == kFormRowsBf16) {
-        static_cast<float2*>(s.out)[(size_t)prow * s.pitch + pcol] = make_float2(re, im);
+        static_cast<float2*>(out)[(size_t)prow * s.pitch + pcol] = make_float2(re, im);
         const size_t li = (size_t)prow * s.lead_pitch + pcol;
         if constexpr (FORM == kFormRowsTf32) {
             float* o = static_cast<float*>(s.lead);
@@ -117,9 +116,9 @@ __device__ __forceinline__ void put_all(const PackSide& s, int prow, int pcol, f
         return;
     }
     const size_t idx = (size_t)prow * s.pitch + pcol;
-    put<FORM, REST>(s, 0, idx, re);
-    put<FORM, REST>(s, 1, idx, im);
-    put<FORM, REST>(s, 2, idx, __fadd_rn(re, im));
+    put<FORM, REST>(s, out, 0, idx, re);
+    put<FORM, REST>(s, out, 1, idx, im);
+    put<FORM, REST>(s, out, 2, idx, __fadd_rn(re, im));
 }
 
 constexpr int TILE = 32;
@@ -130,16 +129,17 @@ __global__ void __launch_bounds__(TILE* ROWS) pack_kernel(PackSide a, PackSide b
 {
     __shared__ float2 tile[TILE][TILE + 1];
     // The GEMM's blocks set up (barriers, TMEM, tensor maps) on the SMs this
-    // kernel's last blocks leave free; they wait for its end before they read.
-    pdl_launch_dependents();
+    // kernel's last blocks leave.  Their exits trigger that launch: an explicit
+    // trigger in every block cost 10 % of a large pack (1266 x 25 x 18768: 102 ->
+    // 114 us), and one in the last wave's blocks as much.
     // Block x of side z covers tiles x, x + gridDim.x, ... of that side's own
     // tile grid (tile t at (t mod tiles_r, t / tiles_r)), so a long-K shape
     // launches no blocks over the other side's extent.  The full packs launch
     // one block per tile; the rest of the planes in the rounding pass uses a
     // smaller grid, as most of its tiles may lie in bands it skips.
-    PackSide s = blockIdx.z == 0 ? a : b;
-    s.src += (long long)blockIdx.y * s.src_batch;
-    s.out = static_cast<uint8_t*>(s.out) + blockIdx.y * s.out_batch;
+    const PackSide& s = blockIdx.z == 0 ? a : b;
+    const float2* const src = s.src + (long long)blockIdx.y * s.src_batch;
+    void* const out = static_cast<uint8_t*>(s.out) + blockIdx.y * s.out_batch;
     const int tiles_r = (s.rows + TILE - 1) / TILE;
     const long long tiles = (long long)tiles_r * ((s.cols + TILE - 1) / TILE);
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -160,8 +160,8 @@ __global__ void __launch_bounds__(TILE* ROWS) pack_kernel(PackSide a, PackSide b
                 for (int q = 0; q < TILE / ROWS; ++q) {
                     const int c = c0 + ty + q * ROWS;
                     if (c < s.cols) {
-                        const float2 v = __ldg(&s.src[(size_t)c * s.ld + r]);
-                        put_all<FORM, REST>(s, c, r, v);
+                        const float2 v = __ldg(&src[(size_t)c * s.ld + r]);
+                        put_all<FORM, REST>(s, out, c, r, v);
                     }
                 }
             }
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(TILE* ROWS) pack_kernel(PackSide a, PackSide b
             for (int q = 0; q < TILE / ROWS; ++q) {
                 const int c = c0 + ty + q * ROWS;
                 if (r < s.rows && c < s.cols) {
-                    tile[ty + q * ROWS][tx] = __ldg(&s.src[(size_t)c * s.ld + r]);
+                    tile[ty + q * ROWS][tx] = __ldg(&src[(size_t)c * s.ld + r]);
                 }
             }
         }
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(TILE* ROWS) pack_kernel(PackSide a, PackSide b
             for (int q = 0; q < TILE / ROWS; ++q) {
                 const int r = r0 + ty + q * ROWS;
                 if (r < s.rows) {
-                    put_all<FORM, REST>(s, r, c, tile[tx][ty + q * ROWS]);
+                    put_all<FORM, REST>(s, out, r, c, tile[tx][ty + q * ROWS]);
                 }
             }
         }

@@ -317,9 +317,6 @@ __device__ __forceinline__ bool warp_all(bool ok) { return __all_sync(0xffffffff
 // kernel before it has completed and its writes are visible.  Every thread of
 // the grid calls it, so the kernel completes after its predecessor.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// In the kernel before: the next one's blocks may start once every block of
-// this one has got here.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ---- CTA pairs (cluster of 2, cta_group::2) -----------------------------------
 
