@@ -900,21 +900,24 @@ constexpr Policy kDefaultPolicy = {4096, 4};
 // tiles load more shared memory per FMA.
 constexpr double kTileEfficiency[kTileCount] = {1.0, 1.0, 0.93, 0.88, 0.87, 0.75};
 
+// Preference for large tiles, of the chain bound in make_strided_plan.
+constexpr double kLargeTiles[kTileCount] = {1.0, 0.85, 0.8, 0.8, 0.65, 0.45};
+
 int span_for(int k, int parts) { return ceil_div(ceil_div(k, 16), parts) * 16; }
 
 // The allowed tile with the least estimated time for p; returns that time
 // (padded work over efficiency) and sets tile, tiles_m, tiles_n.
-double choose_tile(BProblem& p, int max_area, int mode)
+double choose_tile(BProblem& p, int max_area, int first_tile = 1, const double* efficiency = kTileEfficiency)
 {
     int best = kTileCount - 1;
     double best_cost = 1e300;
-    for (int t = 0; t < kTileCount; ++t) {
-        if (t == 0 || tile_bm(t) * tile_bn(t) > max_area) {
+    for (int t = first_tile; t < kTileCount; ++t) {
+        if (tile_bm(t) * tile_bn(t) > max_area) {
             continue;
         }
         const double work =
             (double)ceil_div(p.m, tile_bm(t)) * ceil_div(p.n, tile_bn(t)) * tile_bm(t) * tile_bn(t) * (p.k + 16);
-        const double cost = work / kTileEfficiency[t];
+        const double cost = work / efficiency[t];
         if (cost < best_cost) {
             best_cost = cost;
             best = t;
@@ -927,11 +930,11 @@ double choose_tile(BProblem& p, int max_area, int mode)
 }
 
 // K partitions of p given the schedule's average work per SM.
-void choose_parts(BProblem& p, int split_cap, double per_sm)
+void choose_parts(BProblem& p, int split_cap, double per_sm, const double* efficiency = kTileEfficiency)
 {
     int parts = 1;
     if (split_cap > 1 && p.k >= 256) {
-        const double task = (double)tile_bm(p.tile) * tile_bn(p.tile) * (p.k + 16) / kTileEfficiency[p.tile];
+        const double task = (double)tile_bm(p.tile) * tile_bn(p.tile) * (p.k + 16) / efficiency[p.tile];
         const int want = (int)std::ceil(task / (0.25 * per_sm));
         parts = std::max(1, std::min({want, split_cap, p.k / 128}));
     }
@@ -950,7 +953,7 @@ void apply_policy(std::vector<BProblem>& ps, const Policy& pol, int sm_count)
 {
     double total = 0.0;
     for (auto& p : ps) {
-        total += choose_tile(p, pol.max_area, kMode3M);
+        total += choose_tile(p, pol.max_area);
     }
     const double per_sm = total / std::max(sm_count, 1);
     for (auto& p : ps) {
@@ -1137,7 +1140,8 @@ int single_tile_bn(int tile) { return tile_bn(tile); }
 // time a block needs by itself.  Blocks that share an SM add a per-term cost
 // for every layer of clusters: one layer holds as many as fit with one block
 // per SM, which is fewer than sm_count / parts (GPC boundaries), so a split
-// of 7 or 8 starts its second layer at 105 or 120 blocks.
+// of 7 or 8 starts its second layer at 105 or 120 blocks.  Beyond kShortChain
+// terms the layers are those that the clusters need at several blocks per SM.
 namespace {
 struct SingleCost {
     double base_us, fixed_us, term_ns, shared_term_ns, merge_us;
@@ -1173,6 +1177,13 @@ bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, Stri
     bp.n = p.n;
     bp.k = p.k;
     const long long sms = std::max(sm_count, 1);
+    // A chain's rounding error grows with the square root of its terms: beyond
+    // kShortChain terms no longer than where a task of a large tile takes a
+    // quarter of an SM's work (at most four partitions), whatever is faster.
+    BProblem ref = bp;
+    const double one = choose_tile(ref, 8192, mode == kMode4M ? 1 : 0, kLargeTiles);
+    choose_parts(ref, 4, one * batch / (double)sms, kLargeTiles);
+    const int chain = std::max(kShortChain, ref.span);
     double best = 1e300;
     for (int t = 1; t < kTileCount; ++t) {
         const int tm = ceil_div(p.m, tile_bm(t)), tn = ceil_div(p.n, tile_bn(t));
@@ -1180,7 +1191,7 @@ bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, Stri
         const SingleCost& c = kSingleCost[t];
         for (int q = 1; q <= 8; ++q) {
             const int span = q == 1 ? p.k : span_for(p.k, q);
-            if (q > 1 && (span < 48 || (q - 1) * span >= p.k)) {
+            if (span > chain || (q > 1 && (span < 48 || (q - 1) * span >= p.k))) {
                 continue;
             }
             const long long tasks = (long long)tm * tn * batch * q;
@@ -1230,8 +1241,13 @@ double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile,
                    int* parts)
 {
     sm_count = std::max(sm_count, 1);
-    double best = 1e300;
-    int bt = kTileCount - 1, bp = 1;
+    double best[kMaxClusterParts + 1];
+    int best_tile[kMaxClusterParts + 1];
+    for (int q = 0; q <= kMaxClusterParts; ++q) {
+        best[q] = 1e300;
+        best_tile[q] = kTileCount - 1;
+    }
+    int bp = 1;
     for (int t = 0; t < kTileCount; ++t) {
         if ((forced_tile >= 0 && t != forced_tile) || (mode == kMode4M && t == 0)) {
             continue;
@@ -1249,7 +1265,21 @@ double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile,
             const long long cap = std::max<long long>(1, (long long)kClusterCap[occ - 1][q - 1] * sm_count / 148);
             const long long layer = std::max<long long>(1, (long long)kClusterCap[0][q - 1] * sm_count / 148);
             const long long waves = (tiles + cap - 1) / cap;
-            const long long load = (tiles + layer - 1) / layer;
+            long long load = (tiles + layer - 1) / layer;
+            if (k > kShortChain) {
+                // Long chains outlast the placement: full waves, then the fewest
+                // blocks per SM that hold the remaining clusters (25 x 1025 x
+                // 59274: 33 clusters of 8 are two layers, not three; 8 partitions
+                // took 438 us, 4, the least by whole layers, 549).
+                load = tiles / cap * occ;
+                if (const long long rest = tiles % cap) {
+                    int o = 1;
+                    while (o < occ && (long long)kClusterCap[o - 1][q - 1] * sm_count / 148 < rest) {
+                        ++o;
+                    }
+                    load += o;
+                }
+            }
             const SingleCost& c = kSingleCost[t];
             // Four-product mode: four FFMA per output and K term instead of
             // three (the per-term costs scaled by that ratio, not fitted).
@@ -1260,20 +1290,30 @@ double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile,
             if (q > 1) {
                 us += c.merge_us * q;
             }
-            if (us < best) {
-                best = us;
-                bt = t;
+            if (us < best[q]) {
+                best[q] = us;
+                best_tile[q] = t;
+                bp = us < best[bp] || best[bp] == 1e300 ? q : bp;
+            }
+        }
+    }
+    // A chain's rounding error grows with the square root of its terms: beyond
+    // kShortChain terms the finest split within 20 % of the least time.
+    if (k > kShortChain) {
+        const double least = best[bp];
+        for (int q = kMaxClusterParts; q > bp && span_for(k, bp) > kShortChain; --q) {
+            if (best[q] <= 1.2 * least) {
                 bp = q;
             }
         }
     }
     if (tile != nullptr) {
-        *tile = bt;
+        *tile = best_tile[bp];
     }
     if (parts != nullptr) {
         *parts = bp;
     }
-    return best;
+    return best[bp];
 }
 
 cudaError_t launch_single(cudaStream_t s, const Problem& p, int mode, int repair, int tile, int parts)

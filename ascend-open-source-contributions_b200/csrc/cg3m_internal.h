@@ -132,11 +132,12 @@ cudaError_t launch_merge(cudaStream_t s, const Problem& p, const Plan& plan, voi
 // packed rows, which also write the leading split planes the risk-plane GEMM
 // reads (launch_rounding_pack, instead of the full pack).  Then two halves:
 // the preparation reads only op(A) and op(B) (packed rows for the FP32 form,
-// energies and, for the tensor-core forms, the residues of the exact
+// energies and, for the tensor-core forms, the row exponents of the exact
 // recompute); the finish needs the GEMM's C and risk plane (FP32: selection,
 // then the recomputes; the tensor-core forms' risk-plane GEMM selected in its
-// epilogue, and they pack the rest of their planes in the finish, for the
-// bands whose tiles the exact recompute leaves to the form).  mark(i) is
+// epilogue; they make the exact recompute's residues in the finish, for the
+// bands of the tiles it takes, and pack the rest of their planes, for the bands
+// whose tiles it leaves to the form).  mark(i) is
 // called after the i-th kernel of each half (1-based) is enqueued.
 cudaError_t launch_rounding_pack(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const ColPanel& panel,
                                  const std::function<void()>& mark);
@@ -258,6 +259,8 @@ cudaError_t launch_single(cudaStream_t s, const Problem& p, int mode, int repair
 // The one-launch plan for an m x n x k problem in `mode`: tile and K
 // partitions (each forced when >= 0), chosen to minimise the estimated time,
 // which is returned in microseconds.
+// FP32 chains up to this many terms are split for speed alone.
+constexpr int kShortChain = 1024;
 double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile, int forced_parts, int* tile,
                    int* parts);
 int single_tile_bm(int tile);

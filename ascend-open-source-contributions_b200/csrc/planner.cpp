@@ -90,10 +90,14 @@ struct TileChoice {
 // 62.9 us, 128 x 64 x 4 parts 38.8 us; 1024^3: 306 vs 174 us).
 const TileChoice kFp32Tiles[] = {{128, 64, 1}};
 // Cost of one wave of 128 x 64 FP32 tiles in K terms of that tile (0.111 us
-// per term): a fixed part of about 56 terms (pipeline fill, epilogue, wave
-// launch; fitted with the microsecond model below) plus the span; the split-K
-// merge costs about 30 terms plus the partial planes it reads.
-constexpr uint64_t kFp32WaveFixed = 56;
+// per term): a fixed part (pipeline fill, epilogue, wave launch; 56 terms in the
+// microsecond model below) plus the span; the split-K merge costs about 30 terms
+// plus the partial planes it reads.  Beyond kShortChain terms splits are chosen
+// with a fixed part of 38 terms: as fast (75 timed shapes, 0.1 %), and finer
+// where the two differ (756 x 344 x 3425: 12 partitions 135.6 us, 3 149.8), which
+// keeps chains short: a chain's relative error grows as 2.6e-8 sqrt(terms)
+// (uniform data: 8.3e-7 at 1024 terms, 1.03e-6 at 1646, 1.43e-6 at 3125).
+constexpr uint64_t kFp32WaveFixed = 56, kLongWaveFixed = 38;
 constexpr uint64_t kMergeFixed = 30;
 constexpr uint64_t kMergeFloatsPerTerm = 41500;
 // With 2..8 partitions the partitions of a tile form one thread-block cluster
@@ -102,6 +106,9 @@ constexpr uint64_t kMergeFloatsPerTerm = 41500;
 // (cudaOccupancyMaxActiveClusters for one block per SM on 148 SMs), and the
 // merge costs about one K term per partition.
 constexpr int kClusterMergeMax = 8;
+// The fixed scratch of the allocation-free entry point and the workspace the
+// reference creates per handle, less what aligns and guards the regions.
+constexpr size_t kDefaultWorkspace = ((size_t)32 << 20) - ((size_t)64 << 10);
 constexpr uint64_t kClusterCapOneBlock[kClusterMergeMax] = {148, 74, 45, 33, 26, 22, 15, 15};
 
 uint64_t fp32_waves(uint64_t tiles, int parts, int sm_count)
@@ -123,6 +130,7 @@ constexpr double kMergeLaunchUs = 2.5;
 // The one-launch engine has to look faster by this much: its model errs by up
 // to 10 % where the two engines meet, the packed one's by 3 %.
 constexpr double kSingleMargin = 1.06;
+constexpr double kSingleGain = 0.7;
 // Tensor-core kernel tile (gemm_tc.cu): 128 x 128, one CTA per SM (TMEM).
 const TileChoice kTcTiles[] = {{128, 128, 1}};
 
@@ -287,6 +295,9 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
     } else if (!tc && !out.rounding) {
         // FP32: waves of 128 x 64 tiles at (span + fixed) each, plus the merge
         // (EstimateCgemmCoreWork's busiest-core work with measured B200 costs).
+        const size_t rows = align_up((size_t)p.m, 32), cols = align_up((size_t)p.n, 32);
+        const size_t planes = 12 * (rows + cols) * (size_t)p.k, partial = 8 * rows * (size_t)p.n;
+        const uint64_t fixed = p.k > kShortChain ? kLongWaveFixed : kFp32WaveFixed;
         uint64_t best = std::numeric_limits<uint64_t>::max();
         for (int parts = 1; parts <= 64; ++parts) {
             const int span = k_span(p.k, parts, granule);
@@ -294,13 +305,20 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
                 continue;
             }
             const uint64_t waves = fp32_waves(default_tiles, parts, sm_count);
-            const uint64_t gemm = waves * ((uint64_t)span + kFp32WaveFixed);
+            const uint64_t gemm = waves * ((uint64_t)span + fixed);
             const uint64_t merge =
                 parts > kClusterMergeMax ? kMergeFixed + (uint64_t)(2 * parts + 2) * p.m * p.n / kMergeFloatsPerTerm
                 : parts > 1              ? (uint64_t)parts
                                          : 0;
-            if (gemm + merge < best) {
-                best = gemm + merge;
+            // Beyond 32 partitions for a clear gain only (54 x 460 x 42520: 18
+            // partitions 372 us, 36 381; 128 x 128 x 65536: 32 295, 64 186), and
+            // not where the partials would push the call past a default workspace.
+            if (parts > 32 && planes <= kDefaultWorkspace && planes + (size_t)parts * partial > kDefaultWorkspace) {
+                break;
+            }
+            const uint64_t cost = (gemm + merge) * (parts > 32 ? 21 : 20);
+            if (cost < best) {
+                best = cost;
                 best_parts = parts;
             }
         }
@@ -354,7 +372,14 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
         int tile = 0, parts = 0;
         const double single = plan_single(p.m, p.n, p.k, 0, sm_count, -1, forced, &tile, &parts);
         out.est_us = packed_time_us(p, out.parts, out.span, default_tiles, sm_count);
-        if (single * kSingleMargin < out.est_us) {
+        // Chains up to twice as long as the packed split's (1.4 times the error)
+        // or short, or a clear gain: narrow outputs pad the packed tile several
+        // times over (25 x 1025 x 59274: 8 partitions in one launch 438 us, 26
+        // packed 1078).
+        const int single_span = parts > 1 ? k_span(p.k, parts) : p.k;
+        const bool chains = opts.k_partitions > 0 || single_span <= std::max(kShortChain, 2 * out.span) ||
+                            single < kSingleGain * out.est_us;
+        if (chains && single * kSingleMargin < out.est_us) {
             out.est_us = single;
             out.engine = 2;
             out.onchip_tile = tile;
