@@ -13,8 +13,8 @@
 // technique", 2025):
 //
 //   1. ozaki_split_kernel: every op(A) row i and op(B) column j gets a power
-//      of two 2^E > max |x| over the row (real and imaginary parts together);
-//      each part becomes the integer a = rn(x 2^(beta - E)), |a| <= 2^beta,
+//      of two 2^E > max |x| over the row (real and imaginary parts together;
+//      the energy kernel finds it); each part becomes the integer a = rn(x 2^(beta - E)), |a| <= 2^beta,
 //      beta = 47, and the row counts its parts for which a != x 2^(beta - E)
 //      (cA_i; cB_j for the columns).  Every prime factor of the kOzMods = 15
 //      moduli p_m <= 241 (pairwise coprime, product M ~ 2^111.1) is 1 mod 4, so
@@ -48,7 +48,7 @@
 // Two products per modulus instead of the four of Re = Ar Br - Ai Bi,
 // Im = Ar Bi + Ai Br: 30 int8 products of n^3 against 56 with 14 moduli that
 // need no square root of -1.  At 4096^3 with every tile dense: products 2.57 ->
-// 1.28 ms, residues 0.34 -> 0.30, reconstruction 0.21 -> 0.22.  A work unit is
+// 1.28 ms, residues 0.34 -> 0.29, reconstruction 0.21 -> 0.23.  A work unit is
 // 256 rows x 512 columns of one product, so 768 operand rows feed 256 x 512
 // outputs (12.1 GB from L2 in all, 9.4 TB/s) and both TMEM accumulators
 // (2 x 256 columns) share the op(A) stage.  Loads alone took 0.91 ms and the

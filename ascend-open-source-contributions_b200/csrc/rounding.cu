@@ -14,9 +14,8 @@
 //                           or 3.75^2 var >= 1e-4; the reference compacts
 //                           flagged indices into per-core lists;
 //   4. recompute (:192-404) each flagged output again, in a fixed order.
-// B200 design: one CTA of 64 threads per row for the energies (the row is
-// staged in shared memory; span is odd so the strided lane reads are
-// conflict-free); a grid-stride select in which each warp writes one 32-bit
+// B200 design: one CTA of 64 threads per row for the energies, each lane
+// reading its span from global memory; a grid-stride select in which each warp writes one 32-bit
 // word of the flag bitmap (its ballot) and adds its flags to a count per
 // 16 x 16 output tile.  The recompute then splits by density, on the device,
 // from those counts: a tile with more than kSparseMax flagged outputs is
@@ -930,8 +929,9 @@ static float bridge_term(int n)
 // op(A) n^2 complex | columns of op(B) n^2 complex | energies 2n floats |
 // flags: one bit per output (written whole by the selection), then one count
 // per 16 x 16 tile, kStatWords counters, the exact recompute's fallback bits
-// (one per output) and a byte per op(A) row and op(B) column marking those the
-// per-output kernels read, all zeroed before every selection | tensor-core
+// (one per output), a byte per op(A) row and op(B) column marking those the
+// per-output kernels read, a byte per op(A) row whose lane-major copy is made,
+// and the band marks, all zeroed before every selection | tensor-core
 // forms: the exact recompute's exponents, residue planes and product residues
 // (OzLayout).
 struct RoundLayout {
@@ -948,7 +948,7 @@ struct RoundLayout {
     uint8_t* need;      // rows of op(A), then columns of op(B), the per-output kernels read; then the op(A)
                         // rows whose lane-major copy is made
     BandMarks marks;    // 256-row bands whose tiles the form's products, the residues read (tensor-core forms)
-    size_t zero_bytes;  // tile_count + stats + fallback_bits + need + band, one memset
+    size_t zero_bytes;  // tile_count + stats + fallback_bits + need + marks, one memset
     OzLayout oz;
 };
 
