@@ -719,18 +719,18 @@ __global__ void __launch_bounds__(kLanes) recompute_sparse(int n, int span,
     const int band = blockIdx.x / (kSparseBand * gjn), first = band * kSparseBand;
     const int rows_in_band = min(kSparseBand, tiles - first), in_band = blockIdx.x - band * kSparseBand * gjn;
     const int gi = first + in_band % rows_in_band, gj = gj0 + in_band / rows_in_band;
-    const uint32_t count = tile_count[(size_t)gj * tiles + gi];
-    if (count == 0) {
-        return;
-    }
-    if (MODE != kFallbackFp64 && count > kSparseMax) {
-        return;
+    if (MODE != kFallbackFp64) {
+        const uint32_t count = tile_count[(size_t)gj * tiles + gi];
+        if (count == 0 || count > kSparseMax) {
+            return;
+        }
     }
     const int l = threadIdx.x;
     const int i0 = gi * kTile, j0 = gj * kTile;
     if (MODE == kFallbackFp64) {
-        // Fallback bits are only ever set inside the exact recompute's tiles:
-        // look at this tile's bits first (one or two words per column).
+        // Fallback bits are only ever set inside the exact recompute's tiles, on
+        // any output there, flagged or not: look at this tile's bits first (one
+        // or two words per column).
         bool any = false;
         if (l < kTile && j0 + l < n) {
             const size_t first = (size_t)(j0 + l) * n + i0, last = first + min(kTile, n - i0) - 1;
