@@ -457,7 +457,7 @@ cg3mStatus_t cg3mCgemm3mStridedBatched(cg3mHandle_t h, cg3mOperation_t transa, c
     const int per_launch = overlap ? 1 : batch_count;
     Problem p{transa, transb, m, n, k, alpha->real, alpha->imag, beta->real, beta->imag, A, lda, B, ldb, C, ldc};
     StridedPlan plan;
-    if (!make_strided_plan(p, 0, per_launch, h->sm_count, &plan)) {
+    if (!make_strided_plan(p, 0, per_launch, h->sm_count, strided_chain_limit(p, 0, per_launch, h->sm_count), &plan)) {
         return CG3M_STATUS_INVALID_VALUE;
     }
     // One problem per launch (a batch of one, or overlapping outputs): the
@@ -465,7 +465,7 @@ cg3mStatus_t cg3mCgemm3mStridedBatched(cg3mHandle_t h, cg3mOperation_t transa, c
     int tile = 0, parts = 1;
     void* ws = nullptr;
     if (per_launch == 1) {
-        plan_single(m, n, k, 0, h->sm_count, -1, 0, &tile, &parts);
+        plan_single(m, n, k, 0, h->sm_count, -1, 0, onchip_chain_limit(m, n, k, 0, h->sm_count), &tile, &parts);
     } else {
         const cg3mStatus_t wst = workspace(h, plan.bytes, &ws);
         if (wst != CG3M_STATUS_SUCCESS) {
@@ -531,14 +531,20 @@ cg3mStatus_t cg3mCgemm3mStridedBatchedEx(cg3mHandle_t h, cg3mOperation_t transa,
     if (batch_count > 1 && action == 2 && apart && opts.k_partitions == 0 &&
         (opts.engine == 0 || (tc && opts.engine == 1)) && h->stage_event_count == 0 &&
         make_plan(p, opts, h->sm_count, &one) && !one.rounding) {
+        // No less accurate than the calls one by one: in the form they run, FP32
+        // chains no longer than theirs, or than the segments a tensor-core form's
+        // calls accumulate.
+        const bool tensor = one.form != CG3M_FORM_FP32;
         double best = one.est_us * batch_count;
         StridedPlan strided;
-        const bool onchip = opts.engine == 0 && make_strided_plan(p, 0, batch_count, h->sm_count, &strided) &&
-                            strided.est_us * (tc ? 1.1 : 1.0) < best;
+        const bool onchip =
+            opts.engine == 0 &&
+            make_strided_plan(p, 0, batch_count, h->sm_count, tensor ? one.tc_segment : one.span, &strided) &&
+            strided.est_us * (tc ? 1.1 : 1.0) < best;
         if (onchip) {
             best = strided.est_us * (tc ? 1.1 : 1.0);
         }
-        if (tc && m > 128 && batch_tc_time_us(p, opts, h->sm_count, batch_count) < best) {
+        if (tensor && m > 128 && batch_tc_time_us(p, opts, h->sm_count, batch_count) < best) {
             // As many problems per launch as fit kBatchPlaneBytes of planes (at
             // least one), in even chunks; fewer when the device has no room.
             Plan plan;
@@ -669,7 +675,7 @@ cg3mStatus_t cg3mCgemm(cg3mHandle_t h, cg3mOperation_t transa, cg3mOperation_t t
     // Four products: the one-launch kernel of the on-chip family (K
     // partitions merged in a cluster; no workspace).
     int tile = 0, parts = 1;
-    plan_single(m, n, k, mode, h->sm_count, -1, 0, &tile, &parts);
+    plan_single(m, n, k, mode, h->sm_count, -1, 0, onchip_chain_limit(m, n, k, mode, h->sm_count), &tile, &parts);
     return to_status(launch_single(h->stream, p, mode, 0, tile, parts));
 }
 
@@ -1064,13 +1070,15 @@ cg3mStatus_t cg3mPlanOnchip(int m, int n, int k, int mode, int batch, int sm_cou
     }
     Problem p{CG3M_OP_N, CG3M_OP_N, m, n, k, 1.0f, 0.0f, 0.0f, 0.0f, nullptr, m, nullptr, k, nullptr, m};
     StridedPlan plan;
-    if (!make_strided_plan(p, mode, batch, sm_count > 0 ? sm_count : 148, &plan)) {
+    const int sms = sm_count > 0 ? sm_count : 148;
+    if (m <= 0 || n <= 0 || k <= 0 || mode < 0 || mode > 1 || batch <= 0 ||
+        !make_strided_plan(p, mode, batch, sms, strided_chain_limit(p, mode, batch, sms), &plan)) {
         return CG3M_STATUS_INVALID_VALUE;
     }
     std::memset(info, 0, sizeof(*info));
     if (batch == 1) {  // one problem: the one-launch kernel
         int tile = 0, parts = 1;
-        plan_single(m, n, k, mode, sm_count > 0 ? sm_count : 148, -1, 0, &tile, &parts);
+        plan_single(m, n, k, mode, sms, -1, 0, onchip_chain_limit(m, n, k, mode, sms), &tile, &parts);
         info->path = 4;
         info->tile_m = single_tile_bm(tile);
         info->tile_n = single_tile_bn(tile);

@@ -900,24 +900,21 @@ constexpr Policy kDefaultPolicy = {4096, 4};
 // tiles load more shared memory per FMA.
 constexpr double kTileEfficiency[kTileCount] = {1.0, 1.0, 0.93, 0.88, 0.87, 0.75};
 
-// Preference for large tiles, of the chain bound in make_strided_plan.
-constexpr double kLargeTiles[kTileCount] = {1.0, 0.85, 0.8, 0.8, 0.65, 0.45};
-
 int span_for(int k, int parts) { return ceil_div(ceil_div(k, 16), parts) * 16; }
 
 // The allowed tile with the least estimated time for p; returns that time
 // (padded work over efficiency) and sets tile, tiles_m, tiles_n.
-double choose_tile(BProblem& p, int max_area, int first_tile = 1, const double* efficiency = kTileEfficiency)
+double choose_tile(BProblem& p, int max_area)
 {
     int best = kTileCount - 1;
     double best_cost = 1e300;
-    for (int t = first_tile; t < kTileCount; ++t) {
+    for (int t = 1; t < kTileCount; ++t) {
         if (tile_bm(t) * tile_bn(t) > max_area) {
             continue;
         }
         const double work =
             (double)ceil_div(p.m, tile_bm(t)) * ceil_div(p.n, tile_bn(t)) * tile_bm(t) * tile_bn(t) * (p.k + 16);
-        const double cost = work / efficiency[t];
+        const double cost = work / kTileEfficiency[t];
         if (cost < best_cost) {
             best_cost = cost;
             best = t;
@@ -930,11 +927,11 @@ double choose_tile(BProblem& p, int max_area, int first_tile = 1, const double* 
 }
 
 // K partitions of p given the schedule's average work per SM.
-void choose_parts(BProblem& p, int split_cap, double per_sm, const double* efficiency = kTileEfficiency)
+void choose_parts(BProblem& p, int split_cap, double per_sm)
 {
     int parts = 1;
     if (split_cap > 1 && p.k >= 256) {
-        const double task = (double)tile_bm(p.tile) * tile_bn(p.tile) * (p.k + 16) / efficiency[p.tile];
+        const double task = (double)tile_bm(p.tile) * tile_bn(p.tile) * (p.k + 16) / kTileEfficiency[p.tile];
         const int want = (int)std::ceil(task / (0.25 * per_sm));
         parts = std::max(1, std::min({want, split_cap, p.k / 128}));
     }
@@ -1164,7 +1161,15 @@ constexpr int kClusterCap[5][kMaxClusterParts] = {{148, 74, 45, 33, 26, 22, 15, 
 // task the partials written and read.
 constexpr double kSplitLaunchUs = 3.0, kSplitUsPerOutput = 0.6e-3;
 
-bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, StridedPlan* out)
+int strided_chain_limit(const Problem& p, int mode, int batch, int sm_count)
+{
+    BatchChains chains(mode, sm_count);
+    chains.add(p.m, p.n, p.k, batch);
+    const int parts = chains.parts(p.m, p.n, p.k, 4);
+    return parts > 1 ? span_for(p.k, parts) : p.k;
+}
+
+bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, int max_span, StridedPlan* out)
 {
     if (batch <= 0 || p.m <= 0 || p.n <= 0 || p.k <= 0 || (mode != kMode3M && mode != kMode4M)) {
         return false;
@@ -1177,21 +1182,16 @@ bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, Stri
     bp.n = p.n;
     bp.k = p.k;
     const long long sms = std::max(sm_count, 1);
-    // A chain's rounding error grows with the square root of its terms: beyond
-    // kShortChain terms no longer than where a task of a large tile takes a
-    // quarter of an SM's work (at most four partitions), whatever is faster.
-    BProblem ref = bp;
-    const double one = choose_tile(ref, 8192, mode == kMode4M ? 1 : 0, kLargeTiles);
-    choose_parts(ref, 4, one * batch / (double)sms, kLargeTiles);
-    const int chain = std::max(kShortChain, ref.span);
+    const int most = std::max(8, ceil_div(p.k, std::max(max_span / 16 * 16, 16)));
     double best = 1e300;
     for (int t = 1; t < kTileCount; ++t) {
         const int tm = ceil_div(p.m, tile_bm(t)), tn = ceil_div(p.n, tile_bn(t));
         const int occ = kSingleOcc[mode == kMode4M ? 1 : 0][t];
         const SingleCost& c = kSingleCost[t];
-        for (int q = 1; q <= 8; ++q) {
+        for (int q = 1; q <= most; ++q) {
             const int span = q == 1 ? p.k : span_for(p.k, q);
-            if (span > chain || (q > 1 && (span < 48 || (q - 1) * span >= p.k))) {
+            const int coarser = q > 2 ? span_for(p.k, q - 1) : p.k;
+            if (span > max_span || (q > 1 && ((span < 48 && coarser <= max_span) || (q - 1) * span >= p.k))) {
                 continue;
             }
             const long long tasks = (long long)tm * tn * batch * q;
@@ -1211,6 +1211,9 @@ bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, Stri
                 bp.span = span;
             }
         }
+    }
+    if (best == 1e300) {
+        return false;
     }
     // Two tiles per task once every block has many of them: half the trips to
     // the task counter, and the pair shares op(B)'s columns.
@@ -1237,8 +1240,8 @@ bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, Stri
     return true;
 }
 
-double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile, int forced_parts, int* tile,
-                   int* parts)
+double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile, int forced_parts, int max_span,
+                   int* tile, int* parts)
 {
     sm_count = std::max(sm_count, 1);
     double best[kMaxClusterParts + 1];
@@ -1253,12 +1256,13 @@ double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile,
             continue;
         }
         const long long tiles = (long long)ceil_div(m, tile_bm(t)) * ceil_div(n, tile_bn(t));
-        for (int q = 1; q <= kMaxClusterParts; ++q) {
+        const int most = std::min(kMaxClusterParts, ceil_div(k, 16));  // partitions of 16 terms or more
+        for (int q = 1; q <= most; ++q) {
             if (forced_parts > 0 && q != forced_parts) {
                 continue;
             }
             const int span = q == 1 ? k : span_for(k, q);
-            if (q > 1 && (q - 1) * span >= k) {
+            if ((q > 1 && (q - 1) * span >= k) || (forced_parts <= 0 && span > max_span)) {
                 continue;
             }
             const int occ = kSingleOcc[mode == kMode4M ? 1 : 0][t];

@@ -100,7 +100,9 @@ cg3mStatus_t validate(int transa, int transb, int m, int n, int k, const cg3mCom
                       const void* B, int ldb, const cg3mComplex* beta, const void* C, int ldc, bool allow_conj_only,
                       int* action);
 
-bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* plan);
+// max_chain > 0 (FP32 form): chains of at most that many terms instead of the
+// call's chain limit; false when no split has them.
+bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* plan, int max_chain = 0);
 
 // Tensor-map encoding through the driver entry point (no -lcuda needed).
 bool encode_tensor_map(CUtensorMap* map, CUtensorMapDataType type, int rank, const uint64_t* dims,
@@ -250,19 +252,47 @@ struct StridedPlan {
     size_t bytes = 0;           // workspace bytes
     double est_us = 0.0;        // estimated time
 };
-bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, StridedPlan* out);
+// Chains of at most max_span terms; false when the shape is empty.
+bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, int max_span, StridedPlan* out);
+int strided_chain_limit(const Problem& p, int mode, int batch, int sm_count);
 // One problem in one launch of the on-chip family: grid (tiles, parts), the
 // `parts` K partitions of a tile merged through its thread-block cluster
 // (parts <= 8, and (parts - 1) * span < k).  tile: 0 128x64, 1 64x64,
 // 2 128x32, 3 32x128, 4 64x32, 5 32x32.  No workspace.
 cudaError_t launch_single(cudaStream_t s, const Problem& p, int mode, int repair, int tile, int parts);
+// How long a product's FP32 chains may be (chains.cpp).
+struct ChainLimit {
+    int span = 0;         // terms
+    int parts = 1;        // partitions of the split that sets it,
+    bool onchip = false;  // and its engine
+    bool tensor = false;  // a tensor-core form's call may run that form
+};
+// The limit of a call with `engine` as in cg3mOptions (2: one launch, with the
+// tile forced when >= 0).
+ChainLimit chain_limit(const Problem& p, int form, int engine, int tile, int sm_count);
+// The same for one problem on the on-chip family, mode as in launch_single.
+int onchip_chain_limit(int m, int n, int k, int mode, int sm_count);
+// The least partitions the problems of an on-chip batch take, given all of them
+// (a task of a large tile takes at most a quarter of an SM's share of the work).
+class BatchChains {
+public:
+    BatchChains(int mode, int sm_count);
+    void add(int m, int n, int k, int count);
+    int parts(int m, int n, int k, int most) const;
+
+private:
+    double task_work(int m, int n, int k, long long* tiles) const;
+    int first_tile, sms;
+    double total = 0.0;
+};
 // The one-launch plan for an m x n x k problem in `mode`: tile and K
-// partitions (each forced when >= 0), chosen to minimise the estimated time,
-// which is returned in microseconds.
-// FP32 chains up to this many terms are split for speed alone.
+// partitions (each forced when >= 0; unforced, chains of at most max_span
+// terms), chosen to minimise the estimated time, which is returned in
+// microseconds (1e300: eight partitions leave longer chains).
+double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile, int forced_parts, int max_span,
+                   int* tile, int* parts);
+// Beyond this many terms the planners look for finer splits than the fastest.
 constexpr int kShortChain = 1024;
-double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile, int forced_parts, int* tile,
-                   int* parts);
 int single_tile_bm(int tile);
 int single_tile_bn(int tile);
 cudaError_t launch_strided(cudaStream_t s, const Problem& p, int mode, int repair, long long sA, long long sB,

@@ -236,7 +236,7 @@ bool batch_tc_plan(const Problem& p, const cg3mOptions& opts, int sm_count, int 
     return true;
 }
 
-bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* plan)
+bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* plan, int max_chain)
 {
     Plan out{};
     out.action = 2;
@@ -272,7 +272,9 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
             --parts;
         }
         int tile = 0;
-        out.est_us = plan_single(p.m, p.n, p.k, 0, sm_count, opts.onchip_tile - 1, parts, &tile, &parts);
+        const int longest =
+            parts > 0 ? p.k : chain_limit(p, opts.form, 2, opts.onchip_tile - 1, sm_count).span;
+        out.est_us = plan_single(p.m, p.n, p.k, 0, sm_count, opts.onchip_tile - 1, parts, longest, &tile, &parts);
         out.engine = 2;
         out.onchip_tile = tile;
         out.tile_m = single_tile_bm(tile);
@@ -284,12 +286,32 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
         return true;
     }
 
+    // The chains the planner may choose; a tensor-core call whose form the rule
+    // rules out runs as plain FP32.
+    ChainLimit limit;
+    int longest = p.k;
+    if (!out.rounding && opts.k_partitions <= 0) {
+        if (max_chain > 0) {
+            longest = max_chain;
+        } else if (!tc || opts.engine == 0) {
+            limit = chain_limit(p, opts.form, opts.engine, -1, sm_count);
+            longest = limit.span;
+        }
+        if (tc && opts.engine == 0 && !limit.tensor) {
+            cg3mOptions fo = opts;
+            fo.form = CG3M_FORM_FP32;
+            fo.rounding = CG3M_ROUNDING_OFF;
+            return make_plan(p, fo, sm_count, plan);
+        }
+    }
+
     // ---- tile x K-partition search -------------------------------------------
     const TileChoice* tiles = tc ? kTcTiles : kFp32Tiles;
     const int granule = tc ? 64 : 16;
     const uint64_t default_tiles = (uint64_t)ceil_div(p.m, tiles[0].bm) * ceil_div(p.n, tiles[0].bn);
     TileChoice best_tile = tiles[0];
     int best_parts = 1;
+    bool packed = true;
     if (opts.k_partitions > 0) {
         best_parts = std::min(opts.k_partitions, 64);
     } else if (!tc && !out.rounding) {
@@ -301,7 +323,10 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
         uint64_t best = std::numeric_limits<uint64_t>::max();
         for (int parts = 1; parts <= 64; ++parts) {
             const int span = k_span(p.k, parts, granule);
-            if ((parts - 1) * span >= p.k || (parts > 1 && span < 64)) {
+            if (parts > 1 && span < 64) {
+                break;
+            }
+            if ((parts - 1) * span >= p.k || (parts > 1 ? span : p.k) > longest) {
                 continue;
             }
             const uint64_t waves = fp32_waves(default_tiles, parts, sm_count);
@@ -322,6 +347,7 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
                 best_parts = parts;
             }
         }
+        packed = best != std::numeric_limits<uint64_t>::max();
     } else if (!out.rounding) {
         // Tensor-core forms: the split with the least estimated time
         // (SelectCgemm3mDecomposition's joint search, :174-200, over one tile).
@@ -370,16 +396,19 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
         const bool narrow = p.k >= 1024 && std::min(p.m, p.n) <= 16 && std::max(p.m, p.n) <= 32;
         const int forced = opts.k_partitions > 0 ? out.parts : narrow ? 8 : 0;
         int tile = 0, parts = 0;
-        const double single = plan_single(p.m, p.n, p.k, 0, sm_count, -1, forced, &tile, &parts);
-        out.est_us = packed_time_us(p, out.parts, out.span, default_tiles, sm_count);
-        // Chains up to twice as long as the packed split's (1.4 times the error)
-        // or short, or a clear gain: narrow outputs pad the packed tile several
-        // times over (25 x 1025 x 59274: 8 partitions in one launch 438 us, 26
-        // packed 1078).
+        double single = plan_single(p.m, p.n, p.k, 0, sm_count, -1, forced, longest, &tile, &parts);
         const int single_span = parts > 1 ? k_span(p.k, parts) : p.k;
-        const bool chains = opts.k_partitions > 0 || single_span <= std::max(kShortChain, 2 * out.span) ||
+        if (single_span > longest) {
+            single = 1e300;
+        }
+        out.est_us = packed ? packed_time_us(p, out.parts, out.span, default_tiles, sm_count) : 1e300;
+        // Within the limit, chains up to twice as long as the packed split's (1.4
+        // times the error) or short, or a clear gain: narrow outputs pad the packed
+        // tile several times over (25 x 1025 x 59274: 8 partitions in one launch
+        // 438 us, 26 packed 1078).
+        const bool chains = !packed || opts.k_partitions > 0 || single_span <= std::max(kShortChain, 2 * out.span) ||
                             single < kSingleGain * out.est_us;
-        if (chains && single * kSingleMargin < out.est_us) {
+        if (single < 1e300 && chains && (!packed || single * kSingleMargin < out.est_us)) {
             out.est_us = single;
             out.engine = 2;
             out.onchip_tile = tile;
@@ -393,13 +422,19 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
         }
     }
 
+    if (!packed) {
+        return false;  // max_chain below every split's chains
+    }
+
     // ---- tensor-core forms on small shapes ---------------------------------------
-    // A tensor-core call carries a fixed cost of 12-13 us (pack, TMEM set-up,
-    // pipeline fill) that the FP32 engines do not.  Where the FP32 planner's
-    // own plan is clearly faster (a 1.1x margin over the rougher tensor-core
-    // model), the call runs that plan in plain FP32 -- its error is the plain
-    // form's, which every form promises not to exceed -- and reports form
-    // FP32.  engine 1 (or a forced K split) keeps the tensor-core path.
+    // A tensor-core call carries a fixed cost of 10-11 us (pack, TMEM set-up,
+    // pipeline fill; kTcCost) that the FP32 engines do not.  Where an FP32 plan is
+    // faster by more than the tensor-core model errs, the call runs that plan in
+    // plain FP32 and reports form FP32: one whose chains are no longer than the
+    // segments the form accumulates, which leaves an error no larger than the
+    // form's (256 terms, segments of 32, uniform: FP32 chains of 32 1.62e-7,
+    // 3xTF32 2.67e-7, split-BF16 4.27e-7).  engine 1 (or a forced K split) keeps
+    // the tensor-core path.
     if (tc) {
         out.est_us = tc_time_us(p, opts.form, out.tc_segment, out.parts, out.span, sm_count);
     }
@@ -408,7 +443,7 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
         fo.form = CG3M_FORM_FP32;
         fo.rounding = CG3M_ROUNDING_OFF;
         Plan fp;
-        if (make_plan(p, fo, sm_count, &fp) && fp.est_us * 1.05 < out.est_us) {
+        if (make_plan(p, fo, sm_count, &fp, out.tc_segment) && fp.est_us * 1.05 < out.est_us) {
             *plan = fp;
             return true;
         }
