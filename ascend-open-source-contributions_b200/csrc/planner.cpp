@@ -351,11 +351,13 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
     } else if (!out.rounding) {
         // Tensor-core forms: the split with the least estimated time
         // (SelectCgemm3mDecomposition's joint search, :174-200, over one tile).
-        // Partitions keep >= 128 K terms, >= 256 beyond the reference's four.
+        // Partitions keep >= 64 K terms, one K-block of the split planes (546 x 739 x
+        // 204, 3xTF32: four of 64 20.0 us, two of 128 23.9), >= 256 beyond the
+        // reference's four.
         double best = std::numeric_limits<double>::max();
         for (int parts = 1; parts <= 64; ++parts) {
             const int span = k_span(p.k, parts, granule);
-            if (parts > 1 && ((parts - 1) * span >= p.k || span < (parts > 4 ? 256 : 128))) {
+            if (parts > 1 && ((parts - 1) * span >= p.k || span < (parts > 4 ? 256 : 64))) {
                 continue;
             }
             const double us =

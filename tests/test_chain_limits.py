@@ -36,3 +36,9 @@ def test_tensor_forms(cg3m):
             assert p["form"] == cg3m.FORM["fp32"] and p["k_span"] <= span, (m, n, k, form)
         elif p["form"] == cg3m.FORM["fp32"]:
             assert p["k_span"] <= segment, (m, n, k, form)
+
+
+# 204 and 213 terms: four partitions of 64 took 19.9 us, two of 128 23.8 (3xTF32)
+@pytest.mark.parametrize("m,n,k", [(546, 739, 204), (535, 704, 213)])
+def test_short_tensor_products_split_four_ways(cg3m, m, n, k):
+    assert cg3m.plan("N", "N", m, n, k, alpha=0.5, form="tf32x3", engine="packed")["k_partitions"] == 4
