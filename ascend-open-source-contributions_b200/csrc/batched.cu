@@ -706,15 +706,22 @@ tile_task<TILE, MODE, kUnroll>(cur, r / proto.parts, r % proto.parts, ring, part
 // memory in place until all reads are done.  Nothing goes through global
 // memory but A, B and C: no workspace, no counters, no second launch.  Both
 // barriers are reached by every thread of every block (no early exits).
+// Shared memory of an SM, and what each block takes besides its own.
+constexpr size_t kSmSmem = 228 * 1024, kBlockSmem = 1024;
 template <int BM, int BN, int MODE>
 struct SingleCfg {
     using G = Cfg<BM, BN, MODE>;
-    static constexpr int STAGES = 4;
-    static constexpr size_t SMEM = (size_t)STAGES * G::STAGE * sizeof(float2);
     // blocks per SM the registers allow (65536 / threads / registers of the micro-kernel)
     static constexpr int BLOCKS = G::THREADS == 256 ? 1 : G::AREA >= 4096 ? (MODE == kMode3M ? 3 : 2)
                                                       : G::AREA >= 2048   ? 4
                                                                           : 5;
+    // Four stages, or three where only those leave room for BLOCKS blocks on an
+    // SM (128 x 32 and 32 x 128, three products: 1.06 times as fast as four
+    // stages and two blocks over 70 shapes, 0.9 to 1.3).
+    static constexpr size_t stage_bytes = (size_t)G::STAGE * sizeof(float2);
+    static constexpr int STAGES = BLOCKS * (4 * stage_bytes + kBlockSmem) <= kSmSmem ? 4 : 3;
+    static constexpr size_t SMEM = STAGES * stage_bytes;
+    static_assert(BLOCKS * (SMEM + kBlockSmem) <= kSmSmem, "the blocks that registers allow fit shared memory");
     static_assert((size_t)2 * BM * BN * sizeof(float) <= SMEM, "partials exceed the ring");
 };
 
@@ -1145,8 +1152,9 @@ int single_tile_bn(int tile) { return tile_bn(tile); }
 
 // Time model of the one-launch kernel (three-product mode), in microseconds,
 // fitted on B200 to 2500 timed (shape, tile, partitions) launches (median
-// error 2-4 % per tile; the tile and split it picks cost a mean 2 % over the
-// best of each shape).  Clusters of `parts` blocks run in waves of as many
+// error 2-4 % per tile then, 3-8 % since the merge loads two outputs at a time,
+// the small tiles' launches being the faster; what the planner picks costs a
+// mean 1.1 % over the best within the chain limit, 210 shapes).  Clusters of `parts` blocks run in waves of as many
 // clusters as fit at once; a wave costs a fixed part and span x the per-term
 // time a block needs by itself.  Blocks that share an SM add a per-term cost
 // for every layer of clusters: one layer holds as many as fit with one block
@@ -1160,8 +1168,16 @@ struct SingleCost {
 constexpr SingleCost kSingleCost[kTileCount] = {{3.396, 3.006, 0.0, 167.65, 0.031},  {6.203, 0.0, 25.64, 70.90, 0.0},
                                                 {4.231, 2.119, 18.57, 76.50, 0.0},   {3.417, 2.711, 16.39, 80.99, 0.135},
                                                 {3.483, 0.0, 17.18, 40.77, 0.131},   {1.719, 0.927, 13.61, 23.63, 0.150}};
-// Blocks per SM of each tile (SingleCfg::BLOCKS), three and four products.
-constexpr int kSingleOcc[2][kTileCount] = {{1, 3, 3, 3, 4, 5}, {1, 2, 2, 2, 4, 5}};
+// Blocks per SM of each tile, three and four products (tile 0: three only).
+template <int MODE>
+constexpr int single_occ(int t)
+{
+    constexpr int occ[kTileCount] = {SingleCfg<128, 64, kMode3M>::BLOCKS, SingleCfg<64, 64, MODE>::BLOCKS,
+                                     SingleCfg<128, 32, MODE>::BLOCKS,    SingleCfg<32, 128, MODE>::BLOCKS,
+                                     SingleCfg<64, 32, MODE>::BLOCKS,     SingleCfg<32, 32, MODE>::BLOCKS};
+    return occ[t];
+}
+int single_occ(int mode, int t) { return mode == kMode4M ? single_occ<kMode4M>(t) : single_occ<kMode3M>(t); }
 // Clusters resident at once on 148 SMs (cudaOccupancyMaxActiveClusters), by
 // blocks per SM (1..5) and cluster size (1..8).
 constexpr int kClusterCap[5][kMaxClusterParts] = {{148, 74, 45, 33, 26, 22, 15, 15},
@@ -1200,7 +1216,7 @@ bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, int 
     double best = 1e300;
     for (int t = 1; t < kTileCount; ++t) {
         const int tm = ceil_div(p.m, tile_bm(t)), tn = ceil_div(p.n, tile_bn(t));
-        const int occ = kSingleOcc[mode == kMode4M ? 1 : 0][t];
+        const int occ = single_occ(mode, t);
         const SingleCost& c = kSingleCost[t];
         for (int q = 1; q <= most; ++q) {
             const int span = q == 1 ? p.k : span_for(p.k, q);
@@ -1279,7 +1295,7 @@ double plan_single(int m, int n, int k, int mode, int sm_count, int forced_tile,
             if ((q > 1 && (q - 1) * span >= k) || (forced_parts <= 0 && span > max_span)) {
                 continue;
             }
-            const int occ = kSingleOcc[mode == kMode4M ? 1 : 0][t];
+            const int occ = single_occ(mode, t);
             const long long cap = std::max<long long>(1, (long long)kClusterCap[occ - 1][q - 1] * sm_count / 148);
             const long long layer = std::max<long long>(1, (long long)kClusterCap[0][q - 1] * sm_count / 148);
             const long long waves = (tiles + cap - 1) / cap;
