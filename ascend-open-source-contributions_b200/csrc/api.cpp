@@ -105,7 +105,7 @@ cg3mStatus_t workspace(cg3mContext* h, size_t bytes, void** out)
     return CG3M_STATUS_SUCCESS;
 }
 
-// Operand planes one batched tensor-core launch may hold in the workspace.
+// Operand planes, or partials, one batched launch may hold in the workspace.
 constexpr size_t kBatchPlaneBytes = size_t(1) << 30;
 
 // Options of cg3mCgemm's three-product case: the FP32 drop-in arithmetic, no
@@ -457,7 +457,7 @@ cg3mStatus_t cg3mCgemm3mStridedBatched(cg3mHandle_t h, cg3mOperation_t transa, c
     const int per_launch = overlap ? 1 : batch_count;
     Problem p{transa, transb, m, n, k, alpha->real, alpha->imag, beta->real, beta->imag, A, lda, B, ldb, C, ldc};
     StridedPlan plan;
-    if (!make_strided_plan(p, 0, per_launch, h->sm_count, strided_chain_limit(p, 0, per_launch, h->sm_count), &plan)) {
+    if (!make_strided_plan(p, 0, per_launch, h->sm_count, &plan)) {
         return CG3M_STATUS_INVALID_VALUE;
     }
     // One problem per launch (a batch of one, or overlapping outputs): the
@@ -539,7 +539,8 @@ cg3mStatus_t cg3mCgemm3mStridedBatchedEx(cg3mHandle_t h, cg3mOperation_t transa,
         StridedPlan strided;
         const bool onchip =
             opts.engine == 0 &&
-            make_strided_plan(p, 0, batch_count, h->sm_count, tensor ? one.tc_segment : one.span, &strided) &&
+            make_strided_plan(p, 0, batch_count, h->sm_count, tensor ? one.tc_segment : one.span, kBatchPlaneBytes,
+                              &strided) &&
             strided.est_us * (tc ? 1.1 : 1.0) < best;
         if (onchip) {
             best = strided.est_us * (tc ? 1.1 : 1.0);
@@ -1071,8 +1072,7 @@ cg3mStatus_t cg3mPlanOnchip(int m, int n, int k, int mode, int batch, int sm_cou
     Problem p{CG3M_OP_N, CG3M_OP_N, m, n, k, 1.0f, 0.0f, 0.0f, 0.0f, nullptr, m, nullptr, k, nullptr, m};
     StridedPlan plan;
     const int sms = sm_count > 0 ? sm_count : 148;
-    if (m <= 0 || n <= 0 || k <= 0 || mode < 0 || mode > 1 || batch <= 0 ||
-        !make_strided_plan(p, mode, batch, sms, strided_chain_limit(p, mode, batch, sms), &plan)) {
+    if (!make_strided_plan(p, mode, batch, sms, &plan)) {
         return CG3M_STATUS_INVALID_VALUE;
     }
     std::memset(info, 0, sizeof(*info));

@@ -1191,15 +1191,36 @@ constexpr int kClusterCap[5][kMaxClusterParts] = {{148, 74, 45, 33, 26, 22, 15, 
 // task the partials written and read.
 constexpr double kSplitLaunchUs = 3.0, kSplitUsPerOutput = 0.6e-3;
 
-int strided_chain_limit(const Problem& p, int mode, int batch, int sm_count)
+namespace {
+
+// Floats of one problem's partials.
+size_t strided_partials(const Problem& p, int parts)
 {
+    return parts > 1 ? align_up((size_t)p.m, 32) * p.n * 2 * parts : 0;
+}
+
+// Where the partials start: after the task counter and the tile counters.
+size_t strided_partial_off(int batch, int tiles) { return align_up((1 + (size_t)batch * tiles) * sizeof(uint32_t), 256); }
+
+}  // namespace
+
+bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, StridedPlan* out)
+{
+    if (batch <= 0 || p.m <= 0 || p.n <= 0 || p.k <= 0 || (mode != kMode3M && mode != kMode4M)) {
+        return false;
+    }
     BatchChains chains(mode, sm_count);
     chains.add(p.m, p.n, p.k, batch);
     const int parts = chains.parts(p.m, p.n, p.k, 4);
-    return parts > 1 ? span_for(p.k, parts) : p.k;
+    // 32 x 32 tiles have the most counters
+    const size_t bytes = strided_partial_off(batch, ceil_div(p.m, 32) * ceil_div(p.n, 32)) +
+                         (size_t)batch * strided_partials(p, parts) * sizeof(float);
+    return make_strided_plan(p, mode, batch, sm_count, parts > 1 ? span_for(p.k, parts) : p.k,
+                             std::max(kPlanWorkspace, bytes), out);
 }
 
-bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, int max_span, StridedPlan* out)
+bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, int max_span, size_t max_bytes,
+                       StridedPlan* out)
 {
     if (batch <= 0 || p.m <= 0 || p.n <= 0 || p.k <= 0 || (mode != kMode3M && mode != kMode4M)) {
         return false;
@@ -1222,6 +1243,10 @@ bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, int 
             const int span = q == 1 ? p.k : span_for(p.k, q);
             const int coarser = q > 2 ? span_for(p.k, q - 1) : p.k;
             if (span > max_span || (q > 1 && ((span < 48 && coarser <= max_span) || (q - 1) * span >= p.k))) {
+                continue;
+            }
+            if (q > 1 && strided_partial_off(batch, tm * tn) + (size_t)batch * strided_partials(p, q) * sizeof(float) >
+                             max_bytes) {
                 continue;
             }
             const long long tasks = (long long)tm * tn * batch * q;

@@ -34,6 +34,10 @@ struct cg3mContext {
 namespace cg3m {
 
 constexpr size_t kDefaultWorkspaceBytes = size_t(32) << 20;  // cann_ops_blas.h:33-35
+// A plan that could do with less keeps within this much: what the default
+// workspace and the allocation-free entry point's array hold, less what aligns
+// and guards the regions.
+constexpr size_t kPlanWorkspace = kDefaultWorkspaceBytes - (size_t(64) << 10);
 constexpr size_t kRegionAlign = 512;                          // cgemm_host.cpp:33 (16 x 32 B)
 
 // Equal problems of one launch at element strides a, b, c (operand planes of
@@ -252,9 +256,13 @@ struct StridedPlan {
     size_t bytes = 0;           // workspace bytes
     double est_us = 0.0;        // estimated time
 };
-// Chains of at most max_span terms; false when the shape is empty.
-bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, int max_span, StridedPlan* out);
-int strided_chain_limit(const Problem& p, int mode, int batch, int sm_count);
+// Chains of at most max_span terms and max_bytes of workspace; false when the
+// shape is empty.
+bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, int max_span, size_t max_bytes,
+                       StridedPlan* out);
+// The same within the batch's chain limit and a default workspace, or the
+// workspace of the split that sets the limit where that is larger.
+bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, StridedPlan* out);
 // One problem in one launch of the on-chip family: grid (tiles, parts), the
 // `parts` K partitions of a tile merged through its thread-block cluster
 // (parts <= 8, and (parts - 1) * span < k).  tile: 0 128x64, 1 64x64,

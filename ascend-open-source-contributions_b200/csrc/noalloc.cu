@@ -103,6 +103,15 @@ extern "C" cg3mStatus_t cg3mCgemm3mNoAlloc(void* stream, cg3mOperation_t transa,
     if (!make_plan(p, opts, sms, &plan)) {
         return CG3M_STATUS_INVALID_VALUE;
     }
+    // A packed plan that outgrows the array gives way to the one-launch engine,
+    // which needs none of it, where that is the faster engine but for its longer
+    // chains; other products of that size are refused.
+    Plan other;
+    if (plan.total > kScratchBytes - kStatusBytes && make_plan(p, opts, sms, &other, p.k) && other.engine == 2) {
+        cg3mOptions one = opts;
+        one.engine = 2;
+        make_plan(p, one, sms, &plan);
+    }
     if (plan.total > kScratchBytes - kStatusBytes) {
         if (std::getenv("CG3M_LOG") != nullptr) {
             std::fprintf(stderr, "cg3mCgemm3mNoAlloc: needs %zu scratch bytes, the fixed array holds %zu\n",

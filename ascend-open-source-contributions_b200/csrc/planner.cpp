@@ -106,9 +106,6 @@ constexpr uint64_t kMergeFloatsPerTerm = 41500;
 // (cudaOccupancyMaxActiveClusters for one block per SM on 148 SMs), and the
 // merge costs about one K term per partition.
 constexpr int kClusterMergeMax = 8;
-// The fixed scratch of the allocation-free entry point and the workspace the
-// reference creates per handle, less what aligns and guards the regions.
-constexpr size_t kDefaultWorkspace = ((size_t)32 << 20) - ((size_t)64 << 10);
 constexpr uint64_t kClusterCapOneBlock[kClusterMergeMax] = {148, 74, 45, 33, 26, 22, 15, 15};
 
 uint64_t fp32_waves(uint64_t tiles, int parts, int sm_count)
@@ -319,6 +316,14 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
         // (EstimateCgemmCoreWork's busiest-core work with measured B200 costs).
         const size_t rows = align_up((size_t)p.m, 32), cols = align_up((size_t)p.n, 32);
         const size_t planes = 12 * (rows + cols) * (size_t)p.k, partial = 8 * rows * (size_t)p.n;
+        // Workspace: no call takes more than a default workspace that did with less
+        // by the rule's split; splits finer than a larger one's may add an eighth.
+        const auto bytes = [&](int parts) { return planes + (parts > kClusterMergeMax ? parts * partial : 0); };
+        size_t room = std::numeric_limits<size_t>::max();
+        if (max_chain <= 0) {
+            const size_t rule = limit.onchip ? 0 : bytes(limit.parts);
+            room = std::max(kPlanWorkspace, rule + (rule > kDefaultWorkspaceBytes ? rule / 8 : 0));
+        }
         const uint64_t fixed = p.k > kShortChain ? kLongWaveFixed : kFp32WaveFixed;
         uint64_t best = std::numeric_limits<uint64_t>::max();
         for (int parts = 1; parts <= 64; ++parts) {
@@ -326,7 +331,7 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
             if (parts > 1 && span < 64) {
                 break;
             }
-            if ((parts - 1) * span >= p.k || (parts > 1 ? span : p.k) > longest) {
+            if ((parts - 1) * span >= p.k || (parts > 1 ? span : p.k) > longest || bytes(parts) > room) {
                 continue;
             }
             const uint64_t waves = fp32_waves(default_tiles, parts, sm_count);
@@ -336,11 +341,7 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
                 : parts > 1              ? (uint64_t)parts
                                          : 0;
             // Beyond 32 partitions for a clear gain only (54 x 460 x 42520: 18
-            // partitions 372 us, 36 381; 128 x 128 x 65536: 32 295, 64 186), and
-            // not where the partials would push the call past a default workspace.
-            if (parts > 32 && planes <= kDefaultWorkspace && planes + (size_t)parts * partial > kDefaultWorkspace) {
-                break;
-            }
+            // partitions 372 us, 36 381; 128 x 128 x 65536: 32 295, 64 186).
             const uint64_t cost = (gemm + merge) * (parts > 32 ? 21 : 20);
             if (cost < best) {
                 best = cost;
