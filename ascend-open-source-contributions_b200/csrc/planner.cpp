@@ -251,6 +251,9 @@ bool make_plan(const Problem& p, const cg3mOptions& opts, int sm_count, Plan* pl
         sm_count = 148;
     }
     const bool tc = opts.form != CG3M_FORM_FP32;
+    if (opts.form < CG3M_FORM_FP32 || opts.form > CG3M_FORM_BF16X9) {
+        return false;  // the host-buffer entry point plans before any call checks its options
+    }
     if (opts.engine < 0 || opts.engine > 2 || opts.onchip_tile < 0 || opts.onchip_tile > 6) {
         return false;
     }
