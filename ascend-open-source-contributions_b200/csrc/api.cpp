@@ -133,6 +133,12 @@ cg3mStatus_t to_status(cudaError_t e)
     return CG3M_STATUS_EXECUTION_FAILED;
 }
 
+bool options_ok(const cg3mOptions& o)
+{
+    return o.form >= CG3M_FORM_FP32 && o.form <= CG3M_FORM_BF16X9 && o.rounding >= CG3M_ROUNDING_AUTO &&
+           o.rounding <= CG3M_ROUNDING_OFF && o.k_partitions >= 0;
+}
+
 cg3mStatus_t run_one(cg3mContext* h, int transa, int transb, int m, int n, int k, const cg3mComplex* alpha,
                      const cg3mComplex* A, int lda, const cg3mComplex* B, int ldb, const cg3mComplex* beta,
                      cg3mComplex* C, int ldc, const cg3mOptions& opts, bool allow_conj_only, cg3mCallInfo* info)
@@ -147,8 +153,7 @@ cg3mStatus_t run_one(cg3mContext* h, int transa, int transb, int m, int n, int k
     if (st != CG3M_STATUS_SUCCESS || action == 0) {
         return st;
     }
-    if (opts.form < CG3M_FORM_FP32 || opts.form > CG3M_FORM_BF16X9 || opts.rounding < CG3M_ROUNDING_AUTO ||
-        opts.rounding > CG3M_ROUNDING_OFF || opts.k_partitions < 0) {
+    if (!options_ok(opts)) {
         return CG3M_STATUS_INVALID_VALUE;
     }
     const cg3mStatus_t bs = bind_device(h);
@@ -512,7 +517,7 @@ cg3mStatus_t cg3mCgemm3mStridedBatchedEx(cg3mHandle_t h, cg3mOperation_t transa,
     if (st != CG3M_STATUS_SUCCESS || action == 0) {
         return st;
     }
-    if (opts.form < CG3M_FORM_FP32 || opts.form > CG3M_FORM_BF16X9) {
+    if (!options_ok(opts)) {
         return CG3M_STATUS_INVALID_VALUE;
     }
     const cg3mStatus_t bs = bind_device(h);
