@@ -139,6 +139,20 @@ bool options_ok(const cg3mOptions& o)
            o.rounding <= CG3M_ROUNDING_OFF && o.k_partitions >= 0;
 }
 
+// Addresses [lo, hi) within which the matrices X + i * stride of a batch lie,
+// each `cols` columns of `rows` elements ld apart.
+struct Reach {
+    uintptr_t lo, hi;
+    Reach(const cg3mComplex* X, int rows, int cols, int ld, int64_t stride, int batch)
+    {
+        const int64_t last = (int64_t)(batch - 1) * stride;
+        lo = (uintptr_t)X + (uintptr_t)(std::min<int64_t>(0, last) * (int64_t)sizeof(cg3mComplex));
+        hi = (uintptr_t)X +
+             (uintptr_t)((std::max<int64_t>(0, last) + (int64_t)(cols - 1) * ld + rows) * (int64_t)sizeof(cg3mComplex));
+    }
+    bool meets(const Reach& o) const { return lo < o.hi && o.lo < hi; }
+};
+
 cg3mStatus_t run_one(cg3mContext* h, int transa, int transb, int m, int n, int k, const cg3mComplex* alpha,
                      const cg3mComplex* A, int lda, const cg3mComplex* B, int ldb, const cg3mComplex* beta,
                      cg3mComplex* C, int ldc, const cg3mOptions& opts, bool allow_conj_only, cg3mCallInfo* info)
@@ -525,11 +539,16 @@ cg3mStatus_t cg3mCgemm3mStridedBatchedEx(cg3mHandle_t h, cg3mOperation_t transa,
         return bs;
     }
     // One launch for the batch when the calls would run the planner's plain
-    // choice (no forced split or engine, no rounding pass) and the outputs do
-    // not overlap; of that launch and the calls one by one, the faster by the
+    // choice (no forced split or engine, no rounding pass) and no output overlaps
+    // another or lies among the operands (one problem's output may be the next
+    // one's operand); of that launch and the calls one by one, the faster by the
     // planner's estimates.
     const long long span_c = (long long)(n - 1) * ldc + m;
-    const bool apart = (strideC < 0 ? -strideC : strideC) >= span_c;
+    const bool an = transa == CG3M_OP_N || transa == CG3M_OP_R, bn = transb == CG3M_OP_N || transb == CG3M_OP_R;
+    const Reach outputs(C, m, n, ldc, strideC, batch_count);
+    const bool apart = (strideC < 0 ? -strideC : strideC) >= span_c &&
+                       !outputs.meets(Reach(A, an ? m : k, an ? k : m, lda, strideA, batch_count)) &&
+                       !outputs.meets(Reach(B, bn ? k : n, bn ? n : k, ldb, strideB, batch_count));
     Problem p{transa, transb, m, n, k, alpha->real, alpha->imag, beta->real, beta->imag, A, lda, B, ldb, C, ldc};
     Plan one;
     const bool tc = opts.form != CG3M_FORM_FP32;

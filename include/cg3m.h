@@ -192,7 +192,8 @@ cg3mStatus_t cg3mCgemm3mStridedBatched(cg3mHandle_t handle, cg3mOperation_t tran
 /* batch_count calls of cg3mCgemm3mEx on equal shapes, X_i = X + i*strideX
  * (complex elements), with the extended entry points' options and op codes (R
  * included) and without the non-finite repair of the strided API above.  When
- * the outputs do not overlap and no split, engine or rounding pass is asked
+ * the outputs overlap neither one another nor the operands (the address ranges
+ * the batch's A, B and C span) and no split, engine or rounding pass is asked
  * for, the batch runs as one launch (tensor-core forms: one pack and one GEMM
  * over all problems, unsplit along K, the operand planes of at most 1 GiB of
  * problems at a time; or one launch of the on-chip FP32 family) where the
