@@ -389,6 +389,18 @@ def default_handle():
     return h
 
 
+def _operand(x):
+    """A torch matrix or batch as the library reads it: complex64 on the GPU,
+    contiguous, lazy conjugate and negative views resolved."""
+    import torch
+
+    if not x.is_cuda:
+        raise ValueError("cg3m runs on CUDA tensors only")
+    if x.dtype != torch.complex64:
+        raise TypeError(f"cg3m multiplies complex64 tensors, not {x.dtype}")
+    return x.resolve_conj().resolve_neg().contiguous()
+
+
 def _op_shape(A, B, ta, tb):
     """(m, n, k) of opt(A) @ opt(B) for the last two dimensions of torch tensors."""
     (ar, ac), (br, bc) = A.shape[-2:], B.shape[-2:]
@@ -405,12 +417,9 @@ def cgemm3m_batched(A, B, transa="N", transb="N", form="fp32"):
     faster way (cg3mCgemm3mStridedBatchedEx)."""
     import torch
 
-    if not (A.is_cuda and B.is_cuda):
-        raise ValueError("cg3m runs on CUDA tensors only")
     if A.dim() != 3 or B.dim() != 3 or A.shape[0] != B.shape[0]:
         raise ValueError("expected two 3-D tensors of one batch size")
-    A = A.contiguous()
-    B = B.contiguous()
+    A, B = _operand(A), _operand(B)
     ta, tb = _op(transa), _op(transb)
     m, n, k = _op_shape(A, B, ta, tb)
     C = torch.empty((A.shape[0], m, n), dtype=torch.complex64, device=A.device)
@@ -435,10 +444,7 @@ def cgemm3m(A, B, transa="N", transb="N", alpha=1.0, beta=0.0, C=None, form="fp3
     """
     import torch
 
-    if not (A.is_cuda and B.is_cuda):
-        raise ValueError("cg3m runs on CUDA tensors only")
-    A = A.contiguous()
-    B = B.contiguous()
+    A, B = _operand(A), _operand(B)
     ta, tb = _op(transa), _op(transb)
     (_, ac), (_, bc) = A.shape, B.shape
     m, n, k = _op_shape(A, B, ta, tb)
@@ -448,7 +454,7 @@ def cgemm3m(A, B, transa="N", transb="N", alpha=1.0, beta=0.0, C=None, form="fp3
     if C is None:
         C = torch.zeros((m, n), dtype=torch.complex64, device=A.device)
     else:
-        C = C.contiguous()
+        C = _operand(C)
     h = default_handle()
     h.cgemm3m(tb, ta, n, m, k, alpha, B, bc, A, ac, beta, C, n, form=form, rounding=rounding)
     return C
