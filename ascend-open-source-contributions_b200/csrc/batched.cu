@@ -614,16 +614,11 @@ __global__ void __launch_bounds__(kThreads, 3) batched_kernel(const BProblem* __
     __shared__ int last_flag;
     __shared__ BProblem cur;  // the task's problem: its fields are read where they are used
     static_assert(sizeof(BProblem) % 4 == 0 && sizeof(BProblem) / 4 <= kThreads, "one word per thread");
-    for (;;) {
-        __syncthreads();  // the previous task's shared-memory reads are done
-        if (threadIdx.x == 0) {
-            task_id = atomicAdd(next, 1);
-        }
-        __syncthreads();
-        const int t = task_id;
-        if (t >= ntasks) {
-            return;
-        }
+    // A block's first task is its own (gridDim.x <= ntasks): blocks are placed one
+    // on every SM before any takes a second, so the longest tasks, first in the
+    // list, start on SMs of their own.  Drawn from the counter, as the later ones
+    // are, they met on one SM by chance: 11 problems 74 -> 133 us.
+    for (int t = blockIdx.x; t < ntasks; t = task_id) {
         const BTask tk = tasks[t];
         if (threadIdx.x < sizeof(BProblem) / 4) {
             reinterpret_cast<uint32_t*>(&cur)[threadIdx.x] =
@@ -637,6 +632,11 @@ __global__ void __launch_bounds__(kThreads, 3) batched_kernel(const BProblem* __
             case 4: tile_task_call<4>(cur, tk.tile, tk.part, ring, partials, counters, &last_flag); break;
             default: tile_task_call<5>(cur, tk.tile, tk.part, ring, partials, counters, &last_flag); break;
         }
+        __syncthreads();  // the task's shared-memory reads are done
+        if (threadIdx.x == 0) {
+            task_id = (int)gridDim.x + atomicAdd(next, 1);
+        }
+        __syncthreads();
     }
 }
 
@@ -904,17 +904,17 @@ namespace {
 // One candidate table: the largest tile area allowed and the cap on K
 // partitions.  Each problem takes the allowed tile with the least estimated
 // time -- padded work (tiles x BM x BN x (k + 16)) over the tile's relative
-// FFMA efficiency -- and is split along K only when one of its tile tasks
-// would exceed a quarter of the batch's average work per SM (the longest task
-// bounds the persistent schedule), keeping >= 128 K terms per partition.
+// FFMA efficiency -- and is split along K as far as BatchChains asks: where a
+// large tile's task would exceed a quarter of the batch's average work per SM
+// (the longest task bounds the persistent schedule), keeping >= 128 K terms per
+// partition, whatever the tile.
 struct Policy {
     int max_area;
     int split_cap;
 };
 
 constexpr Policy kPolicies[] = {{4096, 1}, {4096, 2}, {4096, 4}, {4096, 8}, {2048, 1},
-                                {2048, 2}, {2048, 4}, {1024, 1}, {1024, 2}, {1024, 4}};
-constexpr Policy kDefaultPolicy = {4096, 4};
+                                {2048, 4}, {2048, 8}, {1024, 1}, {1024, 4}, {1024, 8}};
 
 // Relative FFMA efficiency of each tile shape (per output-element-term), from
 // the per-term cost of blocks sharing an SM (kSingleCost below): the narrower
@@ -923,9 +923,9 @@ constexpr double kTileEfficiency[kTileCount] = {1.0, 1.0, 0.93, 0.88, 0.87, 0.75
 
 int span_for(int k, int parts) { return ceil_div(ceil_div(k, 16), parts) * 16; }
 
-// The allowed tile with the least estimated time for p; returns that time
-// (padded work over efficiency) and sets tile, tiles_m, tiles_n.
-double choose_tile(BProblem& p, int max_area)
+// The allowed tile with the least estimated time for p (padded work over
+// efficiency).
+void choose_tile(BProblem& p, int max_area)
 {
     int best = kTileCount - 1;
     double best_cost = 1e300;
@@ -944,38 +944,18 @@ double choose_tile(BProblem& p, int max_area)
     p.tile = best;
     p.tiles_m = ceil_div(p.m, tile_bm(best));
     p.tiles_n = ceil_div(p.n, tile_bn(best));
-    return best_cost;
-}
-
-// K partitions of p given the schedule's average work per SM.
-void choose_parts(BProblem& p, int split_cap, double per_sm)
-{
-    int parts = 1;
-    if (split_cap > 1 && p.k >= 256) {
-        const double task = (double)tile_bm(p.tile) * tile_bn(p.tile) * (p.k + 16) / kTileEfficiency[p.tile];
-        const int want = (int)std::ceil(task / (0.25 * per_sm));
-        parts = std::max(1, std::min({want, split_cap, p.k / 128}));
-    }
-    p.parts = parts;
-    p.span = span_for(p.k, parts);
-    while (p.parts > 1 && (p.parts - 1) * p.span >= p.k) {
-        --p.parts;
-        p.span = span_for(p.k, p.parts);
-    }
-    if (p.parts == 1) {
-        p.span = p.k;
-    }
 }
 
 void apply_policy(std::vector<BProblem>& ps, const Policy& pol, int sm_count)
 {
-    double total = 0.0;
-    for (auto& p : ps) {
-        total += choose_tile(p, pol.max_area);
+    BatchChains chains(kMode3M, sm_count);
+    for (const auto& p : ps) {
+        chains.add(p.m, p.n, p.k, 1);
     }
-    const double per_sm = total / std::max(sm_count, 1);
     for (auto& p : ps) {
-        choose_parts(p, pol.split_cap, per_sm);
+        choose_tile(p, pol.max_area);
+        p.parts = chains.parts(p.m, p.n, p.k, pol.split_cap);
+        p.span = p.parts > 1 ? span_for(p.k, p.parts) : p.k;
     }
 }
 
@@ -1088,8 +1068,8 @@ std::string signature(int device, const std::vector<BProblem>& ps)
 
 // Times every candidate policy (median of 3 launches after one warm-up) with
 // the caller's A and B and a scratch C, and returns the fastest.  The
-// caller's C is never written.
-Policy autotune(cg3mBatchPlan* plan, cudaStream_t s)
+// caller's C is never written.  `untuned` where nothing can be timed.
+Policy autotune(cg3mBatchPlan* plan, cudaStream_t s, const Policy& untuned)
 {
     size_t celems = 0;
     for (const auto& p : plan->host) {
@@ -1098,7 +1078,7 @@ Policy autotune(cg3mBatchPlan* plan, cudaStream_t s)
     float2* scratch = nullptr;
     if (cudaMalloc(&scratch, sizeof(float2) * std::max<size_t>(1, celems)) != cudaSuccess) {
         cudaGetLastError();
-        return kDefaultPolicy;
+        return untuned;
     }
     cudaMemsetAsync(scratch, 0, sizeof(float2) * std::max<size_t>(1, celems), s);
     std::vector<BProblem> trial = plan->host;
@@ -1110,7 +1090,7 @@ Policy autotune(cg3mBatchPlan* plan, cudaStream_t s)
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    Policy best = kDefaultPolicy;
+    Policy best = untuned;
     float best_ms = 1e30f;
     for (const Policy& pol : kPolicies) {
         if (materialise(plan, trial, pol) != cudaSuccess) {
@@ -1186,6 +1166,35 @@ constexpr int kClusterCap[5][kMaxClusterParts] = {{148, 74, 45, 33, 26, 22, 15, 
                                                   {592, 296, 187, 142, 112, 93, 78, 71},
                                                   {740, 370, 235, 175, 142, 116, 97, 86}};
 }  // namespace
+
+// The policy of a batch that is not timed: four partitions at most, and the
+// tiles with the least bound on the schedule, the longest task on an SM of its
+// own plus an SM's share of the work (the model above).  A few problems need
+// small tiles to reach every SM; with 64 x 64 wherever they fit, 80 batches of 1
+// to 48 problems took 1.9 times as long (2 problems 68 us, now 40).
+static Policy untuned_policy(const std::vector<BProblem>& ps, int sm_count)
+{
+    Policy best{};
+    double least = 1e300;
+    for (const int area : {4096, 2048, 1024}) {
+        const Policy pol{area, 4};
+        std::vector<BProblem> trial = ps;
+        apply_policy(trial, pol, sm_count);
+        double longest = 0.0, total = 0.0;
+        for (const auto& p : trial) {
+            const SingleCost& c = kSingleCost[p.tile];
+            const double terms = 1e-3 * (p.parts > 1 ? p.span : p.k);
+            longest = std::max(longest, c.fixed_us + terms * (c.term_ns + c.shared_term_ns));
+            total += (double)p.tiles_m * p.tiles_n * p.parts * (c.fixed_us + terms * c.shared_term_ns);
+        }
+        const double us = longest + total / std::max(sm_count, 1);
+        if (us < least) {
+            least = us;
+            best = pol;
+        }
+    }
+    return best;
+}
 
 // A K split in the strided kernel: its last block's merge, and per output of a
 // task the partials written and read.
@@ -1543,7 +1552,7 @@ cg3mStatus_t cg3mBatchPlanCreate(cg3mHandle_t handle, const cg3mProblem* problem
     }
     plan->device = dev;
     plan->blocks_per_sm = std::max(1, plan->blocks_per_sm);
-    Policy pol = kDefaultPolicy;
+    Policy pol = untuned_policy(plan->host, plan->sm_count);
     const std::string sig = signature(dev, plan->host);
     bool cached = false;
     {
@@ -1555,7 +1564,7 @@ cg3mStatus_t cg3mBatchPlanCreate(cg3mHandle_t handle, const cg3mProblem* problem
         }
     }
     if (tune && !cached && !plan->host.empty()) {
-        pol = autotune(plan, handle->stream);
+        pol = autotune(plan, handle->stream, pol);
         std::lock_guard<std::mutex> lock(g_tune_mutex);
         g_tuned[sig] = pol;
     }
