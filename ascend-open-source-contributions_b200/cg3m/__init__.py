@@ -389,16 +389,16 @@ def default_handle():
     return h
 
 
-def _operand(x):
+def _operand(x, torch):
     """A torch matrix or batch as the library reads it: complex64 on the GPU,
     contiguous, lazy conjugate and negative views resolved."""
-    import torch
-
     if not x.is_cuda:
         raise ValueError("cg3m runs on CUDA tensors only")
-    if x.dtype != torch.complex64:
+    if x.dtype is not torch.complex64:
         raise TypeError(f"cg3m multiplies complex64 tensors, not {x.dtype}")
-    return x.resolve_conj().resolve_neg().contiguous()
+    if x.is_conj() or x.is_neg():
+        x = x.resolve_conj().resolve_neg()
+    return x.contiguous()
 
 
 def _op_shape(A, B, ta, tb):
@@ -419,7 +419,7 @@ def cgemm3m_batched(A, B, transa="N", transb="N", form="fp32"):
 
     if A.dim() != 3 or B.dim() != 3 or A.shape[0] != B.shape[0]:
         raise ValueError("expected two 3-D tensors of one batch size")
-    A, B = _operand(A), _operand(B)
+    A, B = _operand(A, torch), _operand(B, torch)
     ta, tb = _op(transa), _op(transb)
     m, n, k = _op_shape(A, B, ta, tb)
     C = torch.empty((A.shape[0], m, n), dtype=torch.complex64, device=A.device)
@@ -444,7 +444,7 @@ def cgemm3m(A, B, transa="N", transb="N", alpha=1.0, beta=0.0, C=None, form="fp3
     """
     import torch
 
-    A, B = _operand(A), _operand(B)
+    A, B = _operand(A, torch), _operand(B, torch)
     ta, tb = _op(transa), _op(transb)
     (_, ac), (_, bc) = A.shape, B.shape
     m, n, k = _op_shape(A, B, ta, tb)
@@ -454,7 +454,7 @@ def cgemm3m(A, B, transa="N", transb="N", alpha=1.0, beta=0.0, C=None, form="fp3
     if C is None:
         C = torch.zeros((m, n), dtype=torch.complex64, device=A.device)
     else:
-        C = _operand(C)
+        C = _operand(C, torch)
     h = default_handle()
     h.cgemm3m(tb, ta, n, m, k, alpha, B, bc, A, ac, beta, C, n, form=form, rounding=rounding)
     return C
