@@ -779,13 +779,29 @@ __global__ void __launch_bounds__(Cfg<BM, BN, MODE>::THREADS, SingleCfg<BM, BN, 
             part_im[c * BM + r] = v.y;
         }
     }
-    cluster_sync();  // every partition's values are in place and visible to the cluster
     const uint32_t re_local = static_cast<uint32_t>(__cvta_generic_to_shared(part_re));
     const uint32_t im_local = static_cast<uint32_t>(__cvta_generic_to_shared(part_im));
     const int per = (BM * BN + p.parts - 1) / p.parts;  // outputs merged by each block
-    const int e_end = min(BM * BN, (part + 1) * per);
+    const int begin = part * per + (int)threadIdx.x, e_end = min(BM * BN, (part + 1) * per);
+    const bool reads_c = !p.epi.unit && !p.epi.beta_zero;
+    float2 old[kMergeAhead] = {};
+    auto load_c = [&](int first) {
+#pragma unroll
+        for (int u = 0; u < kMergeAhead; ++u) {
+            const int e = first + u * G::THREADS, row = m0 + e % BM, col = n0 + e / BM;
+            old[u] = e < e_end && row < p.m && col < p.n ? p.C[(size_t)col * p.ldc + row]
+                                                                     : make_float2(0.0f, 0.0f);
+        }
+    };
+    if (reads_c) {
+        load_c(begin);
+    }   // C on the way while the cluster meets
+    cluster_sync();  // every partition's values are in place and visible to the cluster
     // kMergeAhead outputs' remote loads are in flight together.
-    for (int first = part * per + (int)threadIdx.x; first < e_end; first += kMergeAhead * G::THREADS) {
+    for (int first = begin; first < e_end; first += kMergeAhead * G::THREADS) {
+        if (reads_c && first != begin) {
+            load_c(first);
+        }
         float tr[kMergeAhead][kMaxClusterParts], ti[kMergeAhead][kMaxClusterParts];
 #pragma unroll
         for (int u = 0; u < kMergeAhead; ++u) {
@@ -817,8 +833,7 @@ __global__ void __launch_bounds__(Cfg<BM, BN, MODE>::THREADS, SingleCfg<BM, BN, 
             if (p.repair && !finite2(v)) {
                 v = repair_product(p, row, col);
             }
-            float2* cp = p.C + (size_t)col * p.ldc + row;
-            *cp = epilogue_value(v.x, v.y, p.epi, cp);
+            p.C[(size_t)col * p.ldc + row] = epilogue_with(v.x, v.y, p.epi, old[u]);
         }
     }
     cluster_sync();  // no block leaves while others may still read its shared memory
