@@ -105,6 +105,10 @@ cg3mStatus_t workspace(cg3mContext* h, size_t bytes, void** out)
     return CG3M_STATUS_SUCCESS;
 }
 
+// A copy between page-locked host memory and the device, one direction;
+// and what a panel's event waits and launches add to its product.
+constexpr double kCopyUs = 5.0, kCopyBytesPerUs = 53e3, kPanelUs = 8.0;
+
 // Operand planes, or partials, one batched launch may hold in the workspace.
 constexpr size_t kBatchPlaneBytes = size_t(1) << 30;
 
@@ -758,6 +762,34 @@ cg3mStatus_t cg3mCgemm3mHost(cg3mHandle_t h, cg3mOperation_t transa, cg3mOperati
     if (panels <= 0) {
         const int per = std::max(tile_n, ceil_div(ceil_div(n, 8), tile_n) * tile_n);
         panels = ceil_div(n, per);
+        // Fewer, where a panel's product outlasts its copies: one of few tiles takes
+        // no less time for being narrow (839 x 1356 x 771 in split-BF16, unsplit:
+        // six panels 605 us, three 470).  Each count's panels go through upload,
+        // product and download in turn.
+        double least = 0.0;
+        for (int count = panels; product && !pass.rounding && count >= 2; --count) {
+            const int w = std::min(n, ceil_div(ceil_div(n, count), tile_n) * tile_n);
+            const double a_up = kCopyUs + (double)m * k * 8.0 / kCopyBytesPerUs;
+            double up = a_up, done = 0.0, down = 0.0;
+            for (int j0 = 0; j0 < n; j0 += w) {
+                const int wj = std::min(w, n - j0);
+                const Problem panel{transa, transb, m, wj, k, alpha->real, alpha->imag, beta->real, beta->imag,
+                                    A, lda, B, ldb, C, ldc};
+                Plan plan;
+                if (!make_plan(panel, o, h->sm_count, &plan) || plan.est_us <= 0.0) {
+                    down = 1e300;
+                    break;
+                }
+                up += kCopyUs + ((double)k * wj + (beta_zero ? 0.0 : (double)m * wj)) * 8.0 / kCopyBytesPerUs;
+                done = std::max(done, up) + kPanelUs + plan.est_us;
+                down = std::max(down, done) + kCopyUs + (double)m * wj * 8.0 / kCopyBytesPerUs;
+            }
+            // by a clear gain over the first count: the copies' times vary
+            if (down < 1e300 && (least == 0.0 || down < 0.95 * least)) {
+                least = least == 0.0 ? down : down / 0.95;
+                panels = ceil_div(n, w);
+            }
+        }
     }
     panels = std::max(1, std::min(panels, n));
     int nb = ceil_div(n, panels);

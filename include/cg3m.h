@@ -324,7 +324,8 @@ cg3mStatus_t cg3mCgemm3mNoAlloc(void* stream, cg3mOperation_t transa, cg3mOperat
  * rounding-correction pass applies to the whole problem, the tensor-core forms
  * run it panel by panel (panels of whole 256-column tiles, at least two of
  * them), the FP32 form as one panel.
- * `panels` <= 0 picks the count (about 8 panels of whole tiles); the device
+ * `panels` <= 0 picks the count (about 8 panels of whole tiles, fewer where a
+ * panel's product outlasts its copies); the device
  * copies are kept in the handle for later calls.  op code R is accepted.
  * C rows past m (padding) are neither read nor written. */
 cg3mStatus_t cg3mCgemm3mHost(cg3mHandle_t handle, cg3mOperation_t transa, cg3mOperation_t transb, int m, int n, int k,
