@@ -753,6 +753,9 @@ cg3mStatus_t cg3mCgemm3mHost(cg3mHandle_t h, cg3mOperation_t transa, cg3mOperati
         }
         o.form = static_cast<cg3mForm_t>(plan.form);  // a small tensor-core call may run as plain FP32
         tile_n = plan.tile_n;
+        if (!plan.rounding && o.rounding == CG3M_ROUNDING_AUTO) {
+            o.rounding = CG3M_ROUNDING_OFF;  // nor in a panel that is square by itself
+        }
         if (plan.rounding && plan.form == CG3M_FORM_FP32) {
             panels = 1;
         } else if (plan.rounding) {
