@@ -128,10 +128,11 @@ template <int FORM, bool REST = false>
 __global__ void __launch_bounds__(TILE* ROWS) pack_kernel(PackSide a, PackSide b)
 {
     __shared__ float2 tile[TILE][TILE + 1];
-    // The GEMM's blocks set up (barriers, TMEM, tensor maps) on the SMs this
-    // kernel's last blocks leave.  Their exits trigger that launch: an explicit
-    // trigger in every block cost 10 % of a large pack (1266 x 25 x 18768: 102 ->
-    // 114 us), and one in the last wave's blocks as much.
+    // The GEMM's launch is triggered by these blocks' exits: once the last one has
+    // left, the GEMM's blocks set up (barriers, TMEM, tensor maps) while this
+    // kernel's writes are flushed.  An explicit trigger in every block, which would
+    // let them in earlier, cost 10 % of a large pack (1266 x 25 x 18768: 102 -> 114
+    // us), and one in the last wave's blocks as much.
     // Block x of side z covers tiles x, x + gridDim.x, ... of that side's own
     // tile grid (tile t at (t mod tiles_r, t / tiles_r)), so a long-K shape
     // launches no blocks over the other side's extent.  The full packs launch
