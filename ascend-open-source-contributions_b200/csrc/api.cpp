@@ -299,7 +299,7 @@ cudaError_t enqueue(cudaStream_t s, const Problem& p, const Plan& plan, void* ws
         }
     }
     if (err == cudaSuccess && plan.rounding) {
-        err = launch_rounding_prep(s, p, plan, ws, cols, &prep_launched, run_marks(count, prep_len, s));
+        err = launch_rounding_prep(s, p, plan, ws, &prep_launched, run_marks(count, prep_len, s));
         count += prep_launched;
         if (err == cudaSuccess) {
             int launched = 0;

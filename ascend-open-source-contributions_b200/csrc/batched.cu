@@ -658,8 +658,8 @@ constexpr size_t kStridedSmem = (size_t)kStages * StridedCfg<MODE, TILE>::STAGE 
 
 template <int MODE, int TILE>
 __global__ void __launch_bounds__(kThreads, (kStridedBlocks<MODE, TILE>))
-    strided_kernel(const __grid_constant__ BProblem proto, long long sA, long long sB, long long sC, int batch, size_t partial_stride,
-                   float* partials, uint32_t* counters)
+    strided_kernel(const __grid_constant__ BProblem proto, long long sA, long long sB, long long sC, int batch,
+                   size_t partial_stride, float* partials, uint32_t* counters)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* ring = reinterpret_cast<float2*>(smem_raw);
@@ -689,7 +689,7 @@ __global__ void __launch_bounds__(kThreads, (kStridedBlocks<MODE, TILE>))
             cur.counter_off = 1 + (size_t)b * tiles;
         }
         __syncthreads();
-tile_task<TILE, MODE, kUnroll>(cur, r / proto.parts, r % proto.parts, ring, partials, counters, &last_flag);
+        tile_task<TILE, MODE, kUnroll>(cur, r / proto.parts, r % proto.parts, ring, partials, counters, &last_flag);
     }
 }
 
@@ -1173,13 +1173,6 @@ constexpr int single_occ(int t)
     return occ[t];
 }
 int single_occ(int mode, int t) { return mode == kMode4M ? single_occ<kMode4M>(t) : single_occ<kMode3M>(t); }
-// Clusters resident at once on 148 SMs (cudaOccupancyMaxActiveClusters), by
-// blocks per SM (1..5) and cluster size (1..8).
-constexpr int kClusterCap[5][kMaxClusterParts] = {{148, 74, 45, 33, 26, 22, 15, 15},
-                                                  {296, 148, 93, 71, 56, 45, 37, 33},
-                                                  {444, 222, 142, 104, 82, 71, 56, 48},
-                                                  {592, 296, 187, 142, 112, 93, 78, 71},
-                                                  {740, 370, 235, 175, 142, 116, 97, 86}};
 }  // namespace
 
 // The policy of a batch that is not timed: four partitions at most, and the

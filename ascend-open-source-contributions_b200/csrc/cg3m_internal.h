@@ -157,8 +157,8 @@ struct LeadSelect {
     uint32_t* stats;
 };
 int rounding_prep_kernels(int form);
-cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const ColPanel& panel,
-                                 int* launched, const std::function<void(int)>& mark);
+cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* launched,
+                                 const std::function<void(int)>& mark);
 cudaError_t launch_rounding_finish(cudaStream_t s, const Problem& p, const Plan& plan, void* ws,
                                    const ColPanel& panel, int* status, int* launched,
                                    const std::function<void(int)>& mark);
@@ -268,6 +268,14 @@ bool make_strided_plan(const Problem& p, int mode, int batch, int sm_count, Stri
 // (parts <= 8, and (parts - 1) * span < k).  tile: 0 128x64, 1 64x64,
 // 2 128x32, 3 32x128, 4 64x32, 5 32x32.  No workspace.
 cudaError_t launch_single(cudaStream_t s, const Problem& p, int mode, int repair, int tile, int parts);
+// Clusters of 1..8 blocks resident at once on 148 SMs, by blocks per SM (1..5;
+// cudaOccupancyMaxActiveClusters: GPC boundaries leave fewer than SMs / blocks).
+constexpr int kClusterCap[5][8] = {{148, 74, 45, 33, 26, 22, 15, 15},
+                                   {296, 148, 93, 71, 56, 45, 37, 33},
+                                   {444, 222, 142, 104, 82, 71, 56, 48},
+                                   {592, 296, 187, 142, 112, 93, 78, 71},
+                                   {740, 370, 235, 175, 142, 116, 97, 86}};
+
 // How long a product's FP32 chains may be (chains.cpp).
 struct ChainLimit {
     int span = 0;         // terms

@@ -36,11 +36,6 @@ struct Split {
 // partitions (cgemm_host.cpp:269-273).
 bool narrow(int m, int n, int k) { return k >= 1024 && std::min(m, n) <= 16 && std::max(m, n) <= 32; }
 
-// Clusters of 1..8 blocks resident at once on 148 SMs, by blocks per SM.
-constexpr int kClusters[3][8] = {{148, 74, 45, 33, 26, 22, 15, 15},
-                                 {296, 148, 93, 71, 56, 45, 37, 33},
-                                 {444, 222, 142, 104, 82, 71, 56, 48}};
-
 // One launch, partitions merged in a cluster: a fixed cost per wave, one per K
 // term of a wave and one per K term of every block of the busiest SM.
 struct TileCost {
@@ -66,7 +61,7 @@ Split onchip_split(int m, int n, int k, bool four_products, int sms, int only_ti
             if ((only_parts > 0 && q != only_parts) || (q > 1 && (q - 1) * span >= k)) {
                 continue;
             }
-            const long long fit = std::max<long long>(1, (long long)kClusters[c.blocks - 1][q - 1] * sms / 148);
+            const long long fit = std::max<long long>(1, (long long)kClusterCap[c.blocks - 1][q - 1] * sms / 148);
             const double waves = (double)((tiles + fit - 1) / fit), load = (double)((tiles * q + sms - 1) / sms);
             const double cost = waves * c.fixed +
                                 span * 1e-3 * (four_products ? 4.0 / 3.0 : 1.0) * (waves * c.term + load * c.shared) +
@@ -87,7 +82,7 @@ Split packed_split(int m, int n, int k, int sms)
     const uint64_t tiles = (uint64_t)ceil_div(m, 128) * ceil_div(n, 64);
     auto waves = [&](int parts) {
         if (parts > 1 && parts <= 8) {
-            const uint64_t fit = std::max<uint64_t>(1, (uint64_t)kClusters[0][parts - 1] * sms / 148);
+            const uint64_t fit = std::max<uint64_t>(1, (uint64_t)kClusterCap[0][parts - 1] * sms / 148);
             return (tiles + fit - 1) / fit;
         }
         return (tiles * parts + sms - 1) / sms;

@@ -14,9 +14,9 @@
 //
 //   1. ozaki_split_kernel: every op(A) row i and op(B) column j gets a power
 //      of two 2^E > max |x| over the row (real and imaginary parts together;
-//      the energy kernel finds it); each part becomes the integer a = rn(x 2^(beta - E)), |a| <= 2^beta,
-//      beta = 47, and the row counts its parts for which a != x 2^(beta - E)
-//      (cA_i; cB_j for the columns).  Every prime factor of the kOzMods = 15
+//      the energy kernel finds it); each part becomes the integer
+//      a = rn(x 2^(beta - E)), |a| <= 2^beta, beta = 47, and the row counts its
+//      parts for which a != x 2^(beta - E) (cA_i; cB_j for the columns).  Every prime factor of the kOzMods = 15
 //      moduli p_m <= 241 (pairwise coprime, product M ~ 2^111.1) is 1 mod 4, so
 //      -1 has a square root r_m mod p_m and z -> (Re z + r_m Im z,
 //      Re z - r_m Im z) turns a complex product mod p_m into two independent
@@ -246,8 +246,8 @@ __device__ __forceinline__ void store_images(const float2 (*re)[3], const float2
     }
 }
 
-// One block per op(A) row (the first nrows_a) or op(B) column of the panel.  Plane layout:
-// [2m + {0 plus, 1 minus}][row][kpitch] int8 for both operands.
+// One block per op(A) row (the first nrows_a) or op(B) column of the panel.
+// Plane layout: [2m + {0 plus, 1 minus}][row][kpitch] int8 for both operands.
 //
 // All FP32: the 47-bit parts go through 16-bit limbs, so a residue is a few
 // exact FP32 products (15 FP32 operations per element and modulus for both
@@ -258,8 +258,8 @@ __device__ __forceinline__ void store_images(const float2 (*re)[3], const float2
 __global__ void __launch_bounds__(256)
     ozaki_split_kernel(int n, int pitch, const float2* __restrict__ rows_a, const float2* __restrict__ rows_b,
                        int8_t* __restrict__ pa, int8_t* __restrict__ pb, int kpitch, size_t plane_bytes,
-                       const int* __restrict__ E, const int* __restrict__ F, int* __restrict__ CA, int* __restrict__ CB,
-                       int nrows_a, int j0, const uint8_t* __restrict__ band_a, const uint8_t* __restrict__ band_b)
+                       const int* __restrict__ E, const int* __restrict__ F, int* __restrict__ CA,
+                       int* __restrict__ CB, int nrows_a, int j0, const uint8_t* __restrict__ band_a, const uint8_t* __restrict__ band_b)
 {
     __shared__ int wcnt[8];
     const int r = panel_row(blockIdx.x, nrows_a, n, j0);
@@ -839,9 +839,9 @@ cudaError_t launch_ozaki_split(cudaStream_t s, int n, int pitch, const ColPanel&
         return cudaErrorInvalidValue;  // the moduli cover the exact products up to order kOzMaxN
     }
     const int nrows_a = n;  // a later panel may be the first to take a tile of a row band
-    ozaki_split_kernel<<<nrows_a + panel.j1 - panel.j0, 256, 0, s>>>(n, pitch, rows_a, rows_b, L.planes_a, L.planes_b, L.kpitch,
-                                              L.plane_bytes, L.E, L.F, L.CA, L.CB, nrows_a, panel.j0, band_a,
-                                              band_b);
+    ozaki_split_kernel<<<nrows_a + panel.j1 - panel.j0, 256, 0, s>>>(
+        n, pitch, rows_a, rows_b, L.planes_a, L.planes_b, L.kpitch, L.plane_bytes, L.E, L.F, L.CA, L.CB, nrows_a,
+        panel.j0, band_a, band_b);
     return cudaGetLastError();
 }
 

@@ -103,15 +103,14 @@ constexpr uint64_t kMergeFloatsPerTerm = 41500;
 // With 2..8 partitions the partitions of a tile form one thread-block cluster
 // and merge through distributed shared memory inside the GEMM (no merge
 // kernel, no partial planes): waves then hold as many clusters as fit at once
-// (cudaOccupancyMaxActiveClusters for one block per SM on 148 SMs), and the
-// merge costs about one K term per partition.
+// (kClusterCap, one block per SM), and the merge costs about one K term per
+// partition.
 constexpr int kClusterMergeMax = 8;
-constexpr uint64_t kClusterCapOneBlock[kClusterMergeMax] = {148, 74, 45, 33, 26, 22, 15, 15};
 
 uint64_t fp32_waves(uint64_t tiles, int parts, int sm_count)
 {
     if (parts > 1 && parts <= kClusterMergeMax) {
-        const uint64_t cap = std::max<uint64_t>(1, kClusterCapOneBlock[parts - 1] * (uint64_t)sm_count / 148);
+        const uint64_t cap = std::max<uint64_t>(1, (uint64_t)kClusterCap[0][parts - 1] * sm_count / 148);
         return (tiles + cap - 1) / cap;
     }
     return (tiles * parts + sm_count - 1) / sm_count;
@@ -181,7 +180,7 @@ bool tc_cluster_merge(const Problem& p, int parts, int sm_count)
     if (p.m <= 128 || parts < 2 || parts > 4) {
         return false;
     }
-    const uint64_t cap = std::max<uint64_t>(1, kClusterCapOneBlock[2 * parts - 1] * (uint64_t)sm_count / 148);
+    const uint64_t cap = std::max<uint64_t>(1, (uint64_t)kClusterCap[0][2 * parts - 1] * sm_count / 148);
     return tc_tiles(p) <= cap;
 }
 

@@ -634,7 +634,8 @@ __global__ void __launch_bounds__(256) lanes_needed_kernel(int n, int tc, const 
     // panels start on whole words (j0 is a multiple of 256)
     const size_t words = ((size_t)j1 * n + 31) / 32;
     const int tiles16 = (n + kTile - 1) / kTile;
-    for (size_t w = (size_t)j0 * n / 32 + (size_t)blockIdx.x * blockDim.x + threadIdx.x; w < words; w += (size_t)gridDim.x * blockDim.x) {
+    for (size_t w = (size_t)j0 * n / 32 + (size_t)blockIdx.x * blockDim.x + threadIdx.x; w < words;
+         w += (size_t)gridDim.x * blockDim.x) {
         const uint32_t fb = tc ? fallback_bits[w] : 0u;
         uint32_t bits = flag_bits[w] | fb;
         // Fast path: a word inside one column and one tile row band whose tile
@@ -1122,8 +1123,8 @@ cudaError_t launch_rounding_pack(cudaStream_t s, const Problem& p, const Plan& p
     return err;
 }
 
-cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, const ColPanel& panel,
-                                 int* launched, const std::function<void(int)>& mark)
+cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& plan, void* ws, int* launched,
+                                 const std::function<void(int)>& mark)
 {
     const int n = p.n;
     const int pitch = row_pitch(n);
@@ -1131,7 +1132,6 @@ cudaError_t launch_rounding_prep(cudaStream_t s, const Problem& p, const Plan& p
     const int span = ((n + kLanes - 1) / kLanes) | 1;
     int count = 0;
     cudaError_t err = cudaSuccess;
-    (void)panel;  // only the FP32 form prepares anything here
     if (plan.form == CG3M_FORM_FP32) {  // the tensor-core forms packed their rows and energies first
         err = launch_pack_rows(s, p, L.rows_a, L.rows_b, pitch);
         mark(++count);

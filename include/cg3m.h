@@ -198,8 +198,10 @@ cg3mStatus_t cg3mCgemm3mStridedBatched(cg3mHandle_t handle, cg3mOperation_t tran
  * over all problems, unsplit along K, the operand planes of at most 1 GiB of
  * problems at a time; or one launch of the on-chip FP32 family) where the
  * planner estimates that faster than the calls one by one; the K split, and
- * with it the last bits, may then differ from the single call's.  Validated
- * once, with the first matrices. */
+ * with it the last bits, may then differ from the single call's.  No less
+ * accurate than the single calls: the form they run, FP32 chains no longer than
+ * theirs.  The planes stay in the handle's workspace until it is destroyed.
+ * Validated once, with the first matrices. */
 cg3mStatus_t cg3mCgemm3mStridedBatchedEx(cg3mHandle_t handle, cg3mOperation_t transa, cg3mOperation_t transb, int m,
                                          int n, int k, const cg3mComplex* alpha, const cg3mComplex* A, int lda,
                                          int64_t strideA, const cg3mComplex* B, int ldb, int64_t strideB,
