@@ -452,7 +452,8 @@ def cgemm3m(A, B, transa="N", transb="N", alpha=1.0, beta=0.0, C=None, form="fp3
     # C^T = op(B)^T op(A)^T, i.e. swap the operands (the reference's C^T
     # convention, gemm_host_common.h:69-74).
     if C is None:
-        C = torch.zeros((m, n), dtype=torch.complex64, device=A.device)
+        # beta == 0: every element is written, none read
+        C = (torch.zeros if beta != 0 else torch.empty)((m, n), dtype=torch.complex64, device=A.device)
     else:
         C = _operand(C, torch)
     h = default_handle()

@@ -75,15 +75,15 @@ class Cgemm3mFunction(torch.autograd.Function):
     def forward(ctx, A, B, transa="N", transb="N", form="fp32"):
         ctx.save_for_backward(A, B)
         ctx.ops = (transa, transb, form)
-        return _mm(A.contiguous(), B.contiguous(), transa, transb, form)
+        return _mm(A, B, transa, transb, form)
 
     @staticmethod
     def backward(ctx, dC):
         A, B = ctx.saved_tensors
         ta, tb, form = ctx.ops
-        dC = dC.contiguous()
-        gA = grad_a(dC, B.contiguous(), ta, tb, form) if ctx.needs_input_grad[0] else None
-        gB = grad_b(dC, A.contiguous(), ta, tb, form) if ctx.needs_input_grad[1] else None
+        dC = dC.contiguous()  # once for both products; they make the other operands contiguous
+        gA = grad_a(dC, B, ta, tb, form) if ctx.needs_input_grad[0] else None
+        gB = grad_b(dC, A, ta, tb, form) if ctx.needs_input_grad[1] else None
         return gA, gB, None, None, None
 
 
